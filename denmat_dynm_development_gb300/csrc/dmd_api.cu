@@ -18,6 +18,7 @@
 #include "dmd_layout.h"
 #include "dmd_pairs.cuh"
 #include "dmd_pairs_cb.cuh"
+#include "dmd_pairs_fx.cuh"
 #include "dmd_sparse.cuh"
 
 using namespace dmd;
@@ -48,7 +49,9 @@ struct dmd_handle {
   int use_cb = 0;
   int lin = 0;                 // linearized master equation (DMD_FLAG_LINEAR)
   int pcfg = 0;                // pair-kernel shape variant of the f64x form (DMD_PAIR_CFG)
-  int pcfg64 = 1;              // pair-kernel shape variant of the f64 form (DMD_PAIR_CFG64)
+  int use_fx = 0;              // f64 form: operators in block-scaled fixed point (dmd_pairs_fx.cuh)
+  int* d_rbJ = nullptr;        // column block of every row block (f64 form)
+  int16_t* d_ex = nullptr;     // exponents of the fixed-point operators [row block][line][group]
   int* d_pos = nullptr;        // k -> energy rank
   int* d_inv = nullptr;        // energy rank -> k
   dmd::RowBlock* d_rb = nullptr;
@@ -322,6 +325,30 @@ void tc_launches(dmd_handle* h, size_t half) {
   h->launches += 1;  // the packing launch; the two passes are counted with the other forms
 }
 
+// the f64 contraction in fixed point: the Hermitian pass and the gated pass (anti-Hermitian part,
+// non-finite states). Against the FP64-pipe form per launch: 0.235 and 0.80 ms on 2.5M nb = 2 pairs, 29 and
+// 73 us on 70k, 125 and 325 us on 46k nb = 4 pairs, so it takes every handle whose operators have the form
+constexpr int kFxCtas = 4;
+template <int NB>
+void fx_pair_launches(dmd_handle* h, size_t half) {
+  const unsigned g = blocks_for(2LL * h->nitems, 4);
+  const size_t smem = FxSmem<NB>::cta_bytes;
+  const double* rs = (const double*)h->d_rs;
+  k_pairs_fx<NB, kFxCtas, false><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
+                                                                   rs, half, (double*)h->d_acc, h->nk, h->d_hflag, h->d_err);
+  k_pairs_fx<NB, kFxCtas, true><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
+                                                                  rs, half, (double*)h->d_acc, h->nk, h->d_hflag, h->d_err);
+}
+
+template <int NB>
+cudaError_t fx_attrs() {
+  const int bytes = (int)FxSmem<NB>::cta_bytes;
+  cudaError_t e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e;
+}
+
 template <int NB>
 int launch_pairs(dmd_handle* h) {
   if (h->npair == 0) return DMD_OK;
@@ -357,22 +384,19 @@ int launch_pairs(dmd_handle* h) {
             default: herm_pair_launches<ArithDF, NB, 2, 2, 4>(h, rs, half); break;
           }
         }
+      } else if (h->use_fx) {
+        fx_pair_launches<NB>(h, half);
       } else if (h->prec == DMD_PREC_F32) {
         herm_pair_launches<ArithF32, NB, 4, 2, 5>(h, (const float*)h->d_rs, half);
       } else if (h->prec == DMD_PREC_BF16X2) {
         herm_pair_launches<ArithBF2, NB, 4, 2, 5>(h, (const float*)h->d_rs, half);
       } else {
         const double* rs = (const double*)h->d_rs;
+        // on the FP64 pipe: the e-e model's operators, and operators without a fixed-point form. nb = 2 adds
+        // the forward partials with FP64 reductions in L2, off that pipe (2.65 -> 2.47 ms per launch on
+        // 9.7M pairs)
         if constexpr (NB == 2) {
-          // shapes of the FP64 contraction (autotuned; 1 by default): 0 reduces the forward partials
-          // over the warp; 1-3 add them with FP64 reductions in L2 (off the FP64 pipe: 2.65 -> 2.47 ms
-          // per launch on the 9.7M-pair workload), with 4 or 5 CTAs per SM
-          switch (h->pcfg64) {
-            case 1: herm_pair_launches<ArithF64, NB, 2, 2, 4, 1, true>(h, rs, half); break;
-            case 2: herm_pair_launches<ArithF64, NB, 2, 2, 5, 1, true>(h, rs, half); break;
-            case 3: herm_pair_launches<ArithF64, NB, 1, 4, 5, 1, true>(h, rs, half); break;
-            default: herm_pair_launches<ArithF64, NB, 2, 2, 4>(h, rs, half); break;
-          }
+          herm_pair_launches<ArithF64, NB, 2, 2, 4, 1, true>(h, rs, half);
         } else {
           herm_pair_launches<ArithF64, NB, 2, 2, 4>(h, rs, half);
         }
@@ -744,6 +768,35 @@ __global__ void k_cb_fill(long long p0, long long cnt, FillSrc src, double add_s
   }
 }
 
+// The stored FP64 elements to fixed point (dmd_pairs_fx.cuh) where they have that form: finite, and no k-point
+// so weakly coupled beside its column block's others that the shared exponents would leave it less than
+// FP64's precision (k_fx_spread). The e-e model rewrites the operators before every evaluation and keeps the
+// FP64-pipe contraction.
+int fx_convert(dmd_handle* h) {
+  h->use_fx = 0;
+  if (h->prec != DMD_PREC_F64 || h->eek) return DMD_OK;
+  const unsigned g = blocks_for(h->nrb, 4), gk = blocks_for(h->nk, 256);
+  double* sc = (double*)h->d_acc;  // scratch: [nk][2], rewritten by every evaluation
+  int bad = 0;
+  CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->st));
+  CK(cudaMemsetAsync(sc, 0, (size_t)h->nk * 16, h->st));
+  if (h->nb == 2) k_fx_spread<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
+  else k_fx_spread<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
+  k_fx_spread_check<<<gk, 256, 0, h->st>>>(h->nk, sc, h->d_flag);
+  CKL();
+  CK(cudaMemcpyAsync(&bad, h->d_flag, sizeof(bad), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  if (bad) return DMD_OK;
+  int rc;
+  if (!h->d_ex && (rc = dalloc(h, &h->d_ex, (size_t)h->nrb * 4 * h->nb2))) return rc;
+  if (h->nb == 2) k_fx_quantise<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex);
+  else k_fx_quantise<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex);
+  CKL();
+  CK(cudaStreamSynchronize(h->st));
+  h->use_fx = 1;
+  return DMD_OK;
+}
+
 struct CbDst;
 int fill_pairs_cb(dmd_handle* h, PairSource& src, const std::vector<CbDst>& dst, bool dev);
 
@@ -757,13 +810,17 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   dmd::PairLayout L;
   const int G = h->nb2 / 4, W = 32 / G;  // lanes per pair, columns per column block
   // pairs per work item: 512 (a warp's share on large workloads), fewer when the workload would
-  // not give every SM its 16 resident warps
+  // not give every SM its 16 resident warps. The fixed-point contraction (two warps per item, whose digits
+  // cost as much as a row block or two) takes items of up to 32 row blocks while they number 2.5 per SM:
+  // 66 against 81 us per launch on 398k pairs (437 and 778 items), 235 against 252 on 2.5M
   int ppi = 512 / G;
   {
     int nsm = 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
     const long long want = (long long)nsm * 16;
-    if (h->npair / ppi < want) ppi = (int)std::max<long long>(1, h->npair / want);
+    const bool fx = h->prec == DMD_PREC_F64 && !h->eek;
+    if (fx && h->npair * G * 2 / (32 * 32) > nsm * 5LL) ppi = 32 * 32 / G;
+    else if (h->npair / ppi < want) ppi = (int)std::max<long long>(1, h->npair / want);
   }
   if (!dmd::build_pair_layout(h->nk, nb, ew.data(), h->npair, d->k1st, d->k2nd, ppi, W, L))
     return fail(h, DMD_E_ARG, "k-pair index out of range");
@@ -771,23 +828,23 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   h->nrb = (long long)L.rb.size();
   // pair-kernel shape (stage lines, resident CTAs per SM); 0 is the default, the others serve tuning
   if (const char* v = getenv("DMD_PAIR_CFG")) h->pcfg = atoi(v);
-  if (const char* v = getenv("DMD_PAIR_CFG64")) h->pcfg64 = atoi(v);
   if (nb == 2) {
     cudaError_t (*const attrs[])() = {
         herm_pair_attrs<ArithDF, 2, 2, 2, 4>, herm_pair_attrs<ArithDF, 2, 2, 3, 3>, herm_pair_attrs<ArithDF, 2, 1, 4, 4>,
-        herm_pair_attrs<ArithDF, 2, 1, 3, 4>, herm_pair_attrs<ArithDF, 2, 1, 6, 3>, herm_pair_attrs<ArithF64, 2, 2, 2, 4>,
-        herm_pair_attrs<ArithF64, 2, 2, 2, 4, 1, true>, herm_pair_attrs<ArithF64, 2, 2, 2, 5, 1, true>,
-        herm_pair_attrs<ArithF64, 2, 1, 4, 5, 1, true>,
+        herm_pair_attrs<ArithDF, 2, 1, 3, 4>, herm_pair_attrs<ArithDF, 2, 1, 6, 3>,
+        herm_pair_attrs<ArithF64, 2, 2, 2, 4, 1, true>,
         herm_pair_attrs<ArithF32, 2, 4, 2, 5>, herm_pair_attrs<ArithBF2, 2, 4, 2, 5>,
         herm_pair_attrs<ArithF32, 2, 4, 2, 2, 4>, herm_pair_attrs<ArithF32, 2, 4, 2, 2, 8>,
         herm_pair_attrs<ArithBF2, 2, 4, 2, 2, 4>};
     for (auto fn : attrs) CK(fn());
+    CK(fx_attrs<2>());
   } else {
     cudaError_t (*const attrs[])() = {herm_pair_attrs<ArithDF, 4, 2, 2, 4>, herm_pair_attrs<ArithF64, 4, 2, 2, 4>,
                                       herm_pair_attrs<ArithF32, 4, 4, 2, 5>, herm_pair_attrs<ArithBF2, 4, 4, 2, 5>,
                                       herm_pair_attrs<ArithF32, 4, 4, 2, 2, 4>, herm_pair_attrs<ArithF32, 4, 4, 2, 2, 8>,
                                       herm_pair_attrs<ArithBF2, 4, 4, 2, 2, 4>};
     for (auto fn : attrs) CK(fn());
+    CK(fx_attrs<4>());
   }
   int rc;
   if ((rc = dalloc(h, &h->d_pos, (size_t)h->nk)) || (rc = dalloc(h, &h->d_rb, L.rb.size())) ||
@@ -798,6 +855,12 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   CK(cudaMemcpy(h->d_inv, L.inv.data(), L.inv.size() * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_rb, L.rb.data(), L.rb.size() * sizeof(dmd::RowBlock), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
+  if (h->prec == DMD_PREC_F64 && !h->eek) {
+    std::vector<int> J(L.rb.size());
+    for (const dmd::WorkItem& w : L.items) std::fill(J.begin() + w.rb0, J.begin() + w.rb1, w.J);
+    if ((rc = dalloc(h, &h->d_rbJ, J.size()))) return rc;
+    CK(cudaMemcpy(h->d_rbJ, J.data(), J.size() * 4, cudaMemcpyHostToDevice));
+  }
   const int esz = elem_bytes(h->prec);
   // deviation form: the constant contraction of diag(f_ref), position order [nk][2][nb2]
   const bool dev = deviation_form(h->prec) && !h->lin;
@@ -838,7 +901,8 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   PairSource* srcp = h->src ? h->src : nullptr;
   ArraySource arrays(d, nb4);
   if (!srcp) srcp = &arrays;
-  return fill_pairs_cb(h, *srcp, dst, dev);
+  if ((rc = fill_pairs_cb(h, *srcp, dst, dev))) return rc;
+  return fx_convert(h);
 }
 
 // Streams the raw operators through two pinned chunks and the fill kernel: the host reads chunk
@@ -1317,7 +1381,7 @@ void release(dmd_handle* h) {
                   h->d_coef, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
                   h->d_dst, h->d_ee_kvec, h->d_ee_kidx, h->d_ee_kmap, h->d_ee_U, h->d_ee_ewf, h->d_ee_f,
                   h->d_ee_dm, h->d_ee_dm1, h->d_ee_dmf, h->d_ee_dm1f, h->d_ee_scr, h->d_ee_Pee, h->d_ee_vqtab,
-                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec};
+                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int i = 0; i < 8; ++i) {
@@ -2767,6 +2831,9 @@ int dmd_add_operators(dmd_handle* h, const double* P1_add, const double* P2_add,
   h->launches += 1 + (h->npair + chunk - 1) / chunk;
   CKL();
   CK(cudaStreamSynchronize(h->st));
+  const int fx = h->use_fx;
+  if ((rc = fx_convert(h))) return rc;
+  if (h->use_fx != fx) drop_graphs(h);
   return DMD_OK;
 }
 
@@ -2786,9 +2853,6 @@ int dmd_autotune(dmd_handle* h, int evals, int* chosen) {
   if (h->use_cb && !h->use_tc && h->nrhs == 1 && h->prec == DMD_PREC_F64X && h->nb == 2) {
     cand = {0, 1, 2, 3, 4};
     knob = &h->pcfg;
-  } else if (h->use_cb && !h->use_tc && h->nrhs == 1 && h->prec == DMD_PREC_F64 && h->nb == 2) {
-    cand = {0, 1, 2, 3};
-    knob = &h->pcfg64;
   } else if (h->use_cb && !h->use_tc && h->nrhs > 1 && h->prec == DMD_PREC_F32) {
     cand = {4, 8};
     knob = &h->brw;

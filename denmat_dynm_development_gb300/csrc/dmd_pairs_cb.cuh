@@ -31,11 +31,18 @@
 //               FP64 rate on this part) do the work; the real and the imaginary half of each step
 //               are one FP32x2 instruction.
 #pragma once
+#include <type_traits>
+
 #include "dmd_common.cuh"
 #include "dmd_layout.h"
 #include "dmd_tma.cuh"
 
 namespace dmd {
+
+// flag raised by the prep kernels: bit 0, some rho_k is not exactly Hermitian; bit 1 (FP64 coordinates
+// only), some coordinate is not finite, which the fixed-point contraction cannot scale (dmd_pairs_fx.cuh)
+#define DMD_HFLAG_NONHERM 1u
+#define DMD_HFLAG_NONFINITE 2u
 
 // ---------------------------------------------------------------------------------------------
 // double-float helpers (no contraction: every operation is an explicit round-to-nearest op)
@@ -326,7 +333,8 @@ __global__ void k_prep_herm(int nk, int nbdm, int bs, const double2* __restrict_
       }
       ra[ab] = A::from_double(vij.y);
       if (ws) ra[NB2 + ab] = A::from_double(lin ? 0.0 : 0.0 - vij.y);
-      if (vij.y != 0.0) atomicOr(hflag, 1u);
+      if (vij.y != 0.0) atomicOr(hflag, DMD_HFLAG_NONHERM);
+      if (std::is_same<typename A::relem, double>::value && !(isfinite(vij.x) && isfinite(vij.y))) atomicOr(hflag, DMD_HFLAG_NONFINITE);
     }
     return;
   }
@@ -393,8 +401,9 @@ __global__ void k_prep_herm(int nk, int nbdm, int bs, const double2* __restrict_
       rh[NB2 + ab] = A::from_double(lin ? 0.0 : -r1.x);      // conj(D) o (1 - H) off the diagonal
       rh[NB2 + ji] = A::from_double(lin ? 0.0 : -r1.y);
     }
+    if (std::is_same<typename A::relem, double>::value && !(isfinite(r1.x) && isfinite(r1.y))) atomicOr(hflag, DMD_HFLAG_NONFINITE);
     if (dif.x != 0.0 || dif.y != 0.0) {  // the anti-Hermitian part is read only when hflag is raised
-      atomicOr(hflag, 1u);
+      atomicOr(hflag, DMD_HFLAG_NONHERM);
       const double2 aij = mk2(__dmul_rn(dif.y, 0.5), __dmul_rn(-dif.x, 0.5));
       const double2 r2 = cmul_rn(d, aij);                     // conj(D) o A
       ra[ab] = A::from_double(r2.x);
@@ -566,7 +575,7 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_herm(const WorkItem* __rest
   typedef typename A::acc Acc;
   typedef typename A::red_t R;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  if (gate && *gate == 0u) return;  // anti-Hermitian pass with nothing to do
+  if (gate && !(*gate & DMD_HFLAG_NONHERM)) return;  // anti-Hermitian pass with nothing to do
   const int wib = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int ngroups = (nrhs + RW - 1) / RW;

@@ -1,0 +1,557 @@
+// The FP64 k-pair contraction on the integer pipes: block-scaled fixed point (layout in dmd_layout.h,
+// coordinates and sums as in dmd_pairs_cb.cuh).
+//
+// Why. This part multiplies FP64 at 1.7 lanes per clock and SM, but adds a 32 x 32 -> 64-bit integer
+// product (mad.wide) at 61 (both measured). The contraction needs 16 nb^4 flops per pair: 2.35 ms on the FP64
+// pipe for 9.7M nb = 2 pairs, 0.75 ms of HBM time. In two-digit fixed point a multiply-add is three
+// mad.wide, a third of the HBM time. Measured, 2.5M nb = 2 pairs (1.27 GB): 235 us per launch, 5.4 TB/s (the FP64
+// pipe: 800 us); 177k nb = 4 pairs (1.45 GB): 320 us, 4.5 TB/s; 70k nb = 2 pairs in L2: 29 us (73). What bounds it
+// is the issue rate (50 %): per row block and matrix 192 mad.wide of some 750 instructions, the rest mainly
+// the cross-lane sums of the forward partials.
+//
+// Operators. The elements of a row block's line (Q1 row or Q2 column: the elements of one output, for up
+// to 32 / 8 pairs) are split in two groups -- products with a diagonal and with an off-diagonal
+// coordinate, which differ by the spin mixing -- and each group shares a binary exponent ex:
+//   q = p 2^(61 - ex) rounded to an integer = h 2^32 + l,  l signed,  |h| <= 2^29
+// in the 8 bytes of the double that it replaces: 61 bits below the group's largest element (FP64 keeps 53
+// below each element). An element of the layout is (re_h, re_l, im_h, im_l).
+// Coordinates. 59 bits (the rows' of nb = 4: 57) below the largest one of their group: the column's over the
+// work item's 32 (8) columns; a row's times the line's 2^ex over the item's rows (so the reverse sums,
+// which run over the item's rows, need no shift per row block). Built from the FP64 coordinates once per
+// item (columns) or row block (rows).
+// Sums. With rh, rl the digits of a coordinate, A0 += h rh and A1 += h rl + l rh are exact in 64 bits: A0
+// takes the 64 (96) terms of a forward sum over the warp or the 128 (512) of a reverse sum over an
+// item, A1 four lines' terms of 2^60 + 2^58 before it is folded into A0. What is dropped is l rl, at most 2^-58 of
+// the group's largest product. A forward sum is rounded to 2^-56 of it per lane and added over the
+// warp as integers, so a row block's sum is rounded to FP64 once; then one FP64 reduction in L2 per row
+// block and value (the FP64 kernel issues one per pair and value). Reverse sums keep A1's remainder and are exact
+// to the end of the item.
+//
+// A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, this kernel
+// returns and the gated launch (which otherwise carries the anti-Hermitian part of a non-Hermitian
+// state, bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do
+// in FP64. Operators with a non-finite element are never converted (dmd_api.cu).
+#pragma once
+#include <type_traits>
+
+#include "dmd_common.cuh"
+#include "dmd_layout.h"
+#include "dmd_pairs_cb.cuh"
+#include "dmd_tma.cuh"
+
+namespace dmd {
+
+constexpr int kFxPBits = 61;         // operator bits
+constexpr int kFxCBits = 59;         // column coordinate bits
+constexpr int kFxBase = 32;          // digit base 2^32
+constexpr int kFxExZero = -20000;    // exponent of a group without a nonzero element
+
+// bits of the row coordinates: a reverse sum's 128 (nb = 2) or 512 (nb = 4) products stay below 2^63
+// in units of 2^32
+__host__ __device__ constexpr int fx_row_bits(int nb) { return nb == 2 ? 59 : 57; }
+
+// e with |x| < 2^e (0 and tiny values: -900, far below any scale that matters and safe to invert)
+__device__ __forceinline__ int fx_expo(double x) {
+  const int f = ((__double2hiint(x) >> 20) & 0x7ff) - 1022;
+  return f < -900 ? -900 : f;
+}
+// x 2^s rounded to an integer (|x 2^s| < 2^62) and split into signed digits: q = h 2^32 + l. Integer
+// arithmetic: the FP64 pipe's conversions and products would cost as much as the item's sums.
+__device__ __forceinline__ int2 fx_digits(double x, int s) {
+  const long long b = __double_as_longlong(x);
+  const int f = (int)(b >> 52) & 0x7ff;
+  long long q = (b & 0xfffffffffffffLL) | (f ? 1LL << 52 : 0LL);
+  const int sh = (f ? f : 1) - 1075 + s;  // <= 9
+  q = sh >= 0 ? q << sh : (sh < -54 ? 0LL : (q + (1LL << (-sh - 1))) >> -sh);
+  if (b < 0) q = -q;
+  const int l = (int)q;
+  return make_int2((int)((q - l) >> kFxBase), l);
+}
+// x 2^e for a converted integer x (0 or 1 <= |x| <= 2^63): an addition to the exponent field where every such
+// result is normal
+__device__ __forceinline__ double fx_scale(double x, int e) {
+  if (e < -1000 || e > 900) return scalbn(x, e);
+  const int hi = __double2hiint(x);
+  return __hiloint2double(hi ? hi + (int)((unsigned)e << 20) : 0, __double2loint(x));
+}
+__device__ __forceinline__ double fx_decode(int h, int l, int ex) {
+  return scalbn((double)((long long)h * (1LL << kFxBase) + l), ex - kFxPBits);
+}
+__device__ __forceinline__ void fx_mul(long long& a0, long long& a1, int h, int l, int2 r, long long a1_0) {
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(a0) : "r"(h), "r"(r.x));
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(a1) : "r"(h), "r"(r.y), "l"(a1_0));
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a1) : "r"(l), "r"(r.x));
+}
+__device__ __forceinline__ int4 fx_lds(uint32_t addr) {
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void fx_mad(long long& a0, long long& a1, int h, int l, int2 r) {
+  // asm: written as 64-bit sums of products the compiler regroups them into trees with extra adds and moves
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a0) : "r"(h), "r"(r.x));
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a1) : "r"(h), "r"(r.y));
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a1) : "r"(l), "r"(r.x));
+}
+// carries of a1 into a0; returns a1's remainder in [0, 2^32)
+__device__ __forceinline__ unsigned fx_fold(long long& a0, long long a1) {
+  a0 += a1 >> kFxBase;
+  return (unsigned)a1;
+}
+
+// Whether line element b of a pair's quarter qg, at step i of the loop, is a diagonal coordinate's: nb = 2
+// walks b = 0..3 (diagonal: 0 and 3); nb = 4 walks its quarter from the diagonal element b = 4 qg + qg on
+template <int NB>
+__host__ __device__ constexpr int fx_group(int i) {
+  return NB == 2 ? ((i == 1 || i == 2) ? 1 : 0) : (i == 0 ? 0 : 1);
+}
+
+// What the shared exponents cost each k-point, one warp per row block: sc[k][0] adds the largest element of every
+// row block that holds a pair of k, sc[k][1] the largest of that pair itself (k by energy rank). An element is off by
+// at most 2^-62 of its block's largest, FP64 by 2^-53 of itself: with sc[0] <= 2^8 sc[1] the sums of k keep
+// FP64's error. Raises *bad at a non-finite element.
+template <int NB>
+__global__ void __launch_bounds__(128) k_fx_spread(long long nrb, const RowBlock* __restrict__ rbs, const int* __restrict__ rbJ,
+                                                   const double2* __restrict__ P, double* __restrict__ sc,
+                                                   int* __restrict__ bad) {
+  constexpr int NE = 2 * NB * NB * NB * NB, W = 128 / (NB * NB);
+  const long long r = blockIdx.x * 4LL + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= nrb) return;
+  const RowBlock b = rbs[r];
+  const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << lane) - 1u));
+  const bool on = (b.mask >> lane) & 1u;  // lane: column J W + lane
+  double mx = 0.0;
+  bool fin = true;
+  if (on) {
+    const double2* p = P + (size_t)b.pair0 * NE + slot;
+#pragma unroll 8
+    for (int e = 0; e < NE; ++e) {
+      const double2 v = p[(size_t)e * n];
+      fin = fin && isfinite(v.x) && isfinite(v.y);
+      mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+    }
+  }
+  if (!fin) *bad = 1;
+  double all = mx, sum = mx;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    all = fmax(all, __shfl_xor_sync(0xffffffffu, all, o));
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&sc[2 * (size_t)b.row], all);
+    atomicAdd(&sc[2 * (size_t)b.row + 1], sum);
+  }
+  if (on && ((b.revmask >> lane) & 1u)) {
+    const size_t c = (size_t)rbJ[r] * W + lane;
+    atomicAdd(&sc[2 * c], all);
+    atomicAdd(&sc[2 * c + 1], mx);
+  }
+}
+__global__ void k_fx_spread_check(int nk, const double* __restrict__ sc, int* __restrict__ bad) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const double all = k < nk ? sc[2 * (size_t)k] : 0.0, own = k < nk ? sc[2 * (size_t)k + 1] : 0.0;
+  if (own > 0.0 && !(all <= 256.0 * own && own > 1e-240)) *bad = 1;  // (fx_expo stops at 2^-900)
+}
+
+// FP64 elements to fixed point in place, one warp per row block; ex: [row block][line][group]
+template <int NB>
+__global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlock* __restrict__ rbs,
+                                                     unsigned char* __restrict__ P, int16_t* __restrict__ ex) {
+  constexpr int NB2 = NB * NB, NL = 2 * NB2;
+  const long long r = blockIdx.x * 4LL + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= nrb) return;
+  const RowBlock b = rbs[r];
+  const int n = __popc(b.mask), m = NB2 * n;
+  double2* p = (double2*)P + (size_t)b.pair0 * 2 * NB2 * NB2;
+  for (int L = 0; L < NL; ++L, p += m) {
+    double mx[2] = {0.0, 0.0};
+    for (int t = lane; t < m; t += 32) {
+      const int e = t / n;
+      const int g = (e / NB == e % NB) ? 0 : 1;
+      const double v = fmax(fabs(p[t].x), fabs(p[t].y));
+      if (g) mx[1] = fmax(mx[1], v);
+      else mx[0] = fmax(mx[0], v);
+    }
+    int E[2];
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      int e = kFxExZero;
+      if (mx[g] > 0.0) e = fx_expo(mx[g]);
+      E[g] = __reduce_max_sync(0xffffffffu, e);
+    }
+    if (lane < 2) ex[(r * NL + L) * 2 + lane] = (int16_t)(lane ? E[1] : E[0]);
+    for (int t = lane; t < m; t += 32) {
+      const int e = t / n;
+      const int g = (e / NB == e % NB) ? 0 : 1;
+      const int s = E[g] == kFxExZero ? 0 : kFxPBits - E[g];
+      const int2 x = fx_digits(p[t].x, s), y = fx_digits(p[t].y, s);
+      reinterpret_cast<int4*>(p)[t] = make_int4(x.x, x.y, y.x, y.y);
+    }
+  }
+}
+
+// Shared memory of a warp: a ring of two chunks of two lines; the row digits and the forward exponents -- of
+// every row block of the item for nb = 2 (lane r makes row block r's when the item starts), of the one at work
+// for nb = 4, whose row blocks are 4 times the work and digits; then zeros.
+template <int NB>
+struct FxSmem {
+  static constexpr int NB2 = NB * NB, G = NB2 / 4, W = 32 / G;
+  static constexpr bool kItemDigits = NB == 2;
+  static constexpr int stage_bytes = 2 * NB2 * W * 16;
+  static constexpr int row_bytes = NB2 * 16;  // a row block's digits: int4 (diagonal h, l, off-diagonal h, l) per line
+  static constexpr int dig = 2 * stage_bytes;
+  static constexpr int zero = dig + (kItemDigits ? kMaxRowBlocksPerItem : 1) * row_bytes;
+  static constexpr int exps = zero + row_bytes;
+  static constexpr int bars = exps + (kItemDigits ? kMaxRowBlocksPerItem * NB2 * 4 : 0);
+  static constexpr int warp_bytes = (bars + 16 + 127) / 128 * 128;
+  static constexpr size_t cta_bytes = 4 * (size_t)warp_bytes;
+};
+
+// a and b summed over the lane pairs that differ in `bit`: the lane with the bit clear gets a's sum
+__device__ __forceinline__ long long fx_merge(long long a, long long b, int bit, int lane) {
+  const bool up = lane & bit;
+  const long long keep = up ? b : a, send = up ? a : b;
+  return keep + __shfl_xor_sync(0xffffffffu, send, bit);
+}
+
+// FP64 contraction of one work item from the decoded elements (non-finite states), straight from global
+// memory: the sums of both parts of the state, with FP64 atomics per pair
+template <int NB>
+__device__ __noinline__ void fx_item_f64(const WorkItem w, const RowBlock* rbs, const int4* P, const int16_t* ex,
+                                         const double* rs0, size_t half, bool anti, double* acc, int nk, int lane) {
+  constexpr int NB2 = NB * NB, NB4 = NB2 * NB2, W = 128 / NB2, NL = 2 * NB2;
+  const int qg = lane / W, sl = lane % W, col = w.J * W + sl;
+  if (col >= nk) return;
+  for (int part = 0; part < (anti ? 2 : 1); ++part) {
+    const double* rs = rs0 + (part ? half : 0);
+    const double* rc = rs + (size_t)col * 2 * NB2;
+    for (int rb = w.rb0; rb < w.rb1; ++rb) {
+      const RowBlock b = rbs[rb];
+      if (!((b.mask >> sl) & 1u)) continue;
+      const bool rev = (b.revmask >> sl) & 1u;
+      const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << sl) - 1u));
+      const double* rr = rs + (size_t)b.row * 2 * NB2;
+      for (int L = 0; L < NL; ++L) {
+        const int m = L / NB2, a = L % NB2;
+        const double kr = m ? rr[a] : rr[NB2 + a];  // r_k[j] or s_k[a]
+        double fx = 0.0, fy = 0.0;
+        for (int i = 0; i < 4; ++i) {
+          const int e = 4 * qg + i;
+          const int g = (e / NB == e % NB) ? 0 : 1;
+          const int4 v = P[(size_t)b.pair0 * 2 * NB4 + ((size_t)L * NB2 + e) * n + slot];
+          const int x = ex[((size_t)rb * NL + L) * 2 + g];
+          const double px = fx_decode(v.x, v.y, x), py = fx_decode(v.z, v.w, x);
+          const double c = m ? rc[NB2 + e] : rc[e];
+          fx = fma(px, c, fx);
+          fy = fma(py, c, fy);
+          if (rev) {  // conj(p) times the row's coordinate, to the other sum of the column
+            const double vx = px * kr, vy = -py * kr;
+            double* d = acc + (size_t)col * 4 * NB2 + (m ? 0 : 2 * NB2) + 2 * e;
+            atomicAdd(d, part ? -vy : vx);
+            atomicAdd(d + 1, part ? vx : vy);
+          }
+        }
+        double* d = acc + (size_t)b.row * 4 * NB2 + 2 * L;
+        atomicAdd(d, part ? -fy : fx);
+        atomicAdd(d + 1, part ? fx : fy);
+      }
+    }
+  }
+}
+
+// One warp per work item and matrix (Q1 or Q2): lane (qg, sl) owns column W J + sl and the quarter qg of
+// every line. With both matrices in one warp the reverse sums and the column's digits took 168 registers and
+// left 12 warps per SM, too few to cover the multiply-adds' latency; one matrix fits 5 CTAs. Chunks of
+// two lines (4 KB) stream through a per-warp ring of two bulk copies. The forward sums (line, re | im,
+// group) are added over the warp by merging: each level of exchange halves the values, so that the
+// lane (group, re | im, line) ends with its total (a full reduction of each value takes five times the shuffles).
+template <int NB, int MINB, bool IMAG>
+__global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restrict__ items, int nitems,
+                                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P,
+                                                        const int16_t* __restrict__ ex, const double* __restrict__ rs0,
+                                                        size_t half, double* __restrict__ acc, int nk,
+                                                        const unsigned int* __restrict__ flag,
+                                                        unsigned int* __restrict__ errflag) {
+  typedef FxSmem<NB> S;
+  constexpr int NB2 = S::NB2, NB4 = NB2 * NB2, W = S::W;
+  constexpr int LF = NB == 2 ? 4 : 8;  // lines per forward flush
+  constexpr int NF = NB2 / LF;         // flushes per row block
+  constexpr int CPR = NB2 / 2;         // chunks (two lines) per row block
+  constexpr int RB = fx_row_bits(NB);
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const unsigned fl = *flag;
+  if (IMAG ? fl == 0u : (fl & DMD_HFLAG_NONFINITE) != 0u) return;
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * 4 + wib, item = task >> 1, m = task & 1;
+  if (item >= nitems) return;
+  const WorkItem w = items[item];
+  if (IMAG && (fl & DMD_HFLAG_NONFINITE)) {
+    if (m == 0) fx_item_f64<NB>(w, rbs, P, ex, rs0, half, (fl & DMD_HFLAG_NONHERM) != 0u, acc, nk, lane);
+    return;
+  }
+  const double* const rs = rs0 + (IMAG ? half : 0);
+  const int qg = lane / W, sl = lane % W;
+  unsigned char* const wbase = smem_raw + (size_t)wib * S::warp_bytes;
+  const uint32_t sbase = smem_u32(wbase);
+  uint64_t* const bar = (uint64_t*)(wbase + S::bars);
+  const int nrb = w.rb1 - w.rb0;  // <= kMaxRowBlocksPerItem = 32
+  RowBlock mine;                  // lane r: the item's row block r
+  mine.row = 0;
+  mine.mask = 0;
+  mine.revmask = 0;
+  mine.pair0 = 0;
+  if (lane < nrb) mine = rbs[w.rb0 + lane];
+  if (lane == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    fence_mbar_init();
+  }
+  // the column's coordinates: r for Q1's forward sums, s for Q2's; the rows': s for Q1, r for Q2
+  const int col = w.J * W + sl;
+  const int co = m ? NB2 : 0, ro = m ? 0 : NB2;
+  double cv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int b = NB == 2 ? i : 4 * qg + ((i + qg) & 3);
+    cv[i] = col < nk ? rs[(size_t)col * 2 * NB2 + co + b] : 0.0;
+  }
+  __syncwarp();
+  const uint64_t pol = policy_evict_first();
+  // address of a row block's lines of this matrix and bytes of a chunk of it (0 past the item's end)
+  const char* const mysrc = (const char*)(P + (size_t)mine.pair0 * 2 * NB4 + (size_t)m * NB4 * __popc(mine.mask));
+  const int mylen = 2 * NB2 * 16 * __popc(mine.mask);
+  auto copy = [&](const char* src, int len, int q) {  // chunk q of a row block into stage q % 2
+    if (lane == 0 && len > 0) {
+      mbar_arrive_expect_tx(&bar[q & 1], len);
+      bulk_g2s(wbase + (q & 1) * S::stage_bytes, src + (size_t)q * len, len, &bar[q & 1], pol);
+    }
+  };
+  const char* src = (const char*)__shfl_sync(FULL, (unsigned long long)mysrc, 0);
+  int len = __shfl_sync(FULL, mylen, 0);
+  copy(src, len, 0);
+  copy(src, len, 1);
+
+  // the largest row coordinate times its line's scale, per group: the reverse sums' exponents
+  int eS0 = -30000, eS1 = -30000;
+  const double* const rr = rs + (size_t)mine.row * 2 * NB2 + ro;
+  const short2* const xr = (const short2*)ex + ((size_t)(w.rb0 + (lane < nrb ? lane : 0)) * 2 + m) * NB2;
+  if (lane < nrb) {
+#pragma unroll 4
+    for (int a = 0; a < NB2; ++a) {
+      const int e = fx_expo(rr[a]);
+      const short2 x = xr[a];
+      eS0 = max(eS0, e + x.x);
+      eS1 = max(eS1, e + x.y);
+    }
+  }
+  eS0 = __reduce_max_sync(FULL, eS0);
+  eS1 = __reduce_max_sync(FULL, eS1);
+  const int lg = lane & 1, lri = (lane >> 1) & 1, ll = (lane >> 2) % LF;
+  int2 cd[4];  // the column's digits
+  int eR;      // their exponent, of this lane's group
+  {
+    int e[2] = {-900, -900};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e[fx_group<NB>(i)] = max(e[fx_group<NB>(i)], fx_expo(cv[i]));
+    e[0] = __reduce_max_sync(FULL, e[0]);
+    e[1] = __reduce_max_sync(FULL, e[1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cd[i] = fx_digits(cv[i], kFxCBits - e[fx_group<NB>(i)]);
+    eR = (lg ? e[1] : e[0]) + 2 * kFxBase - kFxPBits - kFxCBits;  // of the forward sums' unit
+  }
+  short exn[NF];   // nb = 4: lane (group, re | im, line of a flush): its lines' exponents and row coordinates,
+  double rown[NF]; // one row block ahead
+  auto fetch = [&](int rbi) {
+    const int row = __shfl_sync(FULL, mine.row, rbi);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      exn[f] = ex[(((size_t)(w.rb0 + rbi) * 2 + m) * NB2 + f * LF + ll) * 2 + lg];
+      rown[f] = rs[(size_t)row * 2 * NB2 + ro + f * LF + ll];
+    }
+  };
+  if constexpr (S::kItemDigits) {  // lanes (row block of 4, line, group)
+    const int a = (lane >> 1) & 3;
+    for (int r0 = 0; r0 < nrb; r0 += 4) {
+      const int r = r0 + (lane >> 3), row = __shfl_sync(FULL, mine.row, r & 31);
+      if (r < nrb) {
+        const short x = ex[(((size_t)(w.rb0 + r) * 2 + m) * NB2 + a) * 2 + lg];
+        ((int2*)(wbase + S::dig))[r * 8 + (lane & 7)] =
+            fx_digits(rs[(size_t)row * 2 * NB2 + ro + a], RB + x - (lg ? eS1 : eS0));
+        ((short*)(wbase + S::exps))[r * 8 + (lane & 7)] = x;
+      }
+    }
+  } else if (nrb > 0) {
+    fetch(0);
+  }
+  for (int i = lane; i < NB2; i += 32) ((int4*)(wbase + S::zero))[i] = make_int4(0, 0, 0, 0);
+  __syncwarp();
+
+  // the column's reverse sums [step][re | im]: B0 2^32 + Br, with the low products of four lines at work in B1
+  long long B0[4][2], B1[4][2];
+  unsigned Br[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) B0[i][0] = B0[i][1] = Br[i][0] = Br[i][1] = 0;
+  bool any_rev = false;
+  int cfail = -1;
+#pragma unroll 1
+  for (int rbi = 0; rbi < nrb; ++rbi) {
+    const int brow = __shfl_sync(FULL, mine.row, rbi);
+    const unsigned bmask = __shfl_sync(FULL, mine.mask, rbi);
+    const unsigned brev = __shfl_sync(FULL, mine.revmask, rbi);
+    const bool active = (bmask >> sl) & 1u, rev = (brev >> sl) & 1u;
+    any_rev |= rev;
+    const char* nsrc = (const char*)__shfl_sync(FULL, (unsigned long long)mysrc, (rbi + 1) & 31);
+    const int nlen = __shfl_sync(FULL, rbi + 1 < nrb ? mylen : 0, (rbi + 1) & 31);
+    short exv[NF];
+    if constexpr (S::kItemDigits) {
+      exv[0] = ((const short*)(wbase + S::exps))[(rbi * NB2 + ll) * 2 + lg];
+    } else {
+      __syncwarp();  // the previous row block's digits have been read
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        exv[f] = exn[f];
+        const int2 d = fx_digits(rown[f], RB + exv[f] - (lg ? eS1 : eS0));
+        if (lri == 0) ((int2*)(wbase + S::dig))[(f * LF + ll) * 2 + lg] = d;
+      }
+      if (rbi + 1 < nrb) fetch(rbi + 1);
+      __syncwarp();
+    }
+    // lanes without a reverse term read zero digits, lanes without a pair zero elements
+    const uint32_t dg = sbase + (rev ? S::dig + (S::kItemDigits ? rbi * S::row_bytes : 0) : S::zero);
+    const uint32_t ns = active ? __popc(bmask) * 16 : 0;
+    const uint32_t s0 = active ? sbase + __popc(bmask & ((1u << sl) - 1u)) * 16 : sbase + S::zero;
+    const uint32_t s1 = active ? s0 + S::stage_bytes : s0;
+    uint32_t eo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) eo[i] = (NB == 2 ? i : 4 * qg + ((i + qg) & 3)) * ns;
+
+    // one line: forward sums of the two groups, reverse sums; returns the lane's merged value (levels 1, 2)
+    auto line = [&](uint32_t sp, int L) -> long long {
+      const int4 rd = fx_lds(dg + L * 16);  // the row coordinate's digits for both groups
+      long long A0[2][2], A1[2][2];         // [group][re | im]; A1 starts at half of A0's unit
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        constexpr int gr[4] = {fx_group<NB>(0), fx_group<NB>(1), fx_group<NB>(2), fx_group<NB>(3)};
+        const int g = gr[i];
+        const int4 p = fx_lds(sp + eo[i]);
+        if (i < 2) {  // the first of its group
+          fx_mul(A0[g][0], A1[g][0], p.x, p.y, cd[i], 1LL << (kFxBase - 1));
+          fx_mul(A0[g][1], A1[g][1], p.z, p.w, cd[i], 1LL << (kFxBase - 1));
+        } else {
+          fx_mad(A0[g][0], A1[g][0], p.x, p.y, cd[i]);
+          fx_mad(A0[g][1], A1[g][1], p.z, p.w, cd[i]);
+        }
+        const int2 d = g ? make_int2(rd.z, rd.w) : make_int2(rd.x, rd.y);
+        fx_mad(B0[i][0], B1[i][0], p.x, p.y, d);
+        fx_mad(B0[i][1], B1[i][1], p.z, p.w, d);
+      }
+      long long t[2][2];
+#pragma unroll
+      for (int g = 0; g < 2; ++g)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) t[g][x] = A0[g][x] + (A1[g][x] >> kFxBase);
+      const long long re = fx_merge(t[0][0], t[1][0], 1, lane), im = fx_merge(t[0][1], t[1][1], 1, lane);
+      return fx_merge(re, im, 2, lane);
+    };
+    // the two lines of chunk q (level 3); false when the copy did not arrive
+    auto two = [&](int q, long long& v) -> bool {
+      const int c = rbi * CPR + q;
+      if (!__all_sync(FULL, mbar_wait_bounded(&bar[q & 1], (unsigned)(c >> 1) & 1u, errflag))) {
+        cfail = c;
+        return false;
+      }
+      const uint32_t sp = (q & 1) ? s1 : s0;
+      const long long v0 = line(sp, 2 * q), v1 = line(sp + NB2 * ns, 2 * q + 1);
+      // the stage is free once every lane has read it: order those reads before the next bulk copy into it
+      fence_proxy_async();
+      __syncwarp();
+      if (q + 2 < CPR) copy(src, len, q + 2);
+      else copy(nsrc, nlen, q + 2 - CPR);
+      v = fx_merge(v0, v1, 4, lane);
+      return true;
+    };
+    auto four = [&](int q, long long& v) -> bool {  // level 4, from chunk q on
+      long long a, b;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        B1[i][0] = Br[i][0];
+        B1[i][1] = Br[i][1];
+      }
+      if (!two(q, a) || !two(q + 1, b)) return false;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        Br[i][0] = fx_fold(B0[i][0], B1[i][0]);
+        Br[i][1] = fx_fold(B0[i][1], B1[i][1]);
+      }
+      v = fx_merge(a, b, 8, lane);
+      return true;
+    };
+    bool ok = true;
+#pragma unroll 1
+    for (int f = 0; f < NF; ++f) {
+      long long v, u;
+      if (!(ok = four(f * LF / 2, v))) break;
+      if constexpr (LF == 8) {
+        if (!(ok = four(f * LF / 2 + 2, u))) break;
+        v = fx_merge(v, u, 16, lane);
+      } else {
+        u = __shfl_xor_sync(FULL, v, 16);
+        v += u;
+      }
+      // the totals of the flush's lines to the row's sums (x i in the anti-Hermitian pass)
+      double d = fx_scale((double)v, (NF == 1 || f == 0 ? exv[0] : exv[NF - 1]) + eR);
+      d += __shfl_xor_sync(FULL, d, 1);
+      if (lg == 0 && lane < 4 * LF) {
+        double* dst = acc + (size_t)brow * 4 * NB2 + 2 * (m * NB2 + f * LF + ll);
+        if (IMAG) atomicAdd(dst + (lri ^ 1), lri ? -d : d);
+        else atomicAdd(dst + lri, d);
+      }
+    }
+    if (!ok) break;
+    src = nsrc;
+    len = nlen;
+  }
+  if (cfail >= 0) {  // drain the copies still in flight (bounded), then leave
+    if (lane == 0) {
+      const int clast = (cfail + 2 < CPR * nrb ? cfail + 2 : CPR * nrb) - 1;
+      for (int i = cfail; i <= clast; ++i) mbar_wait_bounded(&bar[i & 1], (unsigned)(i >> 1) & 1u, nullptr, 1u << 16);
+    }
+    __syncwarp();
+    return;
+  }
+  // the column block's sums (Y' from Q1, X' from Q2) through the now free first stage, so that a warp's
+  // reductions touch consecutive doubles (one lane per column would touch 32 sectors each)
+  if (__any_sync(FULL, any_rev)) {
+    double2* const out = (double2*)wbase + (size_t)sl * NB2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int b = NB == 2 ? i : 4 * qg + ((i + qg) & 3);
+      const int e = (fx_group<NB>(i) ? eS1 : eS0) + 2 * kFxBase - kFxPBits - RB;  // of B0's unit
+      double v[2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        // B0 2^32 + Br to 64 bits: below 2^46 with 16 bits of Br, else rounded to B0's unit
+        const int h = (int)(B0[i][x] >> 32);
+        const bool low = (unsigned)(h ^ (h >> 31)) < (1u << 14);
+        const long long q = low ? (long long)((unsigned long long)B0[i][x] << 16 | Br[i][x] >> 16) : B0[i][x] + (Br[i][x] >> 31);
+        v[x] = fx_scale((double)q, low ? e - 16 : e);
+      }
+      // conj(p): the imaginary sum has the opposite sign
+      out[b] = IMAG ? mk2(v[1], v[0]) : mk2(v[0], -v[1]);
+    }
+    __syncwarp();
+    constexpr int R = 2 * NB2;  // reals per column: consecutive lanes take consecutive reals of one or more columns
+    double* const dst = acc + (size_t)w.J * W * 4 * NB2 + (m ? 0 : R);
+#pragma unroll
+    for (int i = 0; i < W * R / 32; ++i) {
+      const int idx = i * 32 + lane, cc = idx / R;
+      if (w.J * W + cc < nk) atomicAdd(dst + (size_t)cc * 4 * NB2 + idx % R, ((const double*)wbase)[idx]);
+    }
+  }
+}
+
+}  // namespace dmd
