@@ -13,6 +13,7 @@
 #include "dmd_adjoint.cuh"
 #include "dmd_batched_tc.cuh"
 #include "dmd_ee.cuh"
+#include "dmd_finish.cuh"
 #include "dmd_gpu.h"
 #include "dmd_kernels.cuh"
 #include "dmd_layout.h"
@@ -59,7 +60,7 @@ struct dmd_handle {
   int nitems = 0;
   long long nrb = 0;
   unsigned int* d_err = nullptr;  // device error flags (bounded waits)
-  unsigned int* d_hflag = nullptr;  // set by the prep kernel when a state is not exactly Hermitian
+  unsigned int* d_hflag = nullptr;  // [4] one per RK4 stage (0 otherwise): set by the prep when a state is not exactly Hermitian
   double2* d_acc0 = nullptr;   // deviation form: contraction of diag(f_ref), position order [nk][2][nb2]
   double* d_fref = nullptr;    // deviation form: window occupations [nk][nb]
   double2* d_ph = nullptr;     // phases D_k(i, j) of the current evaluation [nk][nb2]
@@ -129,7 +130,9 @@ struct dmd_handle {
   double* d_f[8] = {nullptr};
   double obs_prefac[8] = {0};
   double t = 0;                // time of the device state
-  long long launches = 0;
+  long long launches = 0, step_launches = 0;  // step_launches: of the captured RK4 step
+  int eval = 0;                // flag in use: the stage of a fused RK4 step, 0 otherwise
+  long long version = 0;       // counts changes that a captured step does not follow (groups compare it)
   cudaGraphExec_t g_rk4 = nullptr;
   cudaGraphExec_t g_rk4_rec = nullptr;  // the RK4 step that also copies its stage inputs and sums to d_rec
   double2* d_rec = nullptr;             // [4][nstate] stage inputs, then [4][nk 2 nb^2] forward sums
@@ -285,7 +288,7 @@ void herm_pair_launches(dmd_handle* h, const typename A::relem* rs, size_t half)
       h->nrhs, cstride, 2 * cstride);
   k_pairs_herm<A, NB, L, NST, MB, true, RW, FA><<<g, 128, S::cta_bytes, h->st>>>(
       h->d_items, h->nitems, h->d_rb, (const typename A::elem*)h->d_P, rs + half, (double*)h->d_acc, h->nk,
-      h->d_hflag, h->d_err, h->nrhs, cstride, 2 * cstride);
+      h->d_hflag + h->eval, h->d_err, h->nrhs, cstride, 2 * cstride);
 }
 
 template <typename A, int NB, int L, int NST, int MB, int RW = 1, bool FA = false>
@@ -335,9 +338,9 @@ void fx_pair_launches(dmd_handle* h, size_t half) {
   const size_t smem = FxSmem<NB>::cta_bytes;
   const double* rs = (const double*)h->d_rs;
   k_pairs_fx<NB, kFxCtas, false><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
-                                                                   rs, half, (double*)h->d_acc, h->nk, h->d_hflag, h->d_err);
+                                                                   rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
   k_pairs_fx<NB, kFxCtas, true><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
-                                                                  rs, half, (double*)h->d_acc, h->nk, h->d_hflag, h->d_err);
+                                                                  rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
 }
 
 template <int NB>
@@ -424,8 +427,47 @@ int launch_finish(dmd_handle* h, FinishArgs a) {
       return DMD_OK;
     }
   }
+  if constexpr (NB == 2 || NB == 4) {
+    if (h->nbdm == NB && h->nrhs == 1) {  // one thread per element (k_finish per launch: 9-17 us at 96-500 k-points)
+      k_finish_el<NB, ArithF64, false><<<blocks_for((long long)h->nk * NB * NB, 32), 32, 0, h->st>>>(a, NextPrep());
+      h->launches++;
+      CKL();
+      return DMD_OK;
+    }
+  }
   if (h->nbdm == NB) k_finish<NB, NB><<<g, 128, 0, h->st>>>(a);
   else k_finish<NB><<<g, 128, 0, h->st>>>(a);
+  h->launches++;
+  CKL();
+  return DMD_OK;
+}
+
+// An RK4 step whose finishes prepare the next stage (k_finish_el): single states of the column-block forms, the
+// window the whole density matrix, operators that do not depend on the state
+bool fused_step(const dmd_handle* h) {
+  return h->use_cb && !h->use_tc && h->nrhs == 1 && h->nbdm == h->nb && !(h->ee_on && h->ee_every);
+}
+
+// finish of stage s (0..3) and coordinates of the next one (stage 3: of the next step's first stage)
+template <int NB>
+int launch_finish_prep(dmd_handle* h, FinishArgs a) {
+  ProfScope ps(h, 2);
+  NextPrep p;
+  p.rs = h->d_rs;
+  p.acc = h->d_acc;
+  p.acc0 = h->d_acc0;
+  p.ph = h->d_ph;
+  p.fref = (deviation_form(h->prec) || h->lin) ? h->d_fref : nullptr;
+  p.hflag = h->d_hflag + (a.stage + 1) % 4;
+  p.phase = h->expt;
+  p.lin = h->lin;
+  p.ta = a.ta;
+  p.ta.stage = (a.stage + 1) % 4;
+  p.ta.ahead = a.stage == 3 ? 1 : 0;
+  const unsigned g = blocks_for((long long)h->nk * NB * NB, 32);
+  if (h->prec == DMD_PREC_F64X) k_finish_el<NB, ArithDF, true><<<g, 32, 0, h->st>>>(a, p);
+  else if (deviation_form(h->prec)) k_finish_el<NB, ArithF32, true><<<g, 32, 0, h->st>>>(a, p);
+  else k_finish_el<NB, ArithF64, true><<<g, 32, 0, h->st>>>(a, p);
   h->launches++;
   CKL();
   return DMD_OK;
@@ -454,7 +496,7 @@ FinishArgs base_finish(dmd_handle* h, const double2* y) {
   a.pos = h->use_cb ? h->d_pos : nullptr;
   a.herm = h->use_cb;
   a.lin = h->lin;
-  a.hflag = h->use_cb ? h->d_hflag : nullptr;
+  a.hflag = h->use_cb ? h->d_hflag + h->eval : nullptr;
   a.nrhs = h->nrhs;
   a.sstride = h->nstate1;
   a.astride = (size_t)h->nk * 2 * h->nb2;
@@ -497,6 +539,7 @@ TimeArg time_value(double t) {
   ta.tref = nullptr;
   ta.step = nullptr;
   ta.stage = 0;
+  ta.ahead = 0;
   return ta;
 }
 
@@ -1369,6 +1412,7 @@ void drop_graphs(dmd_handle* h) {
   if (h->g_rk4) cudaGraphExecDestroy(h->g_rk4);
   if (h->g_rk4_rec) cudaGraphExecDestroy(h->g_rk4_rec);
   h->g_rk4 = h->g_rk4_rec = nullptr;
+  h->version++;
 }
 
 void release(dmd_handle* h) {
@@ -1754,7 +1798,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
       (rc = dalloc(h, &h->d_K, 6 * h->nstate)) || (rc = dalloc(h, &h->d_tref, 2)) ||
       (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_coef_i, 64)) ||
       (rc = dalloc(h, &h->d_coef, 64)) || (rc = dalloc(h, &h->d_flag, 1)) || (rc = dalloc(h, &h->d_err, 1)) ||
-      (rc = dalloc(h, &h->d_hflag, 1)) || (rc = dalloc(h, &h->d_ph, nk * h->nb2)))
+      (rc = dalloc(h, &h->d_hflag, 4)) || (rc = dalloc(h, &h->d_ph, nk * h->nb2)))
     return bail(rc);
   std::vector<double> ew(nk * h->nb);
   for (size_t k = 0; k < nk; ++k)
@@ -1787,7 +1831,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
   }
   if (cudaMemset(h->d_y, 0, h->nstate * 16) != cudaSuccess || cudaMemset(h->d_step, 0, 8) != cudaSuccess ||
       cudaMemset(h->d_err, 0, sizeof(unsigned int)) != cudaSuccess ||
-      cudaMemset(h->d_hflag, 0, sizeof(unsigned int)) != cudaSuccess)
+      cudaMemset(h->d_hflag, 0, 4 * sizeof(unsigned int)) != cudaSuccess)
     return bail(fail(h, DMD_E_CUDA, "init"));
   *out = h;
   return DMD_OK;
@@ -2087,13 +2131,16 @@ int dmd_get_state(dmd_handle* h, double* t, double* y) {
 // its forward sums (after the contraction) to recA[s].
 static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* recA = nullptr) {
   const size_t na = (size_t)h->nk * 2 * h->nb2;
+  const bool fused = fused_step(h);
   for (int s = 0; s < 4; ++s) {
     TimeArg ta;
     ta.t = 0;
     ta.tref = h->d_tref;
     ta.step = h->d_step;
     ta.stage = s;
+    ta.ahead = 0;
     const double2* in = (s == 0) ? h->d_y : h->d_ytmp;
+    h->eval = fused ? s : 0;
     FinishArgs fa = base_finish(h, in);
     fa.mode = 1;
     fa.stage = s;
@@ -2102,10 +2149,19 @@ static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* re
     fa.K = h->d_K;
     fa.ybase = h->d_y;
     fa.ytmp = h->d_ytmp;
+    fa.ta = ta;
     if (recU) CK(cudaMemcpyAsync(recU + (size_t)s * h->nstate, in, h->nstate * 16, cudaMemcpyDeviceToDevice, h->st));
-    int rc = rhs(h, in, ta, fa);
+    int rc;
+    if (fused) {  // the coordinates are there: from rk4_begin or the finish before
+      rc = h->nb == 2 ? launch_pairs<2>(h) : launch_pairs<4>(h);
+      if (!rc && recA) CK(cudaMemcpyAsync(recA + (size_t)s * na, h->d_acc, na * 16, cudaMemcpyDeviceToDevice, h->st));
+      if (!rc) rc = h->nb == 2 ? launch_finish_prep<2>(h, fa) : launch_finish_prep<4>(h, fa);
+      h->eval = 0;
+    } else {
+      rc = rhs(h, in, ta, fa);
+      if (!rc && recA) CK(cudaMemcpyAsync(recA + (size_t)s * na, h->d_acc, na * 16, cudaMemcpyDeviceToDevice, h->st));
+    }
     if (rc) return rc;
-    if (recA) CK(cudaMemcpyAsync(recA + (size_t)s * na, h->d_acc, na * 16, cudaMemcpyDeviceToDevice, h->st));
   }
   {
     ProfScope ps(h, 3);
@@ -2113,6 +2169,25 @@ static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* re
   }
   h->launches++;
   CKL();
+  return DMD_OK;
+}
+
+// before the first of a run of RK4 steps (d_tref, d_step set): the first stage's coordinates of a fused step
+static int rk4_begin(dmd_handle* h) {
+  if (!fused_step(h)) return DMD_OK;
+  CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
+  TimeArg ta;
+  ta.t = 0;
+  ta.tref = h->d_tref;
+  ta.step = h->d_step;
+  ta.stage = 0;
+  ta.ahead = 0;
+  return h->nb == 2 ? launch_prep<2>(h, h->d_y, ta) : launch_prep<4>(h, h->d_y, ta);
+}
+
+// after the last one: the coordinates prepared for a step that does not follow leave no flag behind
+static int rk4_end(dmd_handle* h) {
+  if (fused_step(h)) CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
   return DMD_OK;
 }
 
@@ -2126,6 +2201,8 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
   CK(cudaMemcpyAsync(h->d_step, &zero, 8, cudaMemcpyHostToDevice, h->st));
   // pageable sources: wait so the host values stay valid
   CK(cudaStreamSynchronize(h->st));
+  int rc0;
+  if ((rc0 = rk4_begin(h))) return rc0;
   if (h->prof_on) {  // one step at a time, events around every kernel
     for (int64_t s = 0; s < nsteps; ++s) {
       int rc = rk4_step_launches(h);
@@ -2134,6 +2211,7 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
       prof_harvest(h);
     }
     h->t = h->t + (double)nsteps * dt;
+    if ((rc0 = rk4_end(h))) return rc0;
     return check_state(h);
   }
   if (!h->g_rk4) {
@@ -2147,13 +2225,14 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
     e = cudaGraphInstantiate(&h->g_rk4, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(h, DMD_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+    h->step_launches = h->launches - l0;
     h->launches = l0;  // captured launches are counted when the graph runs
   }
-  const long long per_step = h->npair ? (h->use_tc ? 21 : h->use_cb ? 17 : 13) : 9;
   for (int64_t s = 0; s < nsteps; ++s) {
     CK(cudaGraphLaunch(h->g_rk4, h->st));
-    h->launches += per_step;
+    h->launches += h->step_launches;
   }
+  if ((rc0 = rk4_end(h))) return rc0;
   h->t = h->t + (double)nsteps * dt;  // = t0 + n*h as the stage times see it
   CK(cudaStreamSynchronize(h->st));
   return check_state(h);
@@ -2475,12 +2554,13 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
       e = cudaGraphInstantiate(&h->g_rk4_rec, g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return fail(h, DMD_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
+      h->step_launches = h->launches - l0;
       h->launches = l0;
     }
-    const long long per_step = h->npair ? (h->use_tc ? 21 : h->use_cb ? 17 : 13) : 9;
+    if ((rc = rk4_begin(h))) return rc;
     for (int64_t s = 0; s < nsteps; ++s) {
       CK(cudaGraphLaunch(h->g_rk4_rec, h->st));
-      h->launches += per_step;
+      h->launches += h->step_launches;
       CK(cudaMemcpyAsync(w.U + (size_t)s * 4 * n, h->d_rec, 4 * n * 16, cudaMemcpyDeviceToDevice, h->st));
       CK(cudaMemcpyAsync(w.A + (size_t)s * 4 * na, h->d_rec + 4 * n, 4 * na * 16, cudaMemcpyDeviceToDevice, h->st));
       for (; j < nobs && obs_step[j] == s + 1; ++j) {
@@ -2489,6 +2569,7 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
         if (s_obs) s_obs[j] = v;
       }
     }
+    if ((rc = rk4_end(h))) return rc;
     CK(cudaMemcpyAsync(h->d_y, ysave, n * 16, cudaMemcpyDeviceToDevice, h->st));
     h->t = tsave;
   }
@@ -2588,6 +2669,7 @@ struct dmd_group {
   cudaStream_t st = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<cudaEvent_t> ev;  // [0] fork, [1..n] joins
+  std::vector<long long> version, step_launches;  // of the members when the step was captured; launches per step
 };
 
 extern "C" {
@@ -2640,7 +2722,19 @@ int dmd_group_rk4(dmd_group* g, double dt, int64_t nsteps) {
         cudaStreamSynchronize(hm->st) != cudaSuccess)
       return fail(hm, DMD_E_CUDA, "group: time reference upload");
   }
+  std::vector<long long> version;
+  for (dmd_handle* hm : g->m) version.push_back(hm->version);
+  if (g->exec && version != g->version) {  // a member's kernels or buffers have changed since the capture
+    cudaGraphExecDestroy(g->exec);
+    g->exec = nullptr;
+  }
+  for (dmd_handle* hm : g->m) {
+    const int rc = rk4_begin(hm);
+    if (rc) return rc;
+    if (cudaStreamSynchronize(hm->st) != cudaSuccess) return fail(hm, DMD_E_CUDA, "group: first stage");
+  }
   if (!g->exec) {  // one step of every member as parallel branches of one graph
+    g->version = version;
     std::vector<long long> l0;
     for (dmd_handle* hm : g->m) l0.push_back(hm->launches);
     CK(cudaStreamBeginCapture(g->st, cudaStreamCaptureModeThreadLocal));
@@ -2666,16 +2760,21 @@ int dmd_group_rk4(dmd_group* g, double dt, int64_t nsteps) {
     e = cudaGraphInstantiate(&g->exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(h, DMD_E_CUDA, std::string("group graph instantiate: ") + cudaGetErrorString(e));
-    for (size_t i = 0; i < g->m.size(); ++i) g->m[i]->launches = l0[i];  // counted when the graph runs
+    g->step_launches.clear();
+    for (size_t i = 0; i < g->m.size(); ++i) {  // counted when the graph runs
+      g->step_launches.push_back(g->m[i]->launches - l0[i]);
+      g->m[i]->launches = l0[i];
+    }
   }
   for (int64_t s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(g->exec, g->st));
   CK(cudaStreamSynchronize(g->st));
   int rc = DMD_OK;
-  for (dmd_handle* hm : g->m) {
-    const long long per_step = hm->npair ? (hm->use_tc ? 21 : hm->use_cb ? 17 : 13) : 9;
-    hm->launches += per_step * nsteps;
+  for (size_t i = 0; i < g->m.size(); ++i) {
+    dmd_handle* hm = g->m[i];
+    hm->launches += g->step_launches[i] * nsteps;
     hm->t = hm->t + (double)nsteps * dt;
-    const int r = check_state(hm);
+    int r = rk4_end(hm);
+    if (!r) r = check_state(hm);
     if (r && !rc) rc = r;
   }
   return rc;

@@ -23,12 +23,13 @@ struct TimeArg {
   const double* tref;     // [t0, h]
   const long long* step;  // completed steps since t0
   int stage;
+  int ahead;              // steps beyond *step (the next step's first stage, prepared at the end of this one)
 };
 
 __device__ __forceinline__ double eval_time(const TimeArg& ta) {
   if (!ta.tref) return ta.t;
   const double t0 = ta.tref[0], h = ta.tref[1];
-  const double t = t0 + (double)(*ta.step) * h;
+  const double t = t0 + (double)(*ta.step + ta.ahead) * h;
   if (ta.stage == 0) return t;
   if (ta.stage == 3) return t + h;
   return t + 0.5 * h;

@@ -1,0 +1,77 @@
+"""The RK4 step whose finishes prepare the next stage (csrc/dmd_finish.cuh) against the same steps taken from the host
+through dmd_func, which prepares every evaluation by itself: the operations and their order per element are the same, so
+the states differ only by the order of the contraction's atomic sums. FP64 forms: 1e-13 of the state's change per
+evaluation and the roundings of the state itself, 1e-14; FP32 forms: their products' 2^-24 of the change, 1e-5."""
+import numpy as np
+import pytest
+
+from test_gpu_fixed_point import built, system  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def handle(s, prec, picture, expt, H):
+    from denmat_dynm_development_gb300.dmd import LindbladGPU
+    return LindbladGPU(nk=s.nk, nb_dm=s.nb_dm, bstart=0, bend=s.nb_dm, e_dm=s.e_dm, k1st=s.k1st, k2nd=s.k2nd, P1=s.P1,
+                       P2=s.P2, prefac_eph=s.prefac_eph, Hcoh=H, picture=picture, expt=expt, precision=prec, f_ref=s.f_dm)
+
+
+def host_rk4(g, t, h, n, y):
+    for _ in range(n):
+        k1 = g.func(t, y)
+        k2 = g.func(t + 0.5 * h, y + 0.5 * h * k1)
+        k3 = g.func(t + 0.5 * h, y + 0.5 * h * k2)
+        k4 = g.func(t + h, y + h * k3)
+        y = y + h / 6.0 * (k1 + 2.0 * k2 + 2.0 * k3 + k4)
+        t += h
+    return y
+
+
+@pytest.mark.parametrize("prec", ["f64", "f64x", "f32", "bf16x2"])
+@pytest.mark.parametrize("nb,nk", [(2, 1), (2, 37), (4, 5), (4, 33)])
+@pytest.mark.parametrize("picture,expt,with_H,herm", [(0, 1, False, True), (0, 1, True, False), (1, 0, True, True),
+                                                      (1, 1, False, False), (0, 0, True, True)])
+def test_fused_step(prec, nb, nk, picture, expt, with_H, herm, oracle, built):  # noqa: F811
+    s = system(oracle, nk, nb, 0.8, 11 * nk + nb)
+    rng = np.random.default_rng(3)
+    H = None
+    if with_H:
+        x = rng.standard_normal((nk, nb, nb)) + 1j * rng.standard_normal((nk, nb, nb))
+        H = 1e-4 * (x + np.conj(np.swapaxes(x, 1, 2)))
+    y = oracle.y_of(s.dm0)
+    if not herm:
+        y = y * (1.0 + 1e-2 * rng.standard_normal(y.size))
+    t0, h, n = 7.0 * oracle.fs, 2.0 * oracle.fs, 5
+    tol = 1e-5 if prec in ("f32", "bf16x2") else 1e-13
+    with handle(s, prec, picture, expt, H) as g:
+        ref = host_rk4(g, t0, h, n, y)
+        change = np.abs(ref - y).max()
+        for _ in range(2):  # a second run starts from its own state
+            g.set_state(t0, y)
+            g.rk4(h, 2)
+            g.rk4(h, n - 2)
+            out = g.get_state()[1]
+            assert np.abs(out - ref).max() <= tol * 4 * n * change + 1e-14 * np.abs(ref).max()
+        # the evaluation after it finds no flag or sum of the step that did not follow
+        a, b = g.func(t0, y), g.func(t0, y)
+        assert np.abs(a - b).max() <= tol * np.abs(b).max()
+
+
+def test_group_follows_a_change_of_a_member(oracle, built):  # noqa: F811
+    """a drift set after the group's first step is in its next one"""
+    from denmat_dynm_development_gb300.dmd import Group
+    s = system(oracle, 20, 2, 0.8, 5)
+    y, h = oracle.y_of(s.dm0), 1.0 * oracle.fs
+    with handle(s, "f64", 0, 1, None) as g, handle(s, "f64", 0, 1, None) as alone:
+        eq = 1e-6 * np.eye(2)[None].repeat(s.nk, 0).astype(np.complex128)
+        with Group([g]) as group:
+            g.set_state(0.0, y)
+            group.rk4(h, 1)
+            g.set_ddmdt_eq(eq)
+            group.rk4(h, 1)
+        alone.set_state(0.0, y)
+        alone.rk4(h, 1)
+        alone.set_ddmdt_eq(eq)
+        alone.rk4(h, 1)
+        a, b = g.get_state()[1], alone.get_state()[1]
+    assert np.abs(a - b).max() <= 1e-14 * np.abs(b).max()
