@@ -37,6 +37,7 @@ struct dmd_handle {
   double add_scale = 0;        // scale of the additive operators (P += add_scale P_add)
   PairSource* src = nullptr;   // set while creating from files: where the raw operators come from
   int picture = 0, expt = 1, prec = 0;
+  int fmt = 0;                 // arithmetic of the stored operators: prec, or F64 where the f64x form shares it
   size_t nstate = 0;  // complex elements of the state (nrhs * nk * nbdm^2)
   size_t nstate1 = 0; // complex elements of one state (nk * nbdm^2)
   int nrhs = 1;       // batched form: states sharing P
@@ -49,7 +50,6 @@ struct dmd_handle {
   // column-block layout (nb = 2)
   int use_cb = 0;
   int lin = 0;                 // linearized master equation (DMD_FLAG_LINEAR)
-  int pcfg = 0;                // pair-kernel shape variant of the f64x form (DMD_PAIR_CFG)
   int use_fx = 0;              // f64 form: operators in block-scaled fixed point (dmd_pairs_fx.cuh)
   int* d_rbJ = nullptr;        // column block of every row block (f64 form)
   int16_t* d_ex = nullptr;     // exponents of the fixed-point operators [row block][line][group]
@@ -254,7 +254,7 @@ int launch_prep(dmd_handle* h, const double2* y, const TimeArg& ta) {
     // batched form: a thread serves up to 8 states of its (k, element), so the phase is computed once
     const int qc = h->nrhs < 8 ? h->nrhs : 8;
     const dim3 g(blocks_for(n, 256), (h->nrhs + qc - 1) / qc);
-    if (h->prec == DMD_PREC_F64X)
+    if (h->fmt == DMD_PREC_F64X)
       k_prep_herm<ArithDF, NB><<<g, 256, 0, h->st>>>(h->nk, h->nbdm, h->bs, y, h->d_ew, h->d_inv, ta, h->expt,
                                                       (float2*)h->d_rs, h->d_acc, h->d_hflag, fref, h->d_acc0, h->lin,
                                                       h->nrhs, qc, h->d_ph, 1);
@@ -328,28 +328,27 @@ void tc_launches(dmd_handle* h, size_t half) {
   h->launches += 1;  // the packing launch; the two passes are counted with the other forms
 }
 
-// the f64 contraction in fixed point: the Hermitian pass and the gated pass (anti-Hermitian part,
-// non-finite states). Against the FP64-pipe form per launch: 0.235 and 0.80 ms on 2.5M nb = 2 pairs, 29 and
-// 73 us on 70k, 125 and 325 us on 46k nb = 4 pairs, so it takes every handle whose operators have the form
+// the f64 and f64x contraction in fixed point. Against the FP64-pipe form per launch: 0.224 and 0.80 ms on 2.5M
+// nb = 2 pairs, 29 and 73 us on 70k, 119 and 325 us on 46k nb = 4 pairs, so it takes every handle whose operators
+// have the form
 constexpr int kFxCtas = 4;
 template <int NB>
 void fx_pair_launches(dmd_handle* h, size_t half) {
   const unsigned g = blocks_for(2LL * h->nitems, 4);
-  const size_t smem = FxSmem<NB>::cta_bytes;
-  const double* rs = (const double*)h->d_rs;
-  k_pairs_fx<NB, kFxCtas, false><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
-                                                                   rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
-  k_pairs_fx<NB, kFxCtas, true><<<g, 128, smem, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex,
-                                                                  rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
+  auto pass = [&](auto k) {
+    k<<<g, 128, FxSmem<NB>::cta_bytes, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex, (const double*)h->d_rs,
+                                                half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
+  };
+  pass(k_pairs_fx<NB, kFxCtas, false>);
+  pass(k_pairs_fx<NB, kFxCtas, true>);
 }
 
 template <int NB>
 cudaError_t fx_attrs() {
   const int bytes = (int)FxSmem<NB>::cta_bytes;
-  cudaError_t e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
+  const cudaError_t e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  return e != cudaSuccess ? e
+                          : cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 template <int NB>
@@ -374,19 +373,8 @@ int launch_pairs(dmd_handle* h) {
         if (h->prec == DMD_PREC_BF16X2) herm_pair_launches<ArithBF2, NB, 4, 2, 2, 4>(h, rs, half);
         else if (h->brw == 8) herm_pair_launches<ArithF32, NB, 4, 2, 2, 8>(h, rs, half);
         else herm_pair_launches<ArithF32, NB, 4, 2, 2, 4>(h, rs, half);
-      } else if (h->prec == DMD_PREC_F64X) {
-        const float2* rs = (const float2*)h->d_rs;
-        if constexpr (NB == 4) {
-          herm_pair_launches<ArithDF, NB, 2, 2, 4>(h, rs, half);
-        } else {
-          switch (h->pcfg) {
-            case 1: herm_pair_launches<ArithDF, NB, 2, 3, 3>(h, rs, half); break;
-            case 2: herm_pair_launches<ArithDF, NB, 1, 4, 4>(h, rs, half); break;
-            case 3: herm_pair_launches<ArithDF, NB, 1, 3, 4>(h, rs, half); break;
-            case 4: herm_pair_launches<ArithDF, NB, 1, 6, 3>(h, rs, half); break;
-            default: herm_pair_launches<ArithDF, NB, 2, 2, 4>(h, rs, half); break;
-          }
-        }
+      } else if (h->fmt == DMD_PREC_F64X) {
+        herm_pair_launches<ArithDF, NB, 2, 2, 4>(h, (const float2*)h->d_rs, half);
       } else if (h->use_fx) {
         fx_pair_launches<NB>(h, half);
       } else if (h->prec == DMD_PREC_F32) {
@@ -465,7 +453,7 @@ int launch_finish_prep(dmd_handle* h, FinishArgs a) {
   p.ta.stage = (a.stage + 1) % 4;
   p.ta.ahead = a.stage == 3 ? 1 : 0;
   const unsigned g = blocks_for((long long)h->nk * NB * NB, 32);
-  if (h->prec == DMD_PREC_F64X) k_finish_el<NB, ArithDF, true><<<g, 32, 0, h->st>>>(a, p);
+  if (h->fmt == DMD_PREC_F64X) k_finish_el<NB, ArithDF, true><<<g, 32, 0, h->st>>>(a, p);
   else if (deviation_form(h->prec)) k_finish_el<NB, ArithF32, true><<<g, 32, 0, h->st>>>(a, p);
   else k_finish_el<NB, ArithF64, true><<<g, 32, 0, h->st>>>(a, p);
   h->launches++;
@@ -817,7 +805,7 @@ __global__ void k_cb_fill(long long p0, long long cnt, FillSrc src, double add_s
 // FP64-pipe contraction.
 int fx_convert(dmd_handle* h) {
   h->use_fx = 0;
-  if (h->prec != DMD_PREC_F64 || h->eek) return DMD_OK;
+  if (h->fmt != DMD_PREC_F64 || h->eek) return DMD_OK;
   const unsigned g = blocks_for(h->nrb, 4), gk = blocks_for(h->nk, 256);
   double* sc = (double*)h->d_acc;  // scratch: [nk][2], rewritten by every evaluation
   int bad = 0;
@@ -861,7 +849,7 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
     int nsm = 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
     const long long want = (long long)nsm * 16;
-    const bool fx = h->prec == DMD_PREC_F64 && !h->eek;
+    const bool fx = h->fmt == DMD_PREC_F64 && !h->eek;
     if (fx && h->npair * G * 2 / (32 * 32) > nsm * 5LL) ppi = 32 * 32 / G;
     else if (h->npair / ppi < want) ppi = (int)std::max<long long>(1, h->npair / want);
   }
@@ -869,12 +857,9 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
     return fail(h, DMD_E_ARG, "k-pair index out of range");
   h->nitems = (int)L.items.size();
   h->nrb = (long long)L.rb.size();
-  // pair-kernel shape (stage lines, resident CTAs per SM); 0 is the default, the others serve tuning
-  if (const char* v = getenv("DMD_PAIR_CFG")) h->pcfg = atoi(v);
   if (nb == 2) {
     cudaError_t (*const attrs[])() = {
-        herm_pair_attrs<ArithDF, 2, 2, 2, 4>, herm_pair_attrs<ArithDF, 2, 2, 3, 3>, herm_pair_attrs<ArithDF, 2, 1, 4, 4>,
-        herm_pair_attrs<ArithDF, 2, 1, 3, 4>, herm_pair_attrs<ArithDF, 2, 1, 6, 3>,
+        herm_pair_attrs<ArithDF, 2, 2, 2, 4>,
         herm_pair_attrs<ArithF64, 2, 2, 2, 4, 1, true>,
         herm_pair_attrs<ArithF32, 2, 4, 2, 5>, herm_pair_attrs<ArithBF2, 2, 4, 2, 5>,
         herm_pair_attrs<ArithF32, 2, 4, 2, 2, 4>, herm_pair_attrs<ArithF32, 2, 4, 2, 2, 8>,
@@ -898,13 +883,13 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   CK(cudaMemcpy(h->d_inv, L.inv.data(), L.inv.size() * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_rb, L.rb.data(), L.rb.size() * sizeof(dmd::RowBlock), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
-  if (h->prec == DMD_PREC_F64 && !h->eek) {
+  if (h->fmt == DMD_PREC_F64 && !h->eek) {
     std::vector<int> J(L.rb.size());
     for (const dmd::WorkItem& w : L.items) std::fill(J.begin() + w.rb0, J.begin() + w.rb1, w.J);
     if ((rc = dalloc(h, &h->d_rbJ, J.size()))) return rc;
     CK(cudaMemcpy(h->d_rbJ, J.data(), J.size() * 4, cudaMemcpyHostToDevice));
   }
-  const int esz = elem_bytes(h->prec);
+  const int esz = elem_bytes(h->fmt);
   // deviation form: the constant contraction of diag(f_ref), position order [nk][2][nb2]
   const bool dev = deviation_form(h->prec) && !h->lin;
   std::vector<double> fw;
@@ -951,7 +936,7 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
 // Streams the raw operators through two pinned chunks and the fill kernel: the host reads chunk
 // c + 1 while the device converts chunk c.
 int fill_pairs_cb(dmd_handle* h, PairSource& src, const std::vector<CbDst>& dst, bool dev) {
-  const int nb4 = h->nb4, esz = elem_bytes(h->prec);
+  const int nb4 = h->nb4, esz = elem_bytes(h->fmt);
   const int nseg = src.has_add() ? 4 : 2;
   const size_t per_pair = (size_t)nseg * nb4 * 16;
   long long chunk = std::max<long long>(1, std::min<long long>(h->npair, (256LL << 20) / (long long)per_pair));
@@ -999,10 +984,10 @@ int fill_pairs_cb(dmd_handle* h, PairSource& src, const std::vector<CbDst>& dst,
     const size_t nn = (size_t)cnt * nb4;
     const FillSrc fs = {dev_raw[b], nn, (size_t)nb4, src.has_add() ? dev_raw[b] + 2 * nn : nullptr, nn, (size_t)nb4};
     if (h->nb == 2)
-      k_cb_fill<2><<<g, 128, 0, h->st>>>(p0, cnt, fs, h->add_scale, d_dst, h->lin, h->prec, esz,
+      k_cb_fill<2><<<g, 128, 0, h->st>>>(p0, cnt, fs, h->add_scale, d_dst, h->lin, h->fmt, esz,
                                          (unsigned char*)h->d_P, h->d_fref, a0);
     else
-      k_cb_fill<4><<<g, 128, 0, h->st>>>(p0, cnt, fs, h->add_scale, d_dst, h->lin, h->prec, esz,
+      k_cb_fill<4><<<g, 128, 0, h->st>>>(p0, cnt, fs, h->add_scale, d_dst, h->lin, h->fmt, esz,
                                          (unsigned char*)h->d_P, h->d_fref, a0);
     e = cudaGetLastError();
     if (e != cudaSuccess) break;
@@ -1481,7 +1466,7 @@ int ee_rebuild(dmd_handle* h, const double2* y, const TimeArg& ta, bool eq) {
     return fail(h, DMD_E_CUDA, "e-e refill");
   const FillSrc fs = {h->d_Praw, (size_t)NB4, (size_t)2 * NB4, h->d_ee_Pee, (size_t)NB4, (size_t)2 * NB4};
   k_cb_fill<NB><<<blocks_for(h->npair, 128), 128, 0, h->st>>>(0, h->npair, fs, h->ee_scale, (const CbDst*)h->d_dst,
-                                                              h->lin, h->prec, elem_bytes(h->prec),
+                                                              h->lin, h->fmt, elem_bytes(h->fmt),
                                                               (unsigned char*)h->d_P, h->d_fref,
                                                               dev ? (double*)h->d_acc0 : nullptr);
   h->launches += eq ? 3 : 4;
@@ -1766,6 +1751,10 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
   h->lin = (d->flags & DMD_FLAG_LINEAR) ? 1 : 0;
   h->adj = (d->flags & DMD_FLAG_ADJOINT) ? 1 : 0;
   h->eek = (d->flags & DMD_FLAG_EE) ? 1 : 0;
+  // the f64x form's operators are the f64 form's: the fixed-point contraction is the faster and the more exact
+  // one (2.5M nb = 2 pairs 224 against 279 us per launch, 9.9M 730 against 792, 70k 29 against 45; 177k nb = 4
+  // pairs 310 against 351). Double-floats remain where the e-e model rewrites the operators before every evaluation
+  h->fmt = (h->prec == DMD_PREC_F64X && !h->eek) ? DMD_PREC_F64 : h->prec;
   h->use_sp = (d->flags & DMD_FLAG_SPARSE) ? 1 : 0;
   h->nrhs = nrhs;
   h->nstate1 = (size_t)h->nk * h->nbdm * h->nbdm;
@@ -1790,7 +1779,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
   const size_t nk = h->nk, nbdm = h->nbdm;
   if ((rc = dalloc(h, &h->d_ew, nk * h->nb)) || (rc = dalloc(h, &h->d_edm, nk * nbdm)) ||
       (rc = dalloc(h, &h->d_kk, (h->nb == 2 || h->nb == 4 || h->use_sp) ? 1 : (size_t)h->npair)) ||
-      (rc = dalloc(h, &h->d_P, (h->use_tc || h->use_sp) ? 1 : ((size_t)h->npair * 2 * h->nb4 * elem_bytes(h->prec) + 15) / 16)) ||
+      (rc = dalloc(h, &h->d_P, (h->use_tc || h->use_sp) ? 1 : ((size_t)h->npair * 2 * h->nb4 * elem_bytes(h->fmt) + 15) / 16)) ||
       (rc = dalloc(h, &h->d_rs, nk * 2 * h->nb2 * nrhs)) || (rc = dalloc(h, &h->d_acc, nk * 2 * h->nb2 * nrhs)) ||
       (rc = dalloc(h, &h->d_y, h->nstate)) || (rc = dalloc(h, &h->d_ytmp, h->nstate)) ||
       (rc = dalloc(h, &h->d_y0, h->nstate)) || (rc = dalloc(h, &h->d_in, h->nstate)) ||
@@ -1813,7 +1802,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
   }
   h->use_cb = ((h->nb == 2 || h->nb == 4) && h->npair > 0 && !h->use_sp) ? 1 : 0;
   if (!h->use_tc)
-    h->pair_bytes = h->use_cb ? (int64_t)h->npair * 2 * h->nb4 * elem_bytes(h->prec) : (int64_t)h->npair * 2 * h->nb4 * 16;
+    h->pair_bytes = h->use_cb ? (int64_t)h->npair * 2 * h->nb4 * elem_bytes(h->fmt) : (int64_t)h->npair * 2 * h->nb4 * 16;
   if (src && !h->use_sp && (!h->use_cb || h->use_tc || h->adj))
     return bail(fail(h, DMD_E_ARG, "streamed operators need the column-block or the sparse form"));
   if (h->eek && (!h->use_cb || h->use_tc || h->nrhs != 1 || h->lin || src || h->adj))
@@ -2922,10 +2911,10 @@ int dmd_add_operators(dmd_handle* h, const double* P1_add, const double* P2_add,
   const FillSrc fs = {h->d_Praw, nb4, 2 * nb4, nullptr, 0, 0};
   const unsigned g = blocks_for(h->npair, 128);
   if (h->nb == 2)
-    k_cb_fill<2><<<g, 128, 0, h->st>>>(0, h->npair, fs, 0.0, (const CbDst*)h->d_dst, 0, h->prec, elem_bytes(h->prec),
+    k_cb_fill<2><<<g, 128, 0, h->st>>>(0, h->npair, fs, 0.0, (const CbDst*)h->d_dst, 0, h->fmt, elem_bytes(h->fmt),
                                        (unsigned char*)h->d_P, h->d_fref, dev ? (double*)h->d_acc0 : nullptr);
   else
-    k_cb_fill<4><<<g, 128, 0, h->st>>>(0, h->npair, fs, 0.0, (const CbDst*)h->d_dst, 0, h->prec, elem_bytes(h->prec),
+    k_cb_fill<4><<<g, 128, 0, h->st>>>(0, h->npair, fs, 0.0, (const CbDst*)h->d_dst, 0, h->fmt, elem_bytes(h->fmt),
                                        (unsigned char*)h->d_P, h->d_fref, dev ? (double*)h->d_acc0 : nullptr);
   h->launches += 1 + (h->npair + chunk - 1) / chunk;
   CKL();
@@ -2949,10 +2938,7 @@ int dmd_autotune(dmd_handle* h, int evals, int* chosen) {
   // candidate shapes of this handle's contraction
   std::vector<int> cand;
   int* knob = nullptr;
-  if (h->use_cb && !h->use_tc && h->nrhs == 1 && h->prec == DMD_PREC_F64X && h->nb == 2) {
-    cand = {0, 1, 2, 3, 4};
-    knob = &h->pcfg;
-  } else if (h->use_cb && !h->use_tc && h->nrhs > 1 && h->prec == DMD_PREC_F32) {
+  if (h->use_cb && !h->use_tc && h->nrhs > 1 && h->prec == DMD_PREC_F32) {
     cand = {4, 8};
     knob = &h->brw;
   } else if (h->use_tc) {

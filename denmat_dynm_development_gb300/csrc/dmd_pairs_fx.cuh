@@ -27,10 +27,10 @@
 // block and value (the FP64 kernel issues one per pair and value). Reverse sums keep A1's remainder and are exact
 // to the end of the item.
 //
-// A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, this kernel
-// returns and the gated launch (which otherwise carries the anti-Hermitian part of a non-Hermitian
-// state, bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do
-// in FP64. Operators with a non-finite element are never converted (dmd_api.cu).
+// A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, the first
+// launch returns and the gated one (which otherwise carries the anti-Hermitian part of a state that is not Hermitian,
+// bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do in FP64. Operators
+// with a non-finite element are never converted (dmd_api.cu).
 #pragma once
 #include <type_traits>
 
@@ -193,6 +193,10 @@ __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlo
   }
 }
 
+// bytes between the (line, re | im) rows of a chunk's forward sums: 32 lanes of 16 bytes and 64 more, so that the
+// 32 8-byte reads of a step fall on all banks twice
+constexpr int kFxFwdStride = 32 * 16 + 64;
+
 // Shared memory of a warp: a ring of two chunks of two lines; the row digits and the forward exponents -- of
 // every row block of the item for nb = 2 (lane r makes row block r's when the item starts), of the one at work
 // for nb = 4, whose row blocks are 4 times the work and digits; then zeros.
@@ -205,7 +209,8 @@ struct FxSmem {
   static constexpr int dig = 2 * stage_bytes;
   static constexpr int zero = dig + (kItemDigits ? kMaxRowBlocksPerItem : 1) * row_bytes;
   static constexpr int exps = zero + row_bytes;
-  static constexpr int bars = exps + (kItemDigits ? kMaxRowBlocksPerItem * NB2 * 4 : 0);
+  static constexpr int fwd = exps + (kItemDigits ? kMaxRowBlocksPerItem * NB2 * 4 : 0);  // forward sums of a chunk
+  static constexpr int bars = fwd + 4 * kFxFwdStride;
   static constexpr int warp_bytes = (bars + 16 + 127) / 128 * 128;
   static constexpr size_t cta_bytes = 4 * (size_t)warp_bytes;
 };
@@ -266,15 +271,14 @@ __device__ __noinline__ void fx_item_f64(const WorkItem w, const RowBlock* rbs, 
 // every line. With both matrices in one warp the reverse sums and the column's digits took 168 registers and
 // left 12 warps per SM, too few to cover the multiply-adds' latency; one matrix fits 5 CTAs. Chunks of
 // two lines (4 KB) stream through a per-warp ring of two bulk copies. The forward sums (line, re | im,
-// group) are added over the warp by merging: each level of exchange halves the values, so that the
-// lane (group, re | im, line) ends with its total (a full reduction of each value takes five times the shuffles).
-template <int NB, int MINB, bool IMAG>
-__global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restrict__ items, int nitems,
-                                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P,
-                                                        const int16_t* __restrict__ ex, const double* __restrict__ rs0,
-                                                        size_t half, double* __restrict__ acc, int nk,
-                                                        const unsigned int* __restrict__ flag,
-                                                        unsigned int* __restrict__ errflag) {
+// group) of a chunk are added over the warp through shared memory, 8 lanes' entries by each lane, and the two
+// bits of lanes that remain by exchanges that halve the values, so that lane (group, re | im, line) ends with its
+// total. (Exchanges alone, 8 instructions per value and level, took a sixth of the kernel's instructions.)
+template <int NB, bool IMAG>
+__device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkItem w, const int m, const RowBlock* __restrict__ rbs,
+                                        const int4* __restrict__ P, const int16_t* __restrict__ ex,
+                                        const double* __restrict__ rs, double* __restrict__ acc, int nk, int lane,
+                                        unsigned int* __restrict__ errflag) {
   typedef FxSmem<NB> S;
   constexpr int NB2 = S::NB2, NB4 = NB2 * NB2, W = S::W;
   constexpr int LF = NB == 2 ? 4 : 8;  // lines per forward flush
@@ -282,20 +286,7 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
   constexpr int CPR = NB2 / 2;         // chunks (two lines) per row block
   constexpr int RB = fx_row_bits(NB);
   constexpr unsigned FULL = 0xffffffffu;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const unsigned fl = *flag;
-  if (IMAG ? fl == 0u : (fl & DMD_HFLAG_NONFINITE) != 0u) return;
-  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int task = blockIdx.x * 4 + wib, item = task >> 1, m = task & 1;
-  if (item >= nitems) return;
-  const WorkItem w = items[item];
-  if (IMAG && (fl & DMD_HFLAG_NONFINITE)) {
-    if (m == 0) fx_item_f64<NB>(w, rbs, P, ex, rs0, half, (fl & DMD_HFLAG_NONHERM) != 0u, acc, nk, lane);
-    return;
-  }
-  const double* const rs = rs0 + (IMAG ? half : 0);
   const int qg = lane / W, sl = lane % W;
-  unsigned char* const wbase = smem_raw + (size_t)wib * S::warp_bytes;
   const uint32_t sbase = smem_u32(wbase);
   uint64_t* const bar = (uint64_t*)(wbase + S::bars);
   const int nrb = w.rb1 - w.rb0;  // <= kMaxRowBlocksPerItem = 32
@@ -425,12 +416,14 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
     const uint32_t ns = active ? __popc(bmask) * 16 : 0;
     const uint32_t s0 = active ? sbase + __popc(bmask & ((1u << sl) - 1u)) * 16 : sbase + S::zero;
     const uint32_t s1 = active ? s0 + S::stage_bytes : s0;
+    // forward sums: lane reads value lane % 8 of lanes 4 k + lane / 8
+    const uint32_t fsum = sbase + S::fwd + ((lane >> 1) & 3) * kFxFwdStride + (lane >> 3) * 16 + (lane & 1) * 8;
     uint32_t eo[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) eo[i] = (NB == 2 ? i : 4 * qg + ((i + qg) & 3)) * ns;
 
-    // one line: forward sums of the two groups, reverse sums; returns the lane's merged value (levels 1, 2)
-    auto line = [&](uint32_t sp, int L) -> long long {
+    // one line: forward sums of the two groups (to the chunk's buffer), reverse sums
+    auto line = [&](uint32_t sp, int L) {
       const int4 rd = fx_lds(dg + L * 16);  // the row coordinate's digits for both groups
       long long A0[2][2], A1[2][2];         // [group][re | im]; A1 starts at half of A0's unit
 #pragma unroll
@@ -449,15 +442,16 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
         fx_mad(B0[i][0], B1[i][0], p.x, p.y, d);
         fx_mad(B0[i][1], B1[i][1], p.z, p.w, d);
       }
-      long long t[2][2];
 #pragma unroll
-      for (int g = 0; g < 2; ++g)
-#pragma unroll
-        for (int x = 0; x < 2; ++x) t[g][x] = A0[g][x] + (A1[g][x] >> kFxBase);
-      const long long re = fx_merge(t[0][0], t[1][0], 1, lane), im = fx_merge(t[0][1], t[1][1], 1, lane);
-      return fx_merge(re, im, 2, lane);
+      for (int x = 0; x < 2; ++x) {
+        const long long t0 = A0[0][x] + (A1[0][x] >> kFxBase), t1 = A0[1][x] + (A1[1][x] >> kFxBase);
+        asm volatile("st.shared.v2.s64 [%0], {%1, %2};" ::"r"(sbase + S::fwd + lane * 16 + ((L & 1) * 2 + x) * kFxFwdStride),
+                     "l"(t0), "l"(t1)
+                     : "memory");
+      }
     };
-    // the two lines of chunk q (level 3); false when the copy did not arrive
+    // the two lines of chunk q: lane (part of 4, line, re | im, group) returns its value's sum over 8 lanes;
+    // false when the copy did not arrive
     auto two = [&](int q, long long& v) -> bool {
       const int c = rbi * CPR + q;
       if (!__all_sync(FULL, mbar_wait_bounded(&bar[q & 1], (unsigned)(c >> 1) & 1u, errflag))) {
@@ -465,16 +459,24 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
         return false;
       }
       const uint32_t sp = (q & 1) ? s1 : s0;
-      const long long v0 = line(sp, 2 * q), v1 = line(sp + NB2 * ns, 2 * q + 1);
+      line(sp, 2 * q);
+      line(sp + NB2 * ns, 2 * q + 1);
       // the stage is free once every lane has read it: order those reads before the next bulk copy into it
       fence_proxy_async();
       __syncwarp();
       if (q + 2 < CPR) copy(src, len, q + 2);
       else copy(nsrc, nlen, q + 2 - CPR);
-      v = fx_merge(v0, v1, 4, lane);
+      v = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        long long o;
+        asm volatile("ld.shared.s64 %0, [%1];" : "=l"(o) : "r"(fsum + k * 64));
+        v += o;
+      }
+      __syncwarp();
       return true;
     };
-    auto four = [&](int q, long long& v) -> bool {  // level 4, from chunk q on
+    auto four = [&](int q, long long& v) -> bool {  // two chunks from q on, merged over the parts' first bit
       long long a, b;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
   if (cfail >= 0) {  // drain the copies still in flight (bounded), then leave
     if (lane == 0) {
       const int clast = (cfail + 2 < CPR * nrb ? cfail + 2 : CPR * nrb) - 1;
-      for (int i = cfail; i <= clast; ++i) mbar_wait_bounded(&bar[i & 1], (unsigned)(i >> 1) & 1u, nullptr, 1u << 16);
+      for (int i = cfail; i <= clast; ++i)  mbar_wait_bounded(&bar[i & 1], (unsigned)(i >> 1) & 1u, nullptr, 1u << 16);
     }
     __syncwarp();
     return;
@@ -552,6 +554,31 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
       if (w.J * W + cc < nk) atomicAdd(dst + (size_t)cc * 4 * NB2 + idx % R, ((const double*)wbase)[idx]);
     }
   }
+}
+
+// IMAG: the gated launch behind every evaluation's first one, for the anti-Hermitian part (sums times i) and for
+// non-finite states. It costs 2.5 us where there is nothing to do; in the same launch, as a second pass of the warp or
+// as blocks that return at once, it cost the pass that always runs 3 to 50 % from 400k pairs on.
+template <int NB, int MINB, bool IMAG>
+__global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restrict__ items, int nitems,
+                                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P,
+                                                        const int16_t* __restrict__ ex, const double* __restrict__ rs,
+                                                        size_t half, double* __restrict__ acc, int nk,
+                                                        const unsigned int* __restrict__ flag,
+                                                        unsigned int* __restrict__ errflag) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const unsigned fl = *flag;
+  if (IMAG ? fl == 0u : (fl & DMD_HFLAG_NONFINITE) != 0u) return;
+  const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * 4 + wib, item = task >> 1, m = task & 1;
+  if (item >= nitems) return;
+  const WorkItem w = items[item];
+  if (IMAG && (fl & DMD_HFLAG_NONFINITE)) {
+    if (m == 0) fx_item_f64<NB>(w, rbs, P, ex, rs, half, (fl & DMD_HFLAG_NONHERM) != 0u, acc, nk, lane);
+    return;
+  }
+  fx_item<NB, IMAG>(smem_raw + (size_t)wib * FxSmem<NB>::warp_bytes, w, m, rbs, P, ex, rs + (IMAG ? half : 0), acc, nk, lane,
+                    errflag);
 }
 
 }  // namespace dmd

@@ -52,7 +52,9 @@ extern "C" {
                               below those of FP64 multiply-adds. Operators without that form (a non-finite
                               element, k-points coupled 2^-8 of their neighbours' strength or less) and handles with
                               DMD_FLAG_EE keep complex128 and FP64 multiply-adds */
-#define DMD_PREC_F64X 1    /* P and rho as (hi, lo) FP32 pairs: ~2^-46 products, double-FP32 sums */
+#define DMD_PREC_F64X 1    /* as DMD_PREC_F64 for the contraction (nb = 2, 4); the adjoint's backward pass and, with
+                              DMD_FLAG_EE, the contraction and the e-e rebuild use (hi, lo) FP32 pairs: ~2^-46
+                              products, double-FP32 sums */
 #define DMD_PREC_F32 2     /* P stored complex64, FP32 products; rho enters as its deviation from f_ref */
 #define DMD_PREC_BF16X2 3  /* P stored as bf16 hi + bf16 lo per component (8 bytes per complex), FP32
                               products; rho enters as its deviation from f_ref */
@@ -289,8 +291,7 @@ int dmd_ee_linear_terms(dmd_handle* h, const double* f_eq, double nfree, double*
 int dmd_ee_read(dmd_handle* h, double* P1ee, double* P2ee, double* nfree);
 
 /* No counterpart in the reference. Shape autotuner: times every compiled shape variant of the
- * handle's contraction (f64x, nb = 2: lines per stage, ring depth, CTAs per SM; CUDA-core batches:
- * states per warp; tensor-core batches: pipeline stages, 2 of which leave room for 2 CTAs per SM) on
+ * handle's contraction (CUDA-core batches: states per warp; tensor-core batches: pipeline stages, 2 of which leave room for 2 CTAs per SM) on
  * `evals` right-hand-side evaluations of the current device state (CUDA events,
  * after one warm-up evaluation each), keeps the fastest and returns its index in *chosen (0 when
  * the handle's form has a single shape). The state is not modified. */
