@@ -123,8 +123,6 @@ struct dmd_handle {
   double* d_tref = nullptr;    // [t0, h]
   long long* d_step = nullptr;
   double* d_red = nullptr;     // reduction partials
-  int* d_coef_i = nullptr;     // RKF45 coefficient tables
-  double* d_coef = nullptr;
   int* d_flag = nullptr;
   double2* d_obs[8] = {nullptr};
   double* d_f[8] = {nullptr};
@@ -256,7 +254,7 @@ int launch_prep(dmd_handle* h, const double2* y, const TimeArg& ta) {
     const dim3 g(blocks_for(n, 256), (h->nrhs + qc - 1) / qc);
     if (h->fmt == DMD_PREC_F64X)
       k_prep_herm<ArithDF, NB><<<g, 256, 0, h->st>>>(h->nk, h->nbdm, h->bs, y, h->d_ew, h->d_inv, ta, h->expt,
-                                                      (float2*)h->d_rs, h->d_acc, h->d_hflag, fref, h->d_acc0, h->lin,
+                                                      (float2*)h->d_rs, h->d_acc, h->d_hflag + h->eval, fref, h->d_acc0, h->lin,
                                                       h->nrhs, qc, h->d_ph, 1);
     else if (h->use_tc)  // one thread per (rank, state chunk) for the tensor-core form
       k_prep_tc<NB><<<dim3(blocks_for(h->nk, 128), (h->nrhs + qc - 1) / qc), 128, 0, h->st>>>(
@@ -264,11 +262,11 @@ int launch_prep(dmd_handle* h, const double2* y, const TimeArg& ta) {
           (float2*)h->d_ph);
     else if (deviation_form(h->prec))
       k_prep_herm<ArithF32, NB><<<g, 256, 0, h->st>>>(h->nk, h->nbdm, h->bs, y, h->d_ew, h->d_inv, ta, h->expt,
-                                                       (float*)h->d_rs, h->use_tc ? nullptr : h->d_acc, h->d_hflag,
+                                                       (float*)h->d_rs, h->use_tc ? nullptr : h->d_acc, h->d_hflag + h->eval,
                                                        fref, h->d_acc0, h->lin, h->nrhs, qc, h->d_ph, h->use_tc ? 0 : 1);
     else
       k_prep_herm<ArithF64, NB><<<g, 256, 0, h->st>>>(h->nk, h->nbdm, h->bs, y, h->d_ew, h->d_inv, ta, h->expt,
-                                                       (double*)h->d_rs, h->d_acc, h->d_hflag, fref, h->d_acc0, h->lin,
+                                                       (double*)h->d_rs, h->d_acc, h->d_hflag + h->eval, fref, h->d_acc0, h->lin,
                                                        h->nrhs, qc, h->d_ph, 1);
   }
   h->launches++;
@@ -417,7 +415,7 @@ int launch_finish(dmd_handle* h, FinishArgs a) {
   }
   if constexpr (NB == 2 || NB == 4) {
     if (h->nbdm == NB && h->nrhs == 1) {  // one thread per element (k_finish per launch: 9-17 us at 96-500 k-points)
-      k_finish_el<NB, ArithF64, false><<<blocks_for((long long)h->nk * NB * NB, 32), 32, 0, h->st>>>(a, NextPrep());
+      k_finish_el<NB, ArithF64, false><<<blocks_for((long long)h->nk * NB * NB, 32), 32, 0, h->st>>>(a, NextPrep(), RkfStage());
       h->launches++;
       CKL();
       return DMD_OK;
@@ -436,9 +434,10 @@ bool fused_step(const dmd_handle* h) {
   return h->use_cb && !h->use_tc && h->nrhs == 1 && h->nbdm == h->nb && !(h->ee_on && h->ee_every);
 }
 
-// finish of stage s (0..3) and coordinates of the next one (stage 3: of the next step's first stage)
+// the finish of a stage, with the coordinates of the next evaluation: at time ta, behind flag `eval`; rkf: a stage of
+// the RKF45 step instead of RK4's
 template <int NB>
-int launch_finish_prep(dmd_handle* h, FinishArgs a) {
+int launch_finish_prep(dmd_handle* h, const FinishArgs& a, const TimeArg& ta, int eval, const RkfStage* rkf) {
   ProfScope ps(h, 2);
   NextPrep p;
   p.rs = h->d_rs;
@@ -446,16 +445,19 @@ int launch_finish_prep(dmd_handle* h, FinishArgs a) {
   p.acc0 = h->d_acc0;
   p.ph = h->d_ph;
   p.fref = (deviation_form(h->prec) || h->lin) ? h->d_fref : nullptr;
-  p.hflag = h->d_hflag + (a.stage + 1) % 4;
+  p.hflag = h->d_hflag + eval;
   p.phase = h->expt;
   p.lin = h->lin;
-  p.ta = a.ta;
-  p.ta.stage = (a.stage + 1) % 4;
-  p.ta.ahead = a.stage == 3 ? 1 : 0;
+  p.ta = ta;
   const unsigned g = blocks_for((long long)h->nk * NB * NB, 32);
-  if (h->fmt == DMD_PREC_F64X) k_finish_el<NB, ArithDF, true><<<g, 32, 0, h->st>>>(a, p);
-  else if (deviation_form(h->prec)) k_finish_el<NB, ArithF32, true><<<g, 32, 0, h->st>>>(a, p);
-  else k_finish_el<NB, ArithF64, true><<<g, 32, 0, h->st>>>(a, p);
+  auto go = [&](auto arith) {
+    typedef decltype(arith) A;
+    if (rkf) k_finish_el<NB, A, true, true><<<g, 32, 0, h->st>>>(a, p, *rkf);
+    else k_finish_el<NB, A, true><<<g, 32, 0, h->st>>>(a, p, RkfStage());
+  };
+  if (h->fmt == DMD_PREC_F64X) go(ArithDF());
+  else if (deviation_form(h->prec)) go(ArithF32());
+  else go(ArithF64());
   h->launches++;
   CKL();
   return DMD_OK;
@@ -1406,8 +1408,7 @@ void release(dmd_handle* h) {
   if (h->g_rk4) cudaGraphExecDestroy(h->g_rk4);
   if (h->g_rk4_rec) cudaGraphExecDestroy(h->g_rk4_rec);
   void* ptrs[] = {h->d_err, h->d_pos, h->d_rb, h->d_items, h->d_ew, h->d_edm, h->d_kk, h->d_P, h->d_H, h->d_eq, h->d_rs, h->d_acc, h->d_y, h->d_ytmp,
-                  h->d_y0, h->d_in, h->d_in1, h->d_out, h->d_K, h->d_tref, h->d_step, h->d_red, h->d_coef_i,
-                  h->d_coef, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
+                  h->d_y0, h->d_in, h->d_in1, h->d_out, h->d_K, h->d_tref, h->d_step, h->d_red, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
                   h->d_dst, h->d_ee_kvec, h->d_ee_kidx, h->d_ee_kmap, h->d_ee_U, h->d_ee_ewf, h->d_ee_f,
                   h->d_ee_dm, h->d_ee_dm1, h->d_ee_dmf, h->d_ee_dm1f, h->d_ee_scr, h->d_ee_Pee, h->d_ee_vqtab,
                   h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ};
@@ -1785,8 +1786,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
       (rc = dalloc(h, &h->d_y0, h->nstate)) || (rc = dalloc(h, &h->d_in, h->nstate)) ||
       (rc = dalloc(h, &h->d_in1, h->nstate)) || (rc = dalloc(h, &h->d_out, h->nstate)) ||
       (rc = dalloc(h, &h->d_K, 6 * h->nstate)) || (rc = dalloc(h, &h->d_tref, 2)) ||
-      (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_coef_i, 64)) ||
-      (rc = dalloc(h, &h->d_coef, 64)) || (rc = dalloc(h, &h->d_flag, 1)) || (rc = dalloc(h, &h->d_err, 1)) ||
+      (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_flag, 1)) || (rc = dalloc(h, &h->d_err, 1)) ||
       (rc = dalloc(h, &h->d_hflag, 4)) || (rc = dalloc(h, &h->d_ph, nk * h->nb2)))
     return bail(rc);
   std::vector<double> ew(nk * h->nb);
@@ -2144,7 +2144,11 @@ static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* re
     if (fused) {  // the coordinates are there: from rk4_begin or the finish before
       rc = h->nb == 2 ? launch_pairs<2>(h) : launch_pairs<4>(h);
       if (!rc && recA) CK(cudaMemcpyAsync(recA + (size_t)s * na, h->d_acc, na * 16, cudaMemcpyDeviceToDevice, h->st));
-      if (!rc) rc = h->nb == 2 ? launch_finish_prep<2>(h, fa) : launch_finish_prep<4>(h, fa);
+      TimeArg tn = ta;  // the next stage's time; behind stage 3 the next step's first
+      tn.stage = (s + 1) % 4;
+      tn.ahead = s == 3 ? 1 : 0;
+      if (!rc)
+        rc = h->nb == 2 ? launch_finish_prep<2>(h, fa, tn, tn.stage, nullptr) : launch_finish_prep<4>(h, fa, tn, tn.stage, nullptr);
       h->eval = 0;
     } else {
       rc = rhs(h, in, ta, fa);
@@ -2265,23 +2269,44 @@ struct Rkf {
   double* K(int j) { return (double*)(h->d_K + (size_t)j * h->nstate); }
 };
 
-int comb(dmd_handle* h, const double* base, int nterms, const int* kidx, const double* coef, double hs, int premul,
-         double* out) {
-  // coefficients by value through a small device table (copied from pageable host memory)
-  int ibuf[8];
-  double cbuf[8];
-  for (int i = 0; i < nterms; ++i) {
-    ibuf[i] = kidx[i];
-    cbuf[i] = coef[i];
+const int kIdx[] = {0, 1, 2, 3, 4};   // slopes of a stage's input
+const int kIdxC[] = {0, 2, 3, 4, 5};  // of the new y and of the error estimate
+
+RkComb rk_comb(int n, const int* k, const double* c, double hs, int premul) {
+  RkComb r;
+  memset(&r, 0, sizeof(r));
+  r.n = n;
+  r.premul = premul;
+  r.h = hs;
+  for (int i = 0; i < n; ++i) {
+    r.k[i] = k[i];
+    r.c[i] = c[i];
   }
-  CK(cudaMemcpyAsync(h->d_coef_i, ibuf, sizeof(int) * nterms, cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->d_coef, cbuf, sizeof(double) * nterms, cudaMemcpyHostToDevice, h->st));
+  return r;
+}
+
+// the input of stage s = 1..5, and (s = 6) the new y
+RkComb rk_input(int s, double hs) {
+  const double* const c[] = {nullptr, &kAh[0], kB3, kB4, kB5, kB6, kC};
+  return s == 6 ? rk_comb(5, kIdxC, kC, hs, 0) : rk_comb(s, kIdx, c[s], hs, s == 1);
+}
+
+int comb(dmd_handle* h, const double* base, const RkComb& cb, double* out) {
   const size_t n = 2 * h->nstate;
-  k_rk_comb<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, base, (const double*)h->d_K, 2 * h->nstate, nterms,
-                                                              h->d_coef_i, h->d_coef, hs, premul, out);
+  k_rk_comb<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, base, (const double*)h->d_K, 2 * h->nstate, cb, out);
   h->launches++;
   CKL();
-  CK(cudaStreamSynchronize(h->st));  // the small tables are reused by the next call
+  return DMD_OK;
+}
+
+// the step control's ratio, from the device
+int read_ratio(dmd_handle* h, double* rmax) {
+  unsigned long long bits = 0;
+  CK(cudaMemcpyAsync(&bits, h->d_red, sizeof(bits), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  double m;
+  memcpy(&m, &bits, sizeof(m));
+  *rmax = m > 2.2250738585072014e-308 ? m : 2.2250738585072014e-308;
   return DMD_OK;
 }
 
@@ -2290,45 +2315,64 @@ int feval(Rkf& r, double t, const double* y, double* out) {
   return rhs_plain(r.h, t, (const double2*)y, (double2*)out);
 }
 
+// One attempt from (t, y) with the slope K(0) there; y becomes the new y.
 int rkf45_step(Rkf& r, double t, double hs, double* y, double* rmax, double eps_abs, double eps_rel) {
   dmd_handle* h = r.h;
   double* yt = (double*)h->d_ytmp;
   int rc;
-  const int i1[] = {0};
-  if ((rc = comb(h, y, 1, i1, &kAh[0], hs, 1, yt))) return rc;
-  if ((rc = feval(r, t + kAh[0] * hs, yt, r.K(1)))) return rc;
-  const int i2[] = {0, 1};
-  if ((rc = comb(h, y, 2, i2, kB3, hs, 0, yt))) return rc;
-  if ((rc = feval(r, t + kAh[1] * hs, yt, r.K(2)))) return rc;
-  const int i3[] = {0, 1, 2};
-  if ((rc = comb(h, y, 3, i3, kB4, hs, 0, yt))) return rc;
-  if ((rc = feval(r, t + kAh[2] * hs, yt, r.K(3)))) return rc;
-  const int i4[] = {0, 1, 2, 3};
-  if ((rc = comb(h, y, 4, i4, kB5, hs, 0, yt))) return rc;
-  if ((rc = feval(r, t + kAh[3] * hs, yt, r.K(4)))) return rc;
-  const int i5[] = {0, 1, 2, 3, 4};
-  if ((rc = comb(h, y, 5, i5, kB6, hs, 0, yt))) return rc;
-  if ((rc = feval(r, t + kAh[4] * hs, yt, r.K(5)))) return rc;
-  const int i6[] = {0, 2, 3, 4, 5};
-  if ((rc = comb(h, y, 5, i6, kC, hs, 0, y))) return rc;
+  for (int s = 1; s <= 5; ++s) {
+    if ((rc = comb(h, y, rk_input(s, hs), yt))) return rc;
+    if ((rc = feval(r, t + kAh[s - 1] * hs, yt, r.K(s)))) return rc;
+  }
+  if ((rc = comb(h, y, rk_input(6, hs), y))) return rc;
   // error estimate and control ratio on the updated y
-  int ebuf[5] = {0, 2, 3, 4, 5};
-  CK(cudaMemcpyAsync(h->d_coef_i, ebuf, sizeof(ebuf), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(h->d_coef, kE, sizeof(kE), cudaMemcpyHostToDevice, h->st));
   const size_t n = 2 * h->nstate;
-  const unsigned nbk = blocks_for((long long)n, 256);
-  if (nbk > red_elems(h)) return fail(h, DMD_E_ARG, "state too large for the error reduction");
-  k_rk_err<<<nbk, 256, 0, h->st>>>(n, y, (const double*)h->d_K, 2 * h->nstate, 5, h->d_coef_i, h->d_coef, hs, eps_abs,
-                                   eps_rel, h->d_red);
+  CK(cudaMemsetAsync(h->d_red, 0, 8, h->st));
+  k_rk_err<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, y, (const double*)h->d_K, 2 * h->nstate,
+                                                             rk_comb(5, kIdxC, kE, hs, 0), eps_abs, eps_rel,
+                                                             (unsigned long long*)h->d_red);
   h->launches++;
   CKL();
-  std::vector<double> bm(nbk);
-  CK(cudaMemcpyAsync(bm.data(), h->d_red, nbk * 8, cudaMemcpyDeviceToHost, h->st));
-  CK(cudaStreamSynchronize(h->st));
-  double m = 2.2250738585072014e-308;
-  for (double v : bm) m = v > m ? v : m;
-  *rmax = m;
-  return DMD_OK;
+  return read_ratio(h, rmax);
+}
+
+// Stage s of a step from (t0, h->d_y) in the fused form: its coordinates are there; the finish forms the next stage's
+// input and coordinates (s = 5: the new y, the error ratio, and the coordinates at (tnext, new y)).
+int rkf45_stage(Rkf& r, int s, double t0, double hs, double tnext, double eps_abs, double eps_rel) {
+  dmd_handle* h = r.h;
+  r.nfev++;
+  h->eval = s & 1;  // two flags in turn: the finish of one evaluation raises the other's
+  FinishArgs fa = base_finish(h, s == 0 ? h->d_y : h->d_ytmp);
+  fa.mode = 1;
+  fa.stage = s;
+  fa.K = h->d_K;
+  fa.ybase = h->d_y;
+  fa.ytmp = h->d_ytmp;
+  fa.ta = time_value(s == 0 ? t0 : t0 + kAh[s - 1] * hs);
+  RkfStage st;
+  memset(&st, 0, sizeof(st));
+  st.next = rk_input(s + 1, hs);
+  if (s == 5) {
+    st.err = rk_comb(5, kIdxC, kE, hs, 0);
+    st.last = 1;
+    st.eps_abs = eps_abs;
+    st.eps_rel = eps_rel;
+    st.rmax = (unsigned long long*)h->d_red;
+  }
+  const TimeArg tn = time_value(s == 5 ? tnext : t0 + kAh[s] * hs);
+  int rc = h->nb == 2 ? launch_pairs<2>(h) : launch_pairs<4>(h);
+  if (!rc) rc = h->nb == 2 ? launch_finish_prep<2>(h, fa, tn, (s + 1) & 1, &st) : launch_finish_prep<4>(h, fa, tn, (s + 1) & 1, &st);
+  h->eval = 0;
+  return rc;
+}
+
+// coordinates of y at t for stage s (0 or 1) of the fused form, with the flags cleared
+int rkf45_prep(dmd_handle* h, int s, double t, const double2* y) {
+  CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
+  h->eval = s & 1;
+  const int rc = h->nb == 2 ? launch_prep<2>(h, y, time_value(t)) : launch_prep<4>(h, y, time_value(t));
+  h->eval = 0;
+  return rc;
 }
 
 }  // namespace
@@ -2345,6 +2389,8 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
   const int sign = (*hstep > 0.0) ? 1 : -1;
   if (sign * (t1 - h->t) < 0.0) return fail(h, DMD_E_ODE, "integration limits and step direction disagree");
   int rc;
+  const bool fused = fused_step(h);
+  bool ready = false;  // fused form: the coordinates at (h->t, y) are there
   while (sign * (t1 - h->t) > 0.0) {
     // gsl_odeiv2_evolve_apply
     const double t0 = h->t;
@@ -2352,15 +2398,28 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
     const double dt = t1 - t0;
     if ((dt < 0.0 && h0 > 0.0) || (dt > 0.0 && h0 < 0.0)) return fail(h, DMD_E_ODE, "step direction");
     CK(cudaMemcpyAsync(y0, y, bytes, cudaMemcpyDeviceToDevice, h->st));
-    if ((rc = feval(r, t0, y, r.K(0)))) return rc;  // dydt_in
-    for (;;) {
+    if (!fused && (rc = feval(r, t0, y, r.K(0)))) return rc;  // dydt_in
+    if (fused && !ready && (rc = rkf45_prep(h, 0, t0, h->d_y))) return rc;
+    for (bool first = true;; first = false) {
       int final_step = 0;
       if ((dt >= 0.0 && h0 > dt) || (dt < 0.0 && h0 < dt)) {
         h0 = dt;
         final_step = 1;
       }
       double rmax;
-      if ((rc = rkf45_step(r, t0, h0, y, &rmax, epsabs, epsrel))) return rc;
+      if (fused) {
+        if (!first) {  // a retry: the slope at (t0, y) stays, the first stage's input is new
+          if ((rc = comb(h, y, rk_input(1, h0), (double*)h->d_ytmp)) || (rc = rkf45_prep(h, 1, t0 + kAh[0] * h0, h->d_ytmp)))
+            return rc;
+        }
+        CK(cudaMemsetAsync(h->d_red, 0, 8, h->st));
+        for (int s = first ? 0 : 1; s < 6; ++s)
+          if ((rc = rkf45_stage(r, s, t0, h0, final_step ? t1 : t0 + h0, epsabs, epsrel))) return rc;
+        if ((rc = read_ratio(h, &rmax))) return rc;
+        ready = true;
+      } else if ((rc = rkf45_step(r, t0, h0, y, &rmax, epsabs, epsrel))) {
+        return rc;
+      }
       h->t = final_step ? t1 : t0 + h0;
       const double h_old = h0;
       // standard control, order 5
@@ -2381,6 +2440,7 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
         if (fabs(h0) < fabs(h_old) && t_next != t_curr) {
           CK(cudaMemcpyAsync(y, y0, bytes, cudaMemcpyDeviceToDevice, h->st));
           h->t = t0;
+          ready = false;
           continue;  // retry with the smaller step (dydt_in reused)
         }
         h0 = h_old;
@@ -2395,6 +2455,7 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
     }
   }
   if (nfev) *nfev = r.nfev;
+  if ((rc = rk4_end(h))) return rc;  // no flag of the coordinates prepared for a step that does not follow
   return check_state(h);
 }
 

@@ -26,14 +26,23 @@ struct NextPrep {
   TimeArg ta;
 };
 
+// A stage of the RKF45 step: its slope goes to slot FinishArgs::stage of K and the next stage's input (the last stage:
+// the new y, in place, and the error ratio) is formed from the slopes so far
+struct RkfStage {
+  RkComb next, err;
+  int last;
+  double eps_abs, eps_rel;
+  unsigned long long* rmax;
+};
+
 template <int NB>
 __device__ __forceinline__ double2 group_get(double2 v, int lane) {
   return mk2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
 }
 
-// A: coordinate type of the next evaluation (PREP)
-template <int NB, typename A, bool PREP>
-__global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p) {
+// A: coordinate type of the next evaluation (PREP); RKF: stages of the RKF45 step instead of RK4's
+template <int NB, typename A, bool PREP, bool RKF = false>
+__global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p, RkfStage r) {
   constexpr int NB2 = NB * NB;
   const int lane = threadIdx.x, e = lane % NB2, i = e / NB, j = e % NB, g0 = lane - e;  // group's first lane
   const int ji = j * NB + i, tl = g0 + ji;                                             // the transposed element's lane
@@ -130,17 +139,30 @@ __global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p) {
     if (live) a.out[el] = f;
     return;
   }
-  const double h = a.tref[1];
+  const size_t n = (size_t)a.nk * NB2;
+  const double h = RKF ? 0.0 : a.tref[1];
   double2 yn = y;
-  if (a.mode == 2) {  // update_dm_euler: dm += 0.5*dt*(ddmdt + ddmdt^dagger)
+  if (RKF) {
+    auto slope = [&](int s) { return s == a.stage ? f : a.K[(size_t)s * n + el]; };
+    const double2 yb = a.ybase[el];
+    yn = mk2(__dadd_rn(yb.x, r.next([&](int s) { return slope(s).x; })),
+             __dadd_rn(yb.y, r.next([&](int s) { return slope(s).y; })));
+    if (live) {
+      a.K[(size_t)a.stage * n + el] = f;
+      (r.last ? a.ybase : a.ytmp)[el] = yn;
+    }
+    if (r.last) {
+      const double ex = rk_ratio(r.err([&](int s) { return slope(s).x; }), yn.x, r.eps_abs, r.eps_rel);
+      const double ey = rk_ratio(r.err([&](int s) { return slope(s).y; }), yn.y, r.eps_abs, r.eps_rel);
+      rk_max(live ? fmax(ex, ey) : 0.0, r.rmax);
+    }
+  } else if (a.mode == 2) {  // update_dm_euler: dm += 0.5*dt*(ddmdt + ddmdt^dagger)
     const double2 fo = group_get<NB>(f, tl);
     yn = cadd_rn(a.ybase[el], cscale_rn(0.5 * h, cadd_rn(f, cconj(fo))));
     if (live) a.ybase[el] = yn;
     return;
-  }
-  const size_t n = (size_t)a.nk * NB2;
-  const double2 yb = a.ybase[el];
-  if (a.stage < 3) {
+  } else if (a.stage < 3) {
+    const double2 yb = a.ybase[el];
     yn = cadd_rn(yb, cscale_rn(a.stage == 2 ? h : 0.5 * h, f));
     if (live) {
       a.K[(size_t)a.stage * n + el] = f;
@@ -148,6 +170,7 @@ __global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p) {
     }
   } else {
     const double h6 = h / 6.0;
+    const double2 yb = a.ybase[el];
     const double2 k1 = a.K[el], k2 = a.K[n + el], k3 = a.K[2 * n + el];
     // y + h/6 * (k1 + 2 k2 + 2 k3 + k4), evaluated left to right
     const double sx = __dadd_rn(__dadd_rn(__dadd_rn(k1.x, __dmul_rn(2.0, k2.x)), __dmul_rn(2.0, k3.x)), f.x);

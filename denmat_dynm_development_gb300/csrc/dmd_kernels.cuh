@@ -610,42 +610,45 @@ __global__ void k_step_inc(long long* step) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *step += 1;
 }
 
-// out = base + h * (c0 K0 + c1 K1 + ...), left to right; premul: (c0*h)*K0 form of the first stage
+// h * (c0 K0 + c1 K1 + ...) of an embedded Runge-Kutta step, left to right; premul: (c0 h) K0, the first stage's form.
+// Passed by value, so that no stage waits for a copy of its coefficients.
+struct RkComb {
+  int n, premul;
+  int k[6];
+  double c[6];
+  double h;
+  // K(j): the j-th slope's component
+  template <typename F>
+  __device__ __forceinline__ double operator()(F K) const {
+    if (premul) return __dmul_rn(__dmul_rn(c[0], h), K(k[0]));
+    double s = __dmul_rn(c[0], K(k[0]));
+    for (int j = 1; j < n; ++j) s = __dadd_rn(s, __dmul_rn(c[j], K(k[j])));
+    return __dmul_rn(h, s);
+  }
+};
+
 __global__ void k_rk_comb(size_t n, const double* __restrict__ base, const double* __restrict__ K, size_t kstride,
-                          int nk_terms, const int* __restrict__ kidx, const double* __restrict__ coef, double h,
-                          int premul, double* __restrict__ out) {
+                          RkComb cb, double* __restrict__ out) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  if (premul) {  // y + c*h*k
-    out[i] = __dadd_rn(base[i], __dmul_rn(__dmul_rn(coef[0], h), K[kidx[0] * kstride + i]));
-    return;
-  }
-  double s = __dmul_rn(coef[0], K[kidx[0] * kstride + i]);
-  for (int j = 1; j < nk_terms; ++j) s = __dadd_rn(s, __dmul_rn(coef[j], K[kidx[j] * kstride + i]));
-  out[i] = __dadd_rn(base[i], __dmul_rn(h, s));
+  out[i] = __dadd_rn(base[i], cb([&](int j) { return K[j * kstride + i]; }));
 }
 
-// yerr = h * (e1 K1 + e3 K3 + ...) and per-block max of |yerr| / (eps_rel * |y| + eps_abs)
-__global__ void k_rk_err(size_t n, const double* __restrict__ y, const double* __restrict__ K, size_t kstride,
-                         int nk_terms, const int* __restrict__ kidx, const double* __restrict__ coef, double h,
-                         double eps_abs, double eps_rel, double* __restrict__ blockmax) {
-  __shared__ double sm[256];
+// the ratio of the step control (gsl standard control on the new y): error over eps_rel |y| + eps_abs
+__device__ __forceinline__ double rk_ratio(double yerr, double y, double eps_abs, double eps_rel) {
+  return fabs(yerr) / fabs(__dadd_rn(__dmul_rn(eps_rel, __dadd_rn(fabs(y), 0.0)), eps_abs));
+}
+
+// its maximum over the state, to *rmax (the bits of a non-negative double order as integers); NaN is passed over
+__device__ __forceinline__ void rk_max(double r, unsigned long long* rmax) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+  if ((threadIdx.x & 31) == 0 && r > 0.0) atomicMax(rmax, (unsigned long long)__double_as_longlong(r));
+}
+__global__ void k_rk_err(size_t n, const double* __restrict__ y, const double* __restrict__ K, size_t kstride, RkComb cb,
+                         double eps_abs, double eps_rel, unsigned long long* __restrict__ rmax) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  double r = 2.2250738585072014e-308;
-  if (i < n) {
-    double s = __dmul_rn(coef[0], K[kidx[0] * kstride + i]);
-    for (int j = 1; j < nk_terms; ++j) s = __dadd_rn(s, __dmul_rn(coef[j], K[kidx[j] * kstride + i]));
-    const double yerr = __dmul_rn(h, s);
-    const double D0 = __dadd_rn(__dmul_rn(eps_rel, __dadd_rn(fabs(y[i]), 0.0)), eps_abs);
-    r = fabs(yerr) / fabs(D0);
-  }
-  sm[threadIdx.x] = r;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + s]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) blockmax[blockIdx.x] = sm[0];
+  rk_max(i < n ? rk_ratio(cb([&](int j) { return K[j * kstride + i]; }), y[i], eps_abs, eps_rel) : 0.0, rmax);
 }
 
 // observable totals (observable.h:356-366), per-block partial sums; block b covers k in a stripe

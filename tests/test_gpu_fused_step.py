@@ -75,3 +75,62 @@ def test_group_follows_a_change_of_a_member(oracle, built):  # noqa: F811
         alone.rk4(h, 1)
         a, b = g.get_state()[1], alone.get_state()[1]
     assert np.abs(a - b).max() <= 1e-14 * np.abs(b).max()
+
+
+def host_rkf45(f, t, t1, h, eps_abs, eps_rel, y):
+    """Fehlberg's pair with the standard control on the new y (GSL's rkf45 driver), on the host"""
+    A = [1 / 4, 3 / 8, 12 / 13, 1.0, 1 / 2]
+    B = [[1 / 4], [3 / 32, 9 / 32], [1932 / 2197, -7200 / 2197, 7296 / 2197],
+         [8341 / 4104, -32832 / 4104, 29440 / 4104, -845 / 4104],
+         [-6080 / 20520, 41040 / 20520, -28352 / 20520, 9295 / 20520, -5643 / 20520]]
+    C = [902880 / 7618050, 0.0, 3953664 / 7618050, 3855735 / 7618050, -1371249 / 7618050, 277020 / 7618050]
+    E = [1 / 360, 0.0, -128 / 4275, -2197 / 75240, 1 / 50, 2 / 55]
+    evals = rejected = 0
+    while t < t1:
+        K = [f(t, y)]
+        evals += 1
+        while True:
+            last = h > t1 - t
+            h = t1 - t if last else h
+            del K[1:]
+            for a, b in zip(A, B):
+                K.append(f(t + a * h, y + h * sum(u * k for u, k in zip(b, K))))
+                evals += 1
+            yn = y + h * sum(u * k for u, k in zip(C, K))
+            r = float((np.abs(h * sum(u * k for u, k in zip(E, K))) / (eps_rel * np.abs(yn) + eps_abs)).max())
+            if r > 1.1:
+                h *= max(0.2, 0.9 / r ** 0.2)
+                rejected += 1
+                continue
+            y, t = yn, t1 if last else t + h
+            if r < 0.5:
+                h *= min(5.0, max(1.0, 0.9 / max(r, 2.3e-308) ** (1 / 6)))
+            break
+    return y, h, evals, rejected
+
+
+@pytest.mark.parametrize("nb,nk", [(2, 37), (4, 9)])
+@pytest.mark.parametrize("h0,eps_abs,eps_rel", [(50.0, 1e-12, 0.0), (0.5, 1e-11, 1e-9), (400.0, 1e-13, 0.0)])
+def test_fused_rkf45(nb, nk, h0, eps_abs, eps_rel, oracle, built):  # noqa: F811
+    """steps accepted, rejected and retried, and a second interval from where the first one ended; the same number of
+    evaluations, the state within the roundings of its own updates (1e-12, evaluations as above)"""
+    s = system(oracle, nk, nb, 0.8, 3 * nk + nb)
+    s.prefac_eph = 2e-5  # a few hundred fs of relaxation: the control has something to do
+    rng = np.random.default_rng(4)
+    y = oracle.y_of(s.dm0) * (1.0 + (1e-3 * rng.standard_normal(2 * nk * nb * nb) if nb == 4 else 0.0))
+    t, rejected = 2.0 * oracle.fs, 0
+    with handle(s, "f64", 0, 1, None) as g:
+        g.set_state(t, y)
+        h = hg = h0 * oracle.fs
+        for t1 in (t + 100.0 * oracle.fs, t + 150.0 * oracle.fs):
+            y, h, evals, rej = host_rkf45(g.func, t, t1, h, eps_abs, eps_rel, y)
+            rejected += rej
+            g.set_state(t, g.get_state()[1])
+            hg, n = g.rkf45_apply(t1, hg, epsabs=eps_abs, epsrel=eps_rel)
+            assert n == evals
+            assert abs(hg - h) <= 1e-4 * h  # (the ratio is a difference of slopes near the tolerance)
+            tg, yg = g.get_state()
+            assert tg == t1 and np.abs(yg - y).max() <= 1e-12 * np.abs(y).max()
+            t, hg, y = t1, h, yg
+            g.set_state(t, y)
+    assert rejected > 0 or h0 < 1.0
