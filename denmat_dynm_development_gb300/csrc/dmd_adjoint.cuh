@@ -21,6 +21,7 @@
 // gradients with respect to the operators (and the initial state's Hermitian part) are exact.
 #pragma once
 #include "dmd_common.cuh"
+#include "dmd_finish.cuh"
 #include "dmd_kernels.cuh"
 #include "dmd_pairs_cb.cuh"
 #include "dmd_tma.cuh"
@@ -45,7 +46,7 @@ struct AdjLocalArgs {
   double2* ubar;        // [k][nbdm^2]: coherent adjoint + local e-ph adjoint
   double2* rtb;         // transposed-contraction sums [k][NB2], zeroed here for the pair pass (or null)
   double2* stb;
-  float4* dfv;          // double-float forms (x, S(x)) of Xb, Yb, rt, st for k_adj_pairs_df (or null)
+  float4* dfv;          // double-float forms of Xb, Yb, rt, st (adj_store_df), instead of the complex128 ones (or null)
   size_t nk2;           // nk NB2
 };
 
@@ -62,6 +63,23 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
 __device__ __forceinline__ float4 dfc_split(double re, double im) {
   const float rh = __double2float_rn(re), ih = __double2float_rn(im);
   return make_float4(rh, ih, __double2float_rn(__dsub_rn(re, (double)rh)), __double2float_rn(__dsub_rn(im, (double)ih)));
+}
+
+// the double-float forms of element el of Xbar, Ybar, rt, st: nb = 4 as (x, S(x)), S(x) = (Im x, -Re x), for the pair
+// pass that stages them in shared memory; nb = 2 x alone
+template <int NB>
+__device__ __forceinline__ void adj_store_df(const AdjLocalArgs& a, size_t el, double2 x, double2 y, double2 r, double2 s) {
+  const double2 v4[4] = {x, y, r, s};
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    if (NB == 2) {
+      a.dfv[(size_t)v * a.nk2 + el] = dfc_split(v4[v].x, v4[v].y);
+    } else {
+      float4* o = a.dfv + 2 * ((size_t)v * a.nk2 + el);
+      o[0] = dfc_split(v4[v].x, v4[v].y);
+      o[1] = dfc_split(v4[v].y, -v4[v].x);
+    }
+  }
 }
 
 template <int NB>
@@ -167,17 +185,87 @@ __global__ void k_adj_local(AdjLocalArgs a) {
       Ybk[e] = cmulc(D[e], db);
       a.rt[(size_t)k * NB2 + e] = cmulc(D[e], r[e]);
       a.st[(size_t)k * NB2 + e] = cmulc(D[e], om[e]);
-      if (a.dfv) {  // (x, S(x)), S(x) = (Im x, -Re x), of the four vectors
-        const double2 v4[4] = {Xbk[e], Ybk[e], a.rt[(size_t)k * NB2 + e], a.st[(size_t)k * NB2 + e]};
-        for (int v = 0; v < 4; ++v) {
-          float4* o = a.dfv + 2 * ((size_t)v * a.nk2 + (size_t)k * NB2 + e);
-          o[0] = dfc_split(v4[v].x, v4[v].y);
-          o[1] = dfc_split(v4[v].y, -v4[v].x);
-        }
-      }
+      if (a.dfv) adj_store_df<NB>(a, (size_t)k * NB2 + e, Xbk[e], Ybk[e], a.rt[(size_t)k * NB2 + e], a.st[(size_t)k * NB2 + e]);
       double2& o = ub[(a.bs + i) * nd + a.bs + j];
       o = cadd(o, rb);
     }
+}
+
+// k_adj_local with one lane per element of rho_k (nb = 2 or 4, the window the whole density matrix), operands by
+// shuffles within the k-point's nb^2 lanes; element by element the same operations in the same order. A thread per k-point
+// ran 500 of them on 4 SMs, each through the whole chain at the FP64 pipe's latency: 28 us per launch, here 5.
+template <int NB>
+__global__ void __launch_bounds__(32) k_adj_local_el(AdjLocalArgs a) {
+  constexpr int NB2 = NB * NB;
+  const int lane = threadIdx.x, e = lane % NB2, i = e / NB, j = e % NB, g0 = lane - e, tl = g0 + j * NB + i;
+  const int kl = (blockIdx.x * 32 + lane) / NB2;
+  const bool live = kl < a.nk;  // dead groups still take part in the shuffles
+  const int k = live ? kl : a.nk - 1;
+  const size_t el = (size_t)k * NB2 + e;
+  const double2 r = a.u[el], v = a.vbar[el];
+  double2 ub = mk2(0.0, 0.0);
+  auto get = [&](double2 x, int row, int col) { return group_get<NB>(x, g0 + row * NB + col); };
+  if (a.want_coh) {  // coherent term -i[H(t), rho]: adjoint i(H v - v H) (H Hermitian, read from its upper triangle)
+    const double* ek = a.edm + (size_t)k * NB;
+    if (a.H) {
+      double2 hv = a.H[el];
+      if (i == j) hv = mk2(hv.x, 0.0);
+      else if (a.picture == 0 && i < j) hv = cmul(hv, ccis((ek[i] - ek[j]) * a.t));
+      const double2 ho = group_get<NB>(hv, tl);
+      if (i > j) hv = cconj(ho);
+      double2 s = mk2(0.0, 0.0);
+#pragma unroll
+      for (int l = 0; l < NB; ++l) s = cadd(s, csub(cmul(get(hv, i, l), get(v, l, j)), cmul(get(v, i, l), get(hv, l, j))));
+      ub = mk2(-s.y, s.x);  // i * s
+    } else if (a.picture == 1) {  // -i[E, rho]: adjoint i (e_i - e_j) v_ij
+      const double w = ek[i] - ek[j];
+      ub = mk2(-w * v.y, w * v.x);
+    }
+  }
+  const size_t ax = (size_t)(a.pos ? a.pos[k] : k) * 2 * NB2 + e;
+  double2 X = a.acc[ax], Y = a.acc[ax + NB2];
+  if (a.herm) {  // X = (M^H)^-1 X'
+    const double2 xo = group_get<NB>(X, tl), yo = group_get<NB>(Y, tl);
+    if (i < j) {
+      X = mk2(0.5 * (X.x - xo.y), 0.5 * (X.y + xo.x));
+      Y = mk2(0.5 * (Y.x - yo.y), 0.5 * (Y.y + yo.x));
+    } else if (i > j) {
+      X = mk2(0.5 * (xo.x + X.y), 0.5 * (xo.y - X.x));
+      Y = mk2(0.5 * (yo.x + Y.y), 0.5 * (yo.y - Y.x));
+    }
+  }
+  double2 D = mk2(1.0, 0.0);
+  if (a.phase && i != j) D = a.ph ? a.ph[el] : ccis((a.ew[(size_t)k * NB + i] - a.ew[(size_t)k * NB + j]) * a.t);
+  const double2 om = (i == j) ? mk2(1.0 - r.x, -r.y) : mk2(-r.x, -r.y);
+  const double2 vo = group_get<NB>(v, tl);
+  const double pf = 0.5 * a.prefac;
+  const double2 cb = mk2(pf * (v.x + vo.x), pf * (v.y - vo.y));
+  const double2 Pdm = cmul(D, X), dmP = cmul(D, Y);
+  double2 pb = mk2(0.0, 0.0), db = mk2(0.0, 0.0), rb = mk2(0.0, 0.0);
+  if (a.lin) {
+    pb = cb;
+  } else {
+#pragma unroll
+    for (int l = 0; l < NB; ++l) {
+      const double2 cil = get(cb, i, l), clj = get(cb, l, j);
+      pb = cadd(pb, cmulc(get(om, l, i), clj));          // (1 - rho)^H cbar
+      db = csub(db, cmul(cil, cconj(get(r, j, l))));     // -cbar rho^H
+      rb = csub(rb, cmul(cil, cconj(get(Pdm, j, l))));   // -cbar Pdm^H
+      rb = csub(rb, cmulc(get(dmP, l, i), clj));         // -dm1P^H cbar
+    }
+  }
+  if (!live) return;
+  if (a.rtb) a.rtb[el] = a.stb[el] = mk2(0.0, 0.0);
+  const double2 Xb = cmulc(D, pb), Yb = cmulc(D, db), rt = cmulc(D, r), st = cmulc(D, om);
+  if (a.dfv) {
+    adj_store_df<NB>(a, el, Xb, Yb, rt, st);
+  } else {
+    a.Xb[el] = Xb;
+    a.Yb[el] = Yb;
+    a.rt[el] = rt;
+    a.st[el] = st;
+  }
+  a.ubar[el] = cadd(ub, rb);
 }
 
 // Transposed pair contraction and the operator gradient. One thread per (pair, index b).
@@ -282,108 +370,140 @@ __global__ void k_conj(size_t n, double2* __restrict__ g) {
   if (i < n) g[i].y = -g[i].y;
 }
 
-// One thread per (pair, index b), as k_adj_pairs. dfv: k_adj_local's double-float forms; P: double-float pair
-// operators; G: double-float gradient [pair][G1 | G2][nb^4].
-template <int NB>
-__global__ void __launch_bounds__(128) k_adj_pairs_df(long long npair, const int2* __restrict__ kk,
-                                                      const float4* __restrict__ P, const float4* __restrict__ dfv,
-                                                      size_t nk2, double* __restrict__ rtb, double* __restrict__ stb,
-                                                      float4* __restrict__ G) {
-  constexpr int NB2 = NB * NB, NB4 = NB2 * NB2;
+// nb = 2: the contraction and the gradient apart, a thread per (pair, index b) each. The contraction is in the chain of
+// the stages and reads the operators; the gradient is not, and one launch adds the outer products of up to
+// kAdjGradStages stages to it in registers, where a pass per stage read and wrote it (36 of 72 MB of traffic on 69k pairs,
+// 42 us per stage; now 16 and 5). v: vectors Xbar, Ybar, rt, st of a stage, [v][nk nb^2] double-floats.
+constexpr int kAdjGradStages = 32;
+
+// (x.im, x.re): conj(p) x = x o (Re p, Re p) + swap(x) o (Im p, -Im p)
+__device__ __forceinline__ float4 df_swap(const float4& x) { return make_float4(x.y, x.x, x.w, x.z); }
+__device__ __forceinline__ float4 df_bipm(const float4& x) { return make_float4(x.y, -x.y, x.w, -x.w); }
+__device__ __forceinline__ float4 df_bimp(const float4& x) { return make_float4(-x.y, x.y, -x.w, x.w); }
+
+__global__ void __launch_bounds__(128) k_adj_contract_df(long long npair, const int2* __restrict__ kk,
+                                                         const float4* __restrict__ P, const float4* __restrict__ v,
+                                                         size_t nk2, double* __restrict__ rtb, double* __restrict__ stb) {
+  constexpr int NB2 = 4, NB4 = 16;
+  constexpr unsigned FULL = 0xffffffffu;
+  typedef ArithDF D;
+  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const bool live = idx < npair * NB2;  // idle lanes of the last warp take part in the shuffles
+  const long long p = (live ? idx : npair * NB2 - 1) / NB2;
+  const int b = (int)(idx & (NB2 - 1));
+  const int2 kp = kk[p];
+  const float4* P1 = P + (size_t)p * 2 * NB4;
+  const float4* P2 = P1 + NB4;
+  const float4 *Xk = v + (size_t)kp.x * NB2, *Xq = v + (size_t)kp.y * NB2, *Yk = Xk + nk2, *Yq = Xq + nk2;
+  const bool rev = live && kp.x < kp.y;
+  D::acc a1, a2, a3, a4;
+  D::zero(a1);
+  D::zero(a2);
+  D::zero(a3);
+  D::zero(a4);
+#pragma unroll
+  for (int a = 0; a < NB2; ++a) {
+    const float4 x = P1[a * NB2 + b], xk = Xk[a];  // conj(P1[a][b]) Xbar[k][a]
+    D::pmac(a1, xk, df_bre(x));
+    D::pmac(a1, df_swap(xk), df_bipm(x));
+    const float4 y = P2[b * NB2 + a], yk = Yk[a];  // conj(P2[b][a]) Ybar[k][a]
+    D::pmac(a2, yk, df_bre(y));
+    D::pmac(a2, df_swap(yk), df_bipm(y));
+  }
+  if (rev) {
+#pragma unroll
+    for (int a = 0; a < NB2; ++a) {
+      const float4 x = P2[a * NB2 + b], xq = Xq[a];  // P2[a][b] Xbar[k'][a]
+      D::pmac(a3, xq, df_bre(x));
+      D::pmac(a3, df_swap(xq), df_bimp(x));
+      const float4 y = P1[b * NB2 + a], yq = Yq[a];  // P1[b][a] Ybar[k'][a]
+      D::pmac(a4, yq, df_bre(y));
+      D::pmac(a4, df_swap(yq), df_bimp(y));
+    }
+  }
+  auto add = [&](double* o, const D::acc& c) {
+    atomicAdd(o, D::re_d(c));
+    atomicAdd(o + 1, D::im_d(c));
+  };
+  if (live) {
+    add(rtb + ((size_t)kp.y * NB2 + b) * 2, a1);
+    add(stb + ((size_t)kp.y * NB2 + b) * 2, a2);
+  }
+  // the k side: pairs are stored by k, so a warp's 8 pairs mostly share it and are added first
+  const bool one = __all_sync(FULL, __shfl_sync(FULL, kp.x, 0) == kp.x);
+  if (one) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      auto sum = [&](D::acc& c) {
+        float4 s = make_float4(c.h.x, c.h.y, c.l.x, c.l.y);
+        const float4 q = make_float4(__shfl_xor_sync(FULL, s.x, o), __shfl_xor_sync(FULL, s.y, o), __shfl_xor_sync(FULL, s.z, o),
+                                     __shfl_xor_sync(FULL, s.w, o));
+        D::red_add4(s, q);
+        c = {make_float2(s.x, s.y), make_float2(s.z, s.w)};
+      };
+      sum(a3);
+      sum(a4);
+    }
+  }
+  if (one ? (threadIdx.x & 31) < NB2 : rev) {
+    add(rtb + ((size_t)kp.x * NB2 + b) * 2, a3);
+    add(stb + ((size_t)kp.x * NB2 + b) * 2, a4);
+  }
+}
+
+// G1[a][b] += conj(Xbar[k][a]) rt[k'][b] (+ conj(st[k][a]) Ybar[k'][b]),
+// G2[a][b] += conj(Ybar[k][b]) st[k'][a] (+ conj(rt[k][b]) Xbar[k'][a]) over the stages, in their order
+__global__ void __launch_bounds__(128) k_adj_grad_df(long long npair, const int2* __restrict__ kk, const float4* __restrict__ v,
+                                                     size_t nk2, int nstage, float4* __restrict__ G) {
+  constexpr int NB2 = 4, NB4 = 16;
   typedef ArithDF D;
   const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= npair * NB2) return;
   const long long p = idx / NB2;
   const int b = (int)(idx - p * NB2);
-  const int2 kp2 = kk[p];
-  const int k = kp2.x, kq = kp2.y;
-  const float4* P1 = P + (size_t)p * 2 * NB4;
-  const float4* P2 = P1 + NB4;
+  const int2 kp = kk[p];
+  const bool rev = kp.x < kp.y;
   float4* G1 = G + (size_t)p * 2 * NB4;
   float4* G2 = G1 + NB4;
-  // element e of vector v at k: (x, S(x)) at dfv[2 ((v nk + k) NB2 + e)]
-  auto vx = [&](int v, int kk_, int e) -> const float4* { return dfv + 2 * ((size_t)v * nk2 + (size_t)kk_ * NB2 + e); };
-  D::acc a1, a2;
-  D::zero(a1);
-  D::zero(a2);
+  D::acc c1[NB2], c2[NB2];
 #pragma unroll
   for (int a = 0; a < NB2; ++a) {
-    const float4 x = P1[a * NB2 + b];  // conj(P1[a][b]) Xbar[k][a]
-    const float4* X = vx(0, k, a);
-    D::pmac(a1, X[0], df_bre(x));
-    D::pmac(a1, X[1], df_bim(x));
-    const float4 y = P2[b * NB2 + a];  // conj(P2[b][a]) Ybar[k][a]
-    const float4* Y = vx(1, k, a);
-    D::pmac(a2, Y[0], df_bre(y));
-    D::pmac(a2, Y[1], df_bim(y));
+    const float4 g = G1[a * NB2 + b], q = G2[a * NB2 + b];
+    c1[a] = {make_float2(g.x, g.y), make_float2(g.z, g.w)};
+    c2[a] = {make_float2(q.x, q.y), make_float2(q.z, q.w)};
   }
-  double* ro = rtb + ((size_t)kq * NB2 + b) * 2;
-  double* so = stb + ((size_t)kq * NB2 + b) * 2;
-  atomicAdd(ro, D::re_d(a1));
-  atomicAdd(ro + 1, D::im_d(a1));
-  atomicAdd(so, D::re_d(a2));
-  atomicAdd(so + 1, D::im_d(a2));
-  const bool rev = k < kq;
-  // G1[a][b] += conj(Xbar[k][a]) rt[k'][b] (+ conj(st[k][a]) Ybar[k'][b]);
-  // G2[a][b] += conj(Ybar[k][b]) st[k'][a] (+ conj(rt[k][b]) Xbar[k'][a])
-  const float4* rq = vx(2, kq, b);
-  const float4* Yq = vx(1, kq, b);
-  const float4 Ykb = vx(1, k, b)[0];
-  const float4 rkb = vx(2, k, b)[0];
-#pragma unroll
-  for (int a = 0; a < NB2; ++a) {
-    float4 g = G1[a * NB2 + b];
-    D::acc c = {make_float2(g.x, g.y), make_float2(g.z, g.w)};
-    const float4 Xka = vx(0, k, a)[0];
-    D::pmac(c, rq[0], df_bre(Xka));
-    D::pmac(c, rq[1], df_bim(Xka));
-    if (rev) {
-      const float4 ska = vx(3, k, a)[0];
-      D::pmac(c, Yq[0], df_bre(ska));
-      D::pmac(c, Yq[1], df_bim(ska));
-    }
-    D::renorm(c);
-    G1[a * NB2 + b] = make_float4(c.h.x, c.h.y, c.l.x, c.l.y);
-    g = G2[a * NB2 + b];
-    c = {make_float2(g.x, g.y), make_float2(g.z, g.w)};
-    const float4* sq = vx(3, kq, a);
-    D::pmac(c, sq[0], df_bre(Ykb));
-    D::pmac(c, sq[1], df_bim(Ykb));
-    if (rev) {
-      const float4* Xq = vx(0, kq, a);
-      D::pmac(c, Xq[0], df_bre(rkb));
-      D::pmac(c, Xq[1], df_bim(rkb));
-    }
-    D::renorm(c);
-    G2[a * NB2 + b] = make_float4(c.h.x, c.h.y, c.l.x, c.l.y);
-  }
-  if (rev) {
-    D::acc a3, a4;
-    D::zero(a3);
-    D::zero(a4);
+  const float4 *k = v + (size_t)kp.x * NB2, *q = v + (size_t)kp.y * NB2;
+#pragma unroll 1
+  for (int s = 0; s < nstage; ++s, k += 4 * nk2, q += 4 * nk2) {
+    const float4 rq = q[2 * nk2 + b], Yq = q[nk2 + b], Yk = k[nk2 + b], rk = k[2 * nk2 + b];
 #pragma unroll
     for (int a = 0; a < NB2; ++a) {
-      const float4 x = P2[a * NB2 + b];  // P2[a][b] Xbar[k'][a]
-      const float4* X = vx(0, kq, a);
-      D::pmac(a3, X[0], df_bre(x));
-      D::pmac(a3, X[1], df_bimn(x));
-      const float4 y = P1[b * NB2 + a];  // P1[b][a] Ybar[k'][a]
-      const float4* Y = vx(1, kq, a);
-      D::pmac(a4, Y[0], df_bre(y));
-      D::pmac(a4, Y[1], df_bimn(y));
+      const float4 Xka = k[a], sqa = q[3 * nk2 + a];
+      D::pmac(c1[a], rq, df_bre(Xka));
+      D::pmac(c1[a], df_swap(rq), df_bipm(Xka));
+      D::pmac(c2[a], sqa, df_bre(Yk));
+      D::pmac(c2[a], df_swap(sqa), df_bipm(Yk));
+      if (rev) {
+        const float4 ska = k[3 * nk2 + a], Xqa = q[a];
+        D::pmac(c1[a], Yq, df_bre(ska));
+        D::pmac(c1[a], df_swap(Yq), df_bipm(ska));
+        D::pmac(c2[a], Xqa, df_bre(rk));
+        D::pmac(c2[a], df_swap(Xqa), df_bipm(rk));
+      }
+      D::renorm(c1[a]);
+      D::renorm(c2[a]);
     }
-    double* r2 = rtb + ((size_t)k * NB2 + b) * 2;
-    double* s2 = stb + ((size_t)k * NB2 + b) * 2;
-    atomicAdd(r2, D::re_d(a3));
-    atomicAdd(r2 + 1, D::im_d(a3));
-    atomicAdd(s2, D::re_d(a4));
-    atomicAdd(s2 + 1, D::im_d(a4));
+  }
+#pragma unroll
+  for (int a = 0; a < NB2; ++a) {
+    G1[a * NB2 + b] = make_float4(c1[a].h.x, c1[a].h.y, c1[a].l.x, c1[a].l.y);
+    G2[a * NB2 + b] = make_float4(c2[a].h.x, c2[a].h.y, c2[a].l.x, c2[a].l.y);
   }
 }
 
 // nb = 4: one warp per pair, a pair's double-float operators (8 KB) and gradient (8 KB) staged in
 // shared memory by bulk copies (TMA unit) in a 2-stage ring per warp, the per-k vectors of both
-// k-points in shared memory. The same sums as k_adj_pairs_df: lanes 0-15 form conj(P1)^T Xbar[k] and
+// k-points in shared memory. The same sums as k_adj_contract_df and k_adj_grad_df: lanes 0-15 form conj(P1)^T Xbar[k] and
 // conj(P2) Ybar[k] for b = lane, lanes 16-31 P2^T Xbar[k'] and P1 Ybar[k'] for b = lane - 16 (k < k'),
 // reading rows with a per-lane rotation so that the 16 lanes hit distinct banks; then every lane
 // updates 8 elements of G1 and 8 of G2 and stores them to global memory (coalesced). A warp takes a
@@ -603,9 +723,15 @@ __global__ void k_axpy(size_t n, double2* __restrict__ out, const double2* __res
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) out[i] = mk2(fma(c, k[i].x, y[i].x), fma(c, k[i].y, y[i].y));
 }
-__global__ void k_scale(size_t n, double2* __restrict__ out, double c, const double2* __restrict__ x) {
+// out[q][i] = c[q] x[i], q = 0..3
+__global__ void k_scale4(size_t n, double2* __restrict__ out, double4 c, const double2* __restrict__ x) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) out[i] = mk2(c * x[i].x, c * x[i].y);
+  if (i >= n) return;
+  const double2 v = x[i];
+  out[i] = mk2(c.x * v.x, c.x * v.y);
+  out[n + i] = mk2(c.y * v.x, c.y * v.y);
+  out[2 * n + i] = mk2(c.z * v.x, c.z * v.y);
+  out[3 * n + i] = mk2(c.w * v.x, c.w * v.y);
 }
 // y_next = y + h/6 (k1 + 2 k2 + 2 k3 + k4)
 __global__ void k_rk4_final(size_t n, double2* __restrict__ out, const double2* __restrict__ y,

@@ -133,6 +133,8 @@ struct dmd_handle {
   long long version = 0;       // counts changes that a captured step does not follow (groups compare it)
   cudaGraphExec_t g_rk4 = nullptr;
   cudaGraphExec_t g_rk4_rec = nullptr;  // the RK4 step that also copies its stage inputs and sums to d_rec
+  double2* adj_stage = nullptr;         // page-locked staging of the adjoint's dJ/dP (two halves)
+  size_t adj_stage_n = 0;
   double2* d_rec = nullptr;             // [4][nstate] stage inputs, then [4][nk 2 nb^2] forward sums
   std::string err;
   // timing / profiling
@@ -1414,6 +1416,7 @@ void release(dmd_handle* h) {
                   h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (h->adj_stage) cudaFreeHost(h->adj_stage);
   for (int i = 0; i < 8; ++i) {
     if (h->d_obs[i]) cudaFree(h->d_obs[i]);
     if (h->d_f[i]) cudaFree(h->d_f[i]);
@@ -1482,15 +1485,6 @@ int ee_rebuild_nb(dmd_handle* h, const double2* y, const TimeArg& ta, bool eq) {
 // ---------------------------------------------------------------------------------------------
 // adjoint (dmd_adjoint_rk4): work buffers, forward RK4 with stored stage inputs, one VJP
 // ---------------------------------------------------------------------------------------------
-// page-locked host buffer (freed on scope exit)
-struct PinnedStage {
-  void* p = nullptr;
-  bool alloc(size_t bytes) { return cudaHostAlloc(&p, bytes, cudaHostAllocDefault) == cudaSuccess; }
-  ~PinnedStage() {
-    if (p) cudaFreeHost(p);
-  }
-};
-
 // memcpy split over host threads (first-touch page faults of a fresh destination run in parallel)
 void parallel_copy(void* dst, const void* src, size_t bytes) {
   const unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
@@ -1514,7 +1508,8 @@ struct AdjWork {
   std::vector<void*> owned;
   double2 *ck = nullptr, *U = nullptr, *yb = nullptr, *ub = nullptr, *kb = nullptr, *tmp = nullptr;
   double2 *Xb = nullptr, *Yb = nullptr, *rt = nullptr, *st = nullptr, *rtb = nullptr, *stb = nullptr, *G = nullptr;
-  float4* dfv = nullptr;  // double-float form: (x, S(x)) of Xbar, Ybar, rt, st
+  float4* dfv = nullptr;  // double-float form of Xbar, Ybar, rt, st (nb = 2: of the last `slot` stages)
+  int slot = 0, slots = 0;
   double2* A = nullptr;    // forward sums (d_acc) at every stage input of the stretch being reversed
   ~AdjWork() {
     for (void* p : owned) cudaFree(p);
@@ -1585,6 +1580,17 @@ int adj_bulk4_launch(dmd_handle* h, const int2* kk, const float4* dfv, size_t nk
   return adj_bulk4_launch_shape<1, 5>(h, kk, dfv, nk2, rtb, stb, G);
 }
 
+// the gradient's share of the stages since its last pass (nb = 2, double-float)
+int adj_grad(dmd_handle* h, AdjWork& w) {
+  if (w.slot == 0 || h->npair == 0) return DMD_OK;
+  k_adj_grad_df<<<blocks_for(h->npair * 4, 128), 128, 0, h->st>>>(h->npair, h->d_kkraw, w.dfv, (size_t)h->nk * h->nb2, w.slot,
+                                                                  (float4*)w.G);
+  w.slot = 0;
+  h->launches++;
+  CKL();
+  return DMD_OK;
+}
+
 // ybar += VJP_f(u, t)(vbar); kprev += c * VJP_f(u, t)(vbar) when kprev is set. accs: the forward sums
 // at u kept when u was evaluated (the phases are then recomputed from t), or null to evaluate them
 template <int NB>
@@ -1626,14 +1632,21 @@ int adj_vjp_nb(dmd_handle* h, AdjWork& w, const double2* u, double t, const doub
   a.stb = w.stb;
   a.dfv = w.dfv;
   a.nk2 = nk2;
-  k_adj_local<NB><<<blocks_for(h->nk, 128), 128, 0, h->st>>>(a);
+  if (NB == 2 && w.dfv) a.dfv = w.dfv + (size_t)w.slot * 4 * nk2;  // kept for the gradient's next pass
+  if constexpr (NB == 2 || NB == 4) {
+    if (h->nbdm == NB) k_adj_local_el<NB><<<blocks_for((long long)h->nk * NB * NB, 32), 32, 0, h->st>>>(a);
+    else k_adj_local<NB><<<blocks_for(h->nk, 128), 128, 0, h->st>>>(a);
+  } else {
+    k_adj_local<NB><<<blocks_for(h->nk, 128), 128, 0, h->st>>>(a);
+  }
   if (h->npair > 0) {
     const int2* kk = h->use_cb ? h->d_kkraw : h->d_kk;
     if (w.dfv && NB == 4) {  // double-float, one warp per pair, operators and gradient staged by bulk copies
       if ((rc = adj_bulk4_launch(h, kk, w.dfv, nk2, (double*)w.rtb, (double*)w.stb, (float4*)w.G))) return rc;
-    } else if (w.dfv) {  // double-float products on the FP32 pipes
-      k_adj_pairs_df<NB><<<blocks_for(h->npair * NB * NB, 128), 128, 0, h->st>>>(
-          h->npair, kk, h->d_Padf, w.dfv, nk2, (double*)w.rtb, (double*)w.stb, (float4*)w.G);
+    } else if (w.dfv) {  // nb = 2, double-float products on the FP32 pipes
+      k_adj_contract_df<<<blocks_for(h->npair * NB * NB, 128), 128, 0, h->st>>>(h->npair, kk, h->d_Padf, a.dfv, nk2,
+                                                                               (double*)w.rtb, (double*)w.stb);
+      if (++w.slot == w.slots && (rc = adj_grad(h, w))) return rc;
     } else {
       const double2* P = h->use_cb ? h->d_Praw : h->d_P;
       k_adj_pairs<NB><<<blocks_for(h->npair * NB * NB, 128), 128, 0, h->st>>>(h->npair, kk, P, w.Xb, w.Yb, w.rt, w.st,
@@ -2553,10 +2566,11 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
       (rc = w.get(&w.A, (size_t)seglen * 4 * (size_t)h->nk * 2 * h->nb2)))
     return rc;
   const size_t na = (size_t)h->nk * 2 * h->nb2;
-  // double-float handles run the backward pair pass in double-float arithmetic (k_adj_pairs_df)
+  // double-float handles run the backward pair pass in double-float arithmetic (k_adj_contract_df, k_adj_pairs_bulk4)
   const bool dfb = h->prec == DMD_PREC_F64X;
   if (dfb) {
-    if ((rc = w.get(&w.dfv, 8 * nk2))) return rc;
+    w.slots = (int)std::min<int64_t>(kAdjGradStages, 4 * nsteps);
+    if ((rc = w.get(&w.dfv, h->nb == 2 ? (size_t)w.slots * 4 * nk2 : 8 * nk2))) return rc;
     if (!h->d_Padf && (rc = dalloc(h, &h->d_Padf, np))) return rc;
     if (!h->padf_ok && np) {
       k_p_to_df<<<blocks_for((long long)np, 256), 256, 0, h->st>>>(np, h->use_cb ? h->d_Praw : h->d_P, h->d_Padf);
@@ -2659,8 +2673,8 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
         h->launches++;
       }
       const double cst[4] = {dt / 6.0, dt / 3.0, dt / 3.0, dt / 6.0};
-      for (int q = 0; q < 4; ++q) k_scale<<<gn, 256, 0, h->st>>>(n, w.kb + q * n, cst[q], w.yb);
-      h->launches += 4;
+      k_scale4<<<gn, 256, 0, h->st>>>(n, w.kb, make_double4(cst[0], cst[1], cst[2], cst[3]), w.yb);
+      h->launches++;
       CKL();
       const double2* U = w.U + (size_t)(s - n0) * 4 * n;
       const double2* As = w.A + (size_t)(s - n0) * 4 * na;  // forward sums of the four stages
@@ -2676,6 +2690,7 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
                                      obs_weight[j] * h->obs_prefac[slot], w.yb);
     h->launches++;
   }
+  if (h->nb == 2 && dfb && (rc = adj_grad(h, w))) return rc;
   if (dJdP && np) {  // device G is [pair][P1 | P2][nb4] with dJ = Re sum(dP o G): conj(G) in FP64 in place
     if (dfb) k_df_to_f64<<<blocks_for((long long)np, 256), 256, 0, h->st>>>(np, (float4*)w.G, 1);
     else k_conj<<<blocks_for((long long)np, 256), 256, 0, h->st>>>(np, w.G);
@@ -2686,20 +2701,46 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
   if (dJdP && np) {  // out: [P1 | P2][pair][nb4], dJ/dRe P = Re G, dJ/dIm P = -Im G: each half gathered on
                      // the device in chunks and copied contiguously
     const size_t nb4 = (size_t)h->nb4, npair = (size_t)h->npair;
-    const size_t chunk = std::max<size_t>(1, std::min<size_t>(npair, (256u << 20) / (nb4 * 16)));
-    double2* tmp = nullptr;
-    if ((rc = w.get(&tmp, chunk * nb4))) return rc;
-    PinnedStage stage;  // page-locked staging, then a threaded copy into the caller's (pageable) array
-    if (!stage.alloc(chunk * nb4 * 16)) return fail(h, DMD_E_NOMEM, "dmd_adjoint_rk4: page-locked staging buffer");
-    for (int m = 0; m < 2; ++m)
-      for (size_t p0 = 0; p0 < npair; p0 += chunk) {
-        const size_t cnt = std::min(chunk, npair - p0);
-        k_gather_half<<<blocks_for((long long)(cnt * nb4), 256), 256, 0, h->st>>>(cnt * nb4, nb4, w.G + p0 * 2 * nb4, m, tmp);
-        h->launches++;
-        CK(cudaMemcpyAsync(stage.p, tmp, cnt * nb4 * 16, cudaMemcpyDeviceToHost, h->st));
-        CK(cudaStreamSynchronize(h->st));
-        parallel_copy(dJdP + 2 * ((size_t)m * npair + p0) * nb4, stage.p, cnt * nb4 * 16);
+    // two page-locked buffers that the handle keeps (64 MB each at most; allocating them took longer than the copies):
+    // a chunk is gathered and copied out while the host copies the one before into the caller's (pageable) array
+    const size_t half = (64u << 20) / 16;  // elements per buffer
+    const size_t chunk = std::max<size_t>(1, std::min<size_t>(npair, half / nb4)), per = chunk * nb4;
+    if (h->adj_stage_n < 2 * per) {
+      if (h->adj_stage) cudaFreeHost(h->adj_stage);
+      h->adj_stage = nullptr;
+      h->adj_stage_n = 0;
+      if (cudaHostAlloc((void**)&h->adj_stage, 2 * per * 16, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(h, DMD_E_NOMEM, "dmd_adjoint_rk4: page-locked staging buffer");
       }
+      h->adj_stage_n = 2 * per;
+    }
+    double2* tmp = nullptr;
+    if ((rc = w.get(&tmp, 2 * per))) return rc;
+    struct Events {
+      cudaEvent_t e[2] = {nullptr, nullptr};
+      ~Events() {
+        for (cudaEvent_t x : e)
+          if (x) cudaEventDestroy(x);
+      }
+    } ev;
+    for (cudaEvent_t& x : ev.e) CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+    const size_t nch = (npair + chunk - 1) / chunk;
+    auto count = [&](size_t c) { return std::min(chunk, npair - (c % nch) * chunk); };
+    for (size_t c = 0; c <= 2 * nch; ++c) {  // chunks of P1's half, then of P2's
+      if (c < 2 * nch) {
+        const size_t p0 = (c % nch) * chunk, nn = count(c) * nb4, o = (c & 1) * per;
+        k_gather_half<<<blocks_for((long long)nn, 256), 256, 0, h->st>>>(nn, nb4, w.G + p0 * 2 * nb4, (int)(c / nch), tmp + o);
+        h->launches++;
+        CK(cudaMemcpyAsync(h->adj_stage + o, tmp + o, nn * 16, cudaMemcpyDeviceToHost, h->st));
+        CK(cudaEventRecord(ev.e[c & 1], h->st));
+      }
+      if (c > 0) {
+        const size_t d = c - 1, o = (d & 1) * per;
+        CK(cudaEventSynchronize(ev.e[d & 1]));
+        parallel_copy(dJdP + 2 * ((d / nch) * npair + (d % nch) * chunk) * nb4, h->adj_stage + o, count(d) * nb4 * 16);
+      }
+    }
   }
   CK(cudaStreamSynchronize(h->st));
   unsigned int derr = 0;
