@@ -120,7 +120,7 @@ struct dmd_handle {
   double2* d_in1 = nullptr;
   double2* d_out = nullptr;
   double2* d_K = nullptr;      // [6][nstate]
-  double* d_tref = nullptr;    // [t0, h]
+  double* d_tref = nullptr;    // [t0, h, h/2, h/6]
   long long* d_step = nullptr;
   double* d_red = nullptr;     // reduction partials
   int* d_flag = nullptr;
@@ -129,6 +129,7 @@ struct dmd_handle {
   double obs_prefac[8] = {0};
   double t = 0;                // time of the device state
   long long launches = 0, step_launches = 0;  // step_launches: of the captured RK4 step
+  int tc_packed = 0;           // the coordinate blocks of the evaluation are there (k_stage_tc2)
   int eval = 0;                // flag in use: the stage of a fused RK4 step, 0 otherwise
   long long version = 0;       // counts changes that a captured step does not follow (groups compare it)
   cudaGraphExec_t g_rk4 = nullptr;
@@ -305,10 +306,14 @@ cudaError_t herm_pair_attrs() {
 // tensor-core batched form: pack the coordinates, then the Hermitian pass and the gated
 // anti-Hermitian pass (dmd_batched_tc.cuh)
 template <int NB>
-void tc_launches(dmd_handle* h, size_t half) {
+void tc_launches(dmd_handle* h, bool packed) {
   const size_t per = (size_t)h->nrhs * h->nk * NB * NB;
-  k_pack_tc<NB><<<dim3(blocks_for((long long)per, 256), 2), 256, 0, h->st>>>(h->nk, h->nrhs, h->ngroups, h->nmb,
-                                                                         (const float*)h->d_rs, h->d_tcA, h->d_hflag);
+  unsigned int* const flag = h->d_hflag + h->eval;
+  if (!packed) {
+    k_pack_tc<NB><<<dim3(blocks_for((long long)per, 256), 2), 256, 0, h->st>>>(h->nk, h->nrhs, h->ngroups, h->nmb,
+                                                                           (const float*)h->d_rs, h->d_tcA, flag);
+    h->launches++;  // the two passes are counted with the other forms
+  }
   const size_t apart = (size_t)h->ngroups * h->nmb * TC_ABLOCK;
   const size_t astride = (size_t)h->nk * 2 * h->nb2;
   const unsigned g = (unsigned)((size_t)h->ntiles * h->nmb);
@@ -318,14 +323,12 @@ void tc_launches(dmd_handle* h, size_t half) {
     kfwd<<<g, 128, smem, h->st>>>(h->d_tiles, h->ntiles, h->d_tcB, h->d_tcA, h->nmb, h->nrhs, h->nk, accf, astride,
                                   ysign, nullptr, h->d_err);
     kimag<<<g, 128, smem, h->st>>>(h->d_tiles, h->ntiles, h->d_tcB, h->d_tcA + apart, h->nmb, h->nrhs, h->nk, accf,
-                                   astride, ysign, h->d_hflag, h->d_err);
+                                   astride, ysign, flag, h->d_err);
   };
   // pipeline depth (the shape the autotuner chooses): 4, 3 or 2 stages of 48 KB
   if (h->tcst == 3) pass(k_pairs_tc<false, 3, NB>, k_pairs_tc<true, 3, NB>, tc_smem_bytes(3));
   else if (h->tcst == 2) pass(k_pairs_tc<false, 2, NB>, k_pairs_tc<true, 2, NB>, tc_smem_bytes(2));
   else pass(k_pairs_tc<false, 4, NB>, k_pairs_tc<true, 4, NB>, tc_smem_bytes(4));
-  (void)half;
-  h->launches += 1;  // the packing launch; the two passes are counted with the other forms
 }
 
 // the f64 and f64x contraction in fixed point. Against the FP64-pipe form per launch: 0.224 and 0.80 ms on 2.5M
@@ -367,7 +370,7 @@ int launch_pairs(dmd_handle* h) {
       // not exactly Hermitian and returns at once unless the prep kernel raised d_hflag
       const size_t half = (size_t)h->nk * 2 * h->nb2 * h->nrhs;  // coordinates per part
       if (h->use_tc) {
-        tc_launches<NB>(h, half);
+        tc_launches<NB>(h, h->tc_packed);
       } else if (h->nrhs > 1) {  // batched form: reduced-precision arithmetics only (dmd_create)
         const float* rs = (const float*)h->d_rs;
         if (h->prec == DMD_PREC_BF16X2) herm_pair_launches<ArithBF2, NB, 4, 2, 2, 4>(h, rs, half);
@@ -436,6 +439,23 @@ bool fused_step(const dmd_handle* h) {
   return h->use_cb && !h->use_tc && h->nrhs == 1 && h->nbdm == h->nb && !(h->ee_on && h->ee_every);
 }
 
+// The same for the nb = 2 batch on the tensor cores, without coherent and drift terms (k_stage_tc2)
+bool fused_tc(const dmd_handle* h) {
+  return h->use_tc && h->nb == 2 && h->nbdm == 2 && h->picture == DMD_PICTURE_INTERACTION && !h->d_H && !h->d_eq;
+}
+
+TcStage tc_stage(dmd_handle* h, const TimeArg& next, int eval) {
+  TcStage p;
+  p.inv = h->d_inv;
+  p.A = h->d_tcA;
+  p.nmb = h->nmb;
+  p.ph_next = (float2*)h->d_ph + (eval & 1 ? (size_t)h->nk * 4 : 0);  // FP32 phases: two buffers in d_ph's place
+  p.hflag = h->d_hflag + eval;
+  p.phase = h->expt;
+  p.ta = next;
+  return p;
+}
+
 // the finish of a stage, with the coordinates of the next evaluation: at time ta, behind flag `eval`; rkf: a stage of
 // the RKF45 step instead of RK4's
 template <int NB>
@@ -484,7 +504,8 @@ FinishArgs base_finish(dmd_handle* h, const double2* y) {
   a.fref = h->d_fref;
   a.x0y0 = h->d_x0y0;
   a.v0 = h->d_v0;
-  a.ph32 = h->use_tc ? (const float2*)h->d_ph : nullptr;  // the tensor-core prep stores FP32 phases
+  // the tensor-core prep stores FP32 phases; a fused step's odd stages use the second buffer
+  a.ph32 = h->use_tc ? (const float2*)h->d_ph + (h->eval & 1 ? (size_t)h->nk * h->nb2 : 0) : nullptr;
   a.pos = h->use_cb ? h->d_pos : nullptr;
   a.herm = h->use_cb;
   a.lin = h->lin;
@@ -1798,7 +1819,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
       (rc = dalloc(h, &h->d_y, h->nstate)) || (rc = dalloc(h, &h->d_ytmp, h->nstate)) ||
       (rc = dalloc(h, &h->d_y0, h->nstate)) || (rc = dalloc(h, &h->d_in, h->nstate)) ||
       (rc = dalloc(h, &h->d_in1, h->nstate)) || (rc = dalloc(h, &h->d_out, h->nstate)) ||
-      (rc = dalloc(h, &h->d_K, 6 * h->nstate)) || (rc = dalloc(h, &h->d_tref, 2)) ||
+      (rc = dalloc(h, &h->d_K, 6 * h->nstate)) || (rc = dalloc(h, &h->d_tref, 4)) ||
       (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_flag, 1)) || (rc = dalloc(h, &h->d_err, 1)) ||
       (rc = dalloc(h, &h->d_hflag, 4)) || (rc = dalloc(h, &h->d_ph, nk * h->nb2)))
     return bail(rc);
@@ -2133,7 +2154,7 @@ int dmd_get_state(dmd_handle* h, double* t, double* y) {
 // its forward sums (after the contraction) to recA[s].
 static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* recA = nullptr) {
   const size_t na = (size_t)h->nk * 2 * h->nb2;
-  const bool fused = fused_step(h);
+  const bool tc = fused_tc(h), fused = tc || fused_step(h);
   for (int s = 0; s < 4; ++s) {
     TimeArg ta;
     ta.t = 0;
@@ -2154,7 +2175,26 @@ static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* re
     fa.ta = ta;
     if (recU) CK(cudaMemcpyAsync(recU + (size_t)s * h->nstate, in, h->nstate * 16, cudaMemcpyDeviceToDevice, h->st));
     int rc;
-    if (fused) {  // the coordinates are there: from rk4_begin or the finish before
+    if (tc) {
+      TimeArg tn = ta;
+      tn.stage = (s + 1) % 4;
+      tn.ahead = s == 3 ? 1 : 0;
+      const TcStage p = tc_stage(h, tn, tn.stage);
+      k_anti_tc2<<<h->ngroups, 128, 0, h->st>>>(fa, p, h->d_tcA + (size_t)h->ngroups * h->nmb * TC_ABLOCK);
+      h->tc_packed = 1;
+      rc = launch_pairs<2>(h);
+      h->tc_packed = 0;
+      if (!rc) {
+        ProfScope ps(h, 2);
+        int nsm = 0;
+        if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
+        const long long ctas = ((long long)h->ngroups * h->nrhs + 3) / 4;
+        k_stage_tc2<<<(unsigned)std::min<long long>(ctas, (long long)kTcStageCtas * nsm), 128, 0, h->st>>>(fa, p, h->ngroups);
+      }
+      h->launches += 2;
+      h->eval = 0;
+      CKL();
+    } else if (fused) {  // the coordinates are there: from rk4_begin or the finish before
       rc = h->nb == 2 ? launch_pairs<2>(h) : launch_pairs<4>(h);
       if (!rc && recA) CK(cudaMemcpyAsync(recA + (size_t)s * na, h->d_acc, na * 16, cudaMemcpyDeviceToDevice, h->st));
       TimeArg tn = ta;  // the next stage's time; behind stage 3 the next step's first
@@ -2180,7 +2220,8 @@ static int rk4_step_launches(dmd_handle* h, double2* recU = nullptr, double2* re
 
 // before the first of a run of RK4 steps (d_tref, d_step set): the first stage's coordinates of a fused step
 static int rk4_begin(dmd_handle* h) {
-  if (!fused_step(h)) return DMD_OK;
+  const bool tc = fused_tc(h);
+  if (!tc && !fused_step(h)) return DMD_OK;
   CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
   TimeArg ta;
   ta.t = 0;
@@ -2188,12 +2229,19 @@ static int rk4_begin(dmd_handle* h) {
   ta.step = h->d_step;
   ta.stage = 0;
   ta.ahead = 0;
-  return h->nb == 2 ? launch_prep<2>(h, h->d_y, ta) : launch_prep<4>(h, h->d_y, ta);
+  const int rc = h->nb == 2 ? launch_prep<2>(h, h->d_y, ta) : launch_prep<4>(h, h->d_y, ta);
+  if (rc || !tc) return rc;
+  const size_t per = (size_t)h->nrhs * h->nk * 4;
+  k_pack_tc<2><<<dim3(blocks_for((long long)per, 256), 1), 256, 0, h->st>>>(h->nk, h->nrhs, h->ngroups, h->nmb,
+                                                                           (const float*)h->d_rs, h->d_tcA, h->d_hflag);
+  h->launches++;
+  CKL();
+  return DMD_OK;
 }
 
 // after the last one: the coordinates prepared for a step that does not follow leave no flag behind
 static int rk4_end(dmd_handle* h) {
-  if (fused_step(h)) CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
+  if (fused_tc(h) || fused_step(h)) CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
   return DMD_OK;
 }
 
@@ -2201,9 +2249,9 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
   if (!h || nsteps < 0 || !(dt == dt)) return DMD_E_ARG;
   if (nsteps == 0) return DMD_OK;
   CK(cudaSetDevice(h->dev));
-  const double tref[2] = {h->t, dt};
+  const double tref[4] = {h->t, dt, 0.5 * dt, dt / 6.0};
   const long long zero = 0;
-  CK(cudaMemcpyAsync(h->d_tref, tref, 16, cudaMemcpyHostToDevice, h->st));
+  CK(cudaMemcpyAsync(h->d_tref, tref, 32, cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(h->d_step, &zero, 8, cudaMemcpyHostToDevice, h->st));
   // pageable sources: wait so the host values stay valid
   CK(cudaStreamSynchronize(h->st));
@@ -2248,8 +2296,8 @@ int dmd_euler(dmd_handle* h, double dt, int64_t nsteps) {
   if (!h || nsteps < 0) return DMD_E_ARG;
   CK(cudaSetDevice(h->dev));
   for (int64_t s = 0; s < nsteps; ++s) {
-    const double tref[2] = {h->t, dt};
-    CK(cudaMemcpyAsync(h->d_tref, tref, 16, cudaMemcpyHostToDevice, h->st));
+    const double tref[4] = {h->t, dt, 0.5 * dt, dt / 6.0};
+    CK(cudaMemcpyAsync(h->d_tref, tref, 32, cudaMemcpyHostToDevice, h->st));
     FinishArgs fa = base_finish(h, h->d_y);
     fa.mode = 2;
     fa.tref = h->d_tref;
@@ -2600,11 +2648,11 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
     if ((rc = w.get(&ysave, n))) return rc;
     if (!h->d_rec && (rc = dalloc(h, &h->d_rec, 4 * (n + na)))) return rc;
     const double tsave = h->t;
-    const double tref[2] = {t0, dt};
+    const double tref[4] = {t0, dt, 0.5 * dt, dt / 6.0};
     const long long zero = 0;
     CK(cudaMemcpyAsync(ysave, h->d_y, n * 16, cudaMemcpyDeviceToDevice, h->st));
     CK(cudaMemcpyAsync(h->d_y, w.ck, n * 16, cudaMemcpyDeviceToDevice, h->st));
-    CK(cudaMemcpyAsync(h->d_tref, tref, 16, cudaMemcpyHostToDevice, h->st));
+    CK(cudaMemcpyAsync(h->d_tref, tref, 32, cudaMemcpyHostToDevice, h->st));
     CK(cudaMemcpyAsync(h->d_step, &zero, 8, cudaMemcpyHostToDevice, h->st));
     CK(cudaStreamSynchronize(h->st));  // pageable sources
     if (!h->g_rk4_rec) {
@@ -2806,9 +2854,9 @@ int dmd_group_rk4(dmd_group* g, double dt, int64_t nsteps) {
   dmd_handle* h = h0;  // error messages go to the first member
   CK(cudaSetDevice(g->dev));
   for (dmd_handle* hm : g->m) {  // every member's stage times start from its own time
-    const double tref[2] = {hm->t, dt};
+    const double tref[4] = {hm->t, dt, 0.5 * dt, dt / 6.0};
     const long long zero = 0;
-    if (cudaMemcpyAsync(hm->d_tref, tref, 16, cudaMemcpyHostToDevice, hm->st) != cudaSuccess ||
+    if (cudaMemcpyAsync(hm->d_tref, tref, 32, cudaMemcpyHostToDevice, hm->st) != cudaSuccess ||
         cudaMemcpyAsync(hm->d_step, &zero, 8, cudaMemcpyHostToDevice, hm->st) != cudaSuccess ||
         cudaStreamSynchronize(hm->st) != cudaSuccess)
       return fail(hm, DMD_E_CUDA, "group: time reference upload");

@@ -27,6 +27,8 @@
 #include <cuda_bf16.h>
 
 #include "dmd_common.cuh"
+#include "dmd_kernels.cuh"
+#include "dmd_pairs_cb.cuh"
 #include "dmd_tc.cuh"
 #include "dmd_tma.cuh"
 
@@ -210,6 +212,221 @@ __global__ void __launch_bounds__(128, 1) k_pairs_tc(const TcTile* __restrict__ 
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tc_dealloc(tmem, 256);
+}
+
+// ---------------------------------------------------------------------------------------------
+// RK4 stage of the nb = 2 batch in one kernel behind the contraction: the split finish (k_finish<2, 2, true>), the
+// update, and the next stage's coordinates straight into the operand blocks. As three kernels (finish, k_prep_tc,
+// k_pack_tc: 72 + 24 + 15 us per evaluation of 96 states on 5000 k-points, more than the contraction's 64) the state went
+// through memory three times, each thread reloaded its k-point's constants for every state, and the FP64 pipe did 60
+// operations per state and k-point.
+// A warp takes one state's elements of a column group's 8 energy ranks, a lane per element (a thread per k-point needs 128
+// registers: 16 warps per SM and 75 us), and walks states with the k-points' constants and phases in registers; its
+// stores are whole 64-byte halves of an operand row. It takes 45 to 55 us there, the FP64 pipe 71 % busy (the update's own
+// multiply-adds and the exact splits); the RK4 step went from 700 to 487 us (1000 k-points, 16 states: 85 us). Slopes are kept in FP32, which holds them exactly (the finish
+// forms them in FP32; no coherent or drift term here). Conversions and comparisons of doubles run on the FP64 pipe too
+// (with them it was 79 % busy): they are integer operations here, and each real takes one fused multiply-add.
+// ---------------------------------------------------------------------------------------------
+struct TcStage {
+  const int* inv;          // energy rank -> k
+  uint16_t* A;             // coordinate blocks, part 0
+  int nmb;
+  float2* ph_next;         // the next evaluation's phases (two buffers in turn: FinishArgs::ph32 is the other one)
+  unsigned int* hflag;     // the next evaluation's flag
+  int phase;
+  TimeArg ta;              // the next evaluation's time
+};
+
+// (float)x, round to nearest even, in integer arithmetic; outside FP32's normal range (zeros apart) the conversion
+static __device__ __noinline__ float narrow_rare(double x) { return (float)x; }
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), sgn = hi & 0x80000000u;
+  const unsigned e = hi - sgn - (897u << 20);  // exponent (and mantissa) above the smallest normal
+  if (e >= (254u << 20)) return ((hi - sgn) | lo) ? narrow_rare(x) : __int_as_float((int)hi);
+  // 29 bits go: half a unit less one, and one more where the last bit kept is odd
+  const unsigned long long m =
+      ((unsigned long long)(hi - sgn) << 32 | lo) - (896ull << 52) + 0xfffffffull + ((lo >> 29) & 1u);
+  return __int_as_float((int)(sgn | (unsigned)(m >> 29)));
+}
+// (double)x
+static __device__ __noinline__ double widen_rare(float x) { return (double)x; }
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = (unsigned)__float_as_int(x), sgn = b & 0x80000000u, u = b - sgn;
+  if (u - 0x800000u >= 0x7f000000u) return u ? widen_rare(x) : __hiloint2double((int)b, 0);
+  return __hiloint2double((int)(sgn | ((u >> 3) + (896u << 20))), (int)(b << 29));
+}
+// x == y, x == -y (NaN as equal patterns) and x != 0
+__device__ __forceinline__ bool same(double x, double y) {
+  const long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+  return a == b || ((a | b) << 1) == 0;
+}
+__device__ __forceinline__ bool opposite(double x, double y) {
+  const long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+  return (a ^ b) == (long long)0x8000000000000000ull || ((a | b) << 1) == 0;
+}
+__device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+__device__ __forceinline__ void tc_store4(uint16_t* blk, int m, int kk, const float* r) {
+  uint32_t h[2], l[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(r[2 * i], r[2 * i + 1]);
+    const __nv_bfloat162 lo =
+        __floats2bfloat162_rn(__fsub_rn(r[2 * i], __low2float(hi)), __fsub_rn(r[2 * i + 1], __high2float(hi)));
+    h[i] = *reinterpret_cast<const uint32_t*>(&hi);
+    l[i] = *reinterpret_cast<const uint32_t*>(&lo);
+  }
+  *reinterpret_cast<uint2*>(blk + tc_ci(m, kk)) = make_uint2(h[0], h[1]);  // 4 elements: half of a swizzled 16-byte unit
+  *reinterpret_cast<uint2*>(blk + tc_ci(m, kk + 32)) = make_uint2(l[0], l[1]);
+}
+
+// the anti-Hermitian part's coordinate blocks, from the stage's input; gated
+__global__ void __launch_bounds__(128) k_anti_tc2(FinishArgs a, TcStage p, uint16_t* __restrict__ A1) {
+  if (*a.hflag == 0u) return;
+  const int pr = blockIdx.x * 8 + (threadIdx.x & 7);
+  if (pr >= a.nk) return;
+  const int k = p.inv[pr];
+  const float2 D = p.phase ? a.ph32[(size_t)k * 4 + 1] : make_float2(1.f, 0.f);
+  for (int q = threadIdx.x >> 3; q < a.nrhs; q += 16) {
+    const double2* y = a.y + (size_t)q * a.sstride + (size_t)k * 4;
+    const double2 y1 = y[1], y2 = y[2];
+    // A_ij = (rho_ij - conj(rho_ji)) / (2i), times conj(D)
+    const float2 af = make_float2((float)__dmul_rn(__dadd_rn(y1.y, y2.y), 0.5), (float)__dmul_rn(__dsub_rn(y2.x, y1.x), 0.5));
+    const float r[4] = {(float)y[0].y, __fmaf_rn(D.x, af.x, D.y * af.y), __fmaf_rn(D.x, af.y, -D.y * af.x), (float)y[3].y};
+    tc_store4(A1 + ((size_t)blockIdx.x * p.nmb + q / TC_M) * TC_ABLOCK, q % TC_M, (threadIdx.x & 7) * 4, r);
+  }
+}
+
+__device__ __forceinline__ float2 quad_get(float2 v, int lane) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
+// A grid of one wave: every warp takes an equal run of the (column group, state) tasks, states innermost, and reloads
+// the constants where its run enters a group (equal shares of a group's states per block leave a second, nearly empty
+// wave or too few warps: 67 and 84 us).
+constexpr int kTcStageCtas = 8;
+__global__ void __launch_bounds__(128, kTcStageCtas) k_stage_tc2(FinishArgs a, TcStage p, int ngroups) {
+  const int lane = threadIdx.x & 31, e = lane & 3, i = e >> 1, j = e & 1, l0 = lane - e, tl = l0 + 2 * j + i;
+  if (a.hflag && blockIdx.x == 0 && threadIdx.x == 0) *a.hflag = 0u;  // every pair launch of this evaluation has completed
+  const long long tasks = (long long)ngroups * a.nrhs, warps = 4LL * gridDim.x, w = 4LL * blockIdx.x + (threadIdx.x >> 5);
+  const long long t1 = tasks * (w + 1) / warps;
+  const float2 zero = make_float2(0.f, 0.f), one = make_float2(1.f, 0.f);
+  const float pf = (float)(a.prefac * 0.5);
+  const double hs = a.tref[a.stage == 2 ? 1 : a.stage == 3 ? 3 : 2];  // h, h/6, h/2
+  const size_t n = a.sstride * a.nrhs;
+  float2* const K = (float2*)a.K;
+  double2* const out = a.stage < 3 ? a.ytmp : a.ybase;
+  // element (rank, e) of a row: 4 ranks of 4 elements per swizzled 16-byte unit and half
+  const int kk = (lane >> 2) * 4 + e;
+  int group = -1, pr = 0;
+  bool live = false, flag = false;
+  size_t ke = 0;
+  float2 x0 = zero, y0 = zero, v0 = zero, D = one, dn = one;
+  double fi = 0.0;
+  float ffi = 0.f, ffj = 0.f;
+  const long long t0 = tasks * w / warps;
+  int gt = (int)(t0 / a.nrhs), q = (int)(t0 - (long long)gt * a.nrhs) - 1;
+  for (int left = (int)(t1 - t0); left > 0; --left) {
+    if (++q == a.nrhs) {
+      q = 0;
+      ++gt;
+    }
+    if (gt != group) {  // this element's constants
+      group = gt;
+      pr = gt * 8 + (lane >> 2);
+      live = pr < a.nk;
+      if (!live) pr = a.nk - 1;
+      const int k = p.inv[pr];
+      ke = (size_t)k * 4 + e;
+      x0 = a.x0y0 ? a.x0y0[(size_t)k * 8 + e] : zero;
+      y0 = a.x0y0 ? a.x0y0[(size_t)k * 8 + 4 + e] : zero;
+      v0 = a.v0 ? a.v0[ke] : zero;
+      fi = a.fref[2 * (size_t)k + i];
+      ffi = (float)fi;
+      ffj = (float)a.fref[2 * (size_t)k + j];
+      D = (a.phase && i != j) ? a.ph32[ke] : one;
+      if (p.phase) {  // D(0, 1) of the next time
+        const double x = (a.ew[2 * (size_t)k] - a.ew[2 * (size_t)k + 1]) * eval_time(p.ta);
+        float sn, cs;
+        sincosf((float)fma(-6.283185307179586, rint(x * 0.15915494309189535), x), &sn, &cs);
+        dn = make_float2(cs, sn);
+        if (live && q == 0) p.ph_next[ke] = i == j ? one : (i < j ? dn : make_float2(cs, -sn));
+      }
+    }
+    const size_t el = (size_t)q * a.sstride + ke;
+    const float2* Xs = (const float2*)a.acc + (size_t)q * a.astride + (size_t)pr * 8 + e;
+    float2 X = Xs[0], Y = Xs[4];
+    const double2 y = a.y[el], yb = a.stage == 0 ? y : a.ybase[el];
+    // X = (M^H)^-1 X'
+    const float2 xo = quad_get(X, tl), yo = quad_get(Y, tl);
+    if (i < j) {
+      X = make_float2(0.5f * (X.x - xo.y), 0.5f * (X.y + xo.x));
+      Y = make_float2(0.5f * (Y.x - yo.y), 0.5f * (Y.y + yo.x));
+    } else if (i > j) {
+      X = make_float2(0.5f * (xo.x + X.y), 0.5f * (xo.y - X.x));
+      Y = make_float2(0.5f * (yo.x + Y.y), 0.5f * (yo.y - Y.x));
+    }
+    // herm_up(rho - F): upper triangle, real diagonal (the diagonal difference in FP64)
+    float2 dh = i == j ? make_float2(narrow(__dsub_rn(y.x, fi)), 0.f) : make_float2(narrow(y.x), narrow(y.y));
+    const float2 dho = quad_get(dh, tl);
+    if (i > j) dh = make_float2(dho.x, -dho.y);
+    const float2 PXd = fmul(D, X), PYd = fmul(D, Y), PXt = ffma(D, x0, PXd), PYt = ffma(D, y0, PYd);
+    float2 c;
+    if (a.lin) {
+      c = PXd;
+    } else {
+      c = make_float2((1.f - ffi) * PXd.x - ffj * PYd.x, (1.f - ffi) * PXd.y - ffj * PYd.y);
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const float2 d1 = quad_get(dh, l0 + 2 * i + l), m = quad_get(PYt, l0 + 2 * i + l);
+        c = ffma(make_float2(-d1.x, -d1.y), quad_get(PXt, l0 + 2 * l + j), c);
+        c = ffma(make_float2(-m.x, -m.y), quad_get(dh, l0 + 2 * l + j), c);
+      }
+    }
+    // (prefac/2)(c + c^dagger) + D o V0; the (1, 0) element is the exact conjugate of the (0, 1) one
+    const float2 co = quad_get(c, tl);
+    float2 f = make_float2(pf * (c.x + co.x), pf * (c.y - co.y));
+    if (a.v0) f = ffma(D, v0, f);
+    const float2 fo = quad_get(f, tl);
+    if (i > j) f = make_float2(fo.x, -fo.y);
+    double2 yn;
+    if (a.stage < 3) {
+      yn = mk2(fma(hs, widen(f.x), yb.x), fma(hs, widen(f.y), yb.y));
+    } else {  // y + h/6 (k1 + 2 k2 + 2 k3 + k4): the sum as a double-float
+      const float2 k1 = K[el], k2 = K[n + el], k3 = K[2 * n + el];
+      auto sum = [&](float u, float v, float w, float x, double base) {
+        float s, t, r, s2, s3;
+        two_sum(u, __fadd_rn(v, v), s, t);
+        two_sum(s, __fadd_rn(w, w), s2, r);
+        t = __fadd_rn(t, r);
+        two_sum(s2, x, s3, r);
+        return fma(hs, widen(s3), fma(hs, widen(__fadd_rn(t, r)), base));
+      };
+      yn = mk2(sum(k1.x, k2.x, k3.x, f.x, yb.x), sum(k1.y, k2.y, k3.y, f.y, yb.y));
+    }
+    if (live) {
+      out[el] = yn;
+      if (a.stage < 3) K[(size_t)a.stage * n + el] = f;
+    }
+    // the next evaluation's coordinates: conj(D) o (rho - diag(f)), element (0, 1) real part, (1, 0) imaginary part
+    const double2 yt = mk2(__shfl_sync(0xffffffffu, yn.x, tl), __shfl_sync(0xffffffffu, yn.y, tl));
+    flag |= live && (i == j ? nonzero(yn.y) : (!same(yn.x, yt.x) || !opposite(yn.y, yt.y)));
+    float r;
+    if (i == j) {
+      r = narrow(__dsub_rn(yn.x, fi));
+    } else {
+      const float ax = narrow(yn.x), ay = narrow(yn.y), bx = narrow(yt.x), by = narrow(yt.y);
+      const float2 hf = make_float2(0.5f * (ax + bx), i < j ? 0.5f * (ay - by) : 0.5f * (by - ay));
+      r = i < j ? __fmaf_rn(dn.x, hf.x, dn.y * hf.y) : __fmaf_rn(dn.x, hf.y, -dn.y * hf.x);
+    }
+    const __nv_bfloat16 hi = __float2bfloat16_rn(r), lo = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(hi)));
+    if (live) {
+      uint16_t* const blk = p.A + ((size_t)gt * p.nmb + q / TC_M) * TC_ABLOCK;
+      blk[tc_ci(q % TC_M, kk)] = __bfloat16_as_ushort(hi);
+      blk[tc_ci(q % TC_M, kk + 32)] = __bfloat16_as_ushort(lo);
+    }
+  }
+  if (__any_sync(0xffffffffu, flag) && lane == 0) atomicOr(p.hflag, 1u);
 }
 
 }  // namespace dmd

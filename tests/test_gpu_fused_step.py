@@ -134,3 +134,32 @@ def test_fused_rkf45(nb, nk, h0, eps_abs, eps_rel, oracle, built):  # noqa: F811
             t, hg, y = t1, h, yg
             g.set_state(t, y)
     assert rejected > 0 or h0 < 1.0
+
+
+@pytest.mark.parametrize("nk,nrhs,linear,expt,herm", [(1, 2, False, 1, True), (7, 5, False, 1, False), (37, 130, False, 0, True),
+                                                      (64, 16, True, 1, True), (333, 33, False, 1, True)])
+def test_fused_batch(nk, nrhs, linear, expt, herm, oracle, built):  # noqa: F811
+    """k_stage_tc2: partly filled column groups, one and two blocks of states, runs that end inside a group, states that
+    are not Hermitian; against the same steps from the host. Both round the slopes to FP32 in the same operations: the
+    states differ by roundings of their own updates (4 n 2^-53) and by next inputs that round the other way (2^-24 of the
+    change per evaluation)."""
+    from denmat_dynm_development_gb300.dmd import LindbladGPU
+    s = system(oracle, nk, 2, 0.8, 17 * nk + nrhs)
+    rng = np.random.default_rng(6)
+    y = np.concatenate([oracle.y_of(s.dm0)] * nrhs).reshape(nrhs, -1)
+    x = 1e-3 * rng.standard_normal((nrhs, nk, 2, 2)) + 1e-3j * rng.standard_normal((nrhs, nk, 2, 2))
+    if herm:
+        x = 0.5 * (x + np.conj(np.swapaxes(x, 2, 3)))
+    y = (y + (x * s.f_dm[None, :, :, None]).reshape(nrhs, -1).view(np.float64)).reshape(-1)
+    t0, h, n = 7.0 * oracle.fs, 2.0 * oracle.fs, 4
+    with LindbladGPU(nk=nk, nb_dm=2, bstart=0, bend=2, e_dm=s.e_dm, k1st=s.k1st, k2nd=s.k2nd, P1=s.P1, P2=s.P2,
+                     prefac_eph=s.prefac_eph, picture=0, expt=expt, precision="bf16x2", f_ref=s.f_dm, nrhs=nrhs,
+                     linear=linear) as g:
+        ref = host_rk4(g, t0, h, n, y)
+        change = np.abs(ref - y).max()
+        g.set_state(t0, y)
+        g.rk4(h, 1)
+        g.rk4(h, n - 1)
+        out = g.get_state()[1]
+        assert np.abs(out - ref).max() <= 4 * n * 2.0 ** -24 * change + 4 * n * 2.0 ** -53 * np.abs(ref).max()
+        assert g.func(t0, y).tobytes() == g.func(t0, y).tobytes()
