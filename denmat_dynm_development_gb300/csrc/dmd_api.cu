@@ -80,6 +80,8 @@ struct dmd_handle {
   int eek = 0;                 // DMD_FLAG_EE: d_Praw, d_kkraw and d_dst kept for the e-e model
   // sparse form (DMD_FLAG_SPARSE): per k-point the products of its output threads, lane-interleaved
   int use_sp = 0;
+  int sp_fx = 0, sp_emax = 0;        // elements in fixed point; exponent of the largest
+  int sp_split = 1;                  // threads per list
   long long sp_nel = 0, sp_nslot = 0;  // stored elements (both directions), ELL slots with padding
   long long* d_sp_base = nullptr;    // [nk] first slot of each k-point
   int* d_sp_len = nullptr;           // [nk] products per thread (padded)
@@ -359,8 +361,19 @@ int launch_pairs(dmd_handle* h) {
   if (h->npair == 0) return DMD_OK;
   ProfScope ps(h, 1);
   if (h->use_sp) {  // stored elements only, one thread per output element of every k-point
-    k_pairs_sparse<NB><<<blocks_for((long long)h->nk * 2 * NB * NB, 256), 256, 0, h->st>>>(
-        h->nk, h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_rs, h->d_acc);
+    const long long nthr = (long long)h->nk * 2 * NB * NB;
+    if (!h->sp_fx)
+      k_pairs_sparse<NB><<<blocks_for(nthr, 256), 256, 0, h->st>>>(h->nk, h->d_sp_base, h->d_sp_len, h->d_sp_val,
+                                                                   h->d_sp_gidx, h->d_rs, h->d_acc);
+    else {
+      const auto k = h->sp_split == 1   ? k_pairs_sparse_fx<NB, 1>
+                     : h->sp_split == 2 ? k_pairs_sparse_fx<NB, 2>
+                     : h->sp_split == 4 ? k_pairs_sparse_fx<NB, 4>
+                                        : k_pairs_sparse_fx<NB, 8>;
+      k<<<blocks_for(nthr, 256 / h->sp_split), 256, 0, h->st>>>(h->nk, h->sp_emax, h->d_sp_base, h->d_sp_len,
+                                                               (const int4*)h->d_sp_val, (const unsigned*)h->d_sp_gidx,
+                                                               h->d_rs, h->d_acc);
+    }
   } else if (!h->use_cb) {
     const long long nthr = h->npair * 4LL * NB * NB;
     k_pairs_f64_atomic<NB><<<blocks_for(nthr, 256), 256, 0, h->st>>>(h->npair, h->d_kk, h->d_P, h->d_rs, h->d_acc);
@@ -1204,6 +1217,29 @@ int upload_pairs_sparse(dmd_handle* h, const dmd_desc* d) {
   CK(cudaMemcpy(h->d_sp_val, val.data(), val.size() * 16, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_sp_gidx, gidx.data(), gidx.size() * 4, cudaMemcpyHostToDevice));
   h->pair_bytes = (int64_t)(nslot * 20 + (long long)nk * 12);
+  // fixed point unless an element is infinite or a coordinate's index leaves no room for the exponent
+  double mx = 0.0;
+  bool fin = true;
+  for (const double2& v : ev) {
+    const double m = std::max(std::fabs(v.x), std::fabs(v.y));
+    fin = fin && std::isfinite(v.x) && std::isfinite(v.y);
+    mx = std::max(mx, m);
+  }
+  if (fin && (long long)nk * TPR <= 1LL << (32 - kSpDBits) && nslot > 0) {
+    std::frexp(mx, &h->sp_emax);
+    k_sparse_quantise<<<blocks_for(nslot, 256), 256, 0, h->st>>>(nslot, h->sp_emax, h->d_sp_val, h->d_sp_gidx);
+    CKL();
+    CK(cudaStreamSynchronize(h->st));
+    h->sp_fx = 1;
+    // threads per list: 8 while they all fit on the chip at once (3 blocks of 256 per SM; 100 k-points, nb = 4: 58 us per
+    // RK4 step, 72 with one thread), else as many as leave each 10 products (2000 k-points: 147 products 267 us with
+    // 8 threads, 283 with 4, 340 with 1; 17 products 136, 113, 95; 500 k-points, 42 products 90, 76, 103)
+    int nsm = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
+    const long long nthr = (long long)nk * TPR;
+    for (int s = 8; s > 1 && h->sp_split == 1; s /= 2)
+      if ((s == 8 && nthr * s <= nsm * 768LL) || nslot >= nthr * s * 10) h->sp_split = s;
+  }
   return DMD_OK;
 }
 

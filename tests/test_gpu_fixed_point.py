@@ -117,3 +117,47 @@ def test_operators_without_a_fixed_point_form(what, oracle, built):
         if what == "weak k-point":
             assert 0 < np.abs(ref[11]).max() < 1e-20 * np.abs(ref).max()
             assert np.abs(out[11] - ref[11]).max() < 1e-11 * np.abs(ref[11]).max()
+
+
+@pytest.mark.parametrize("nk,nb,density,fill,spread", [(1, 4, 1.0, 1.0, 0.0), (13, 3, 1.0, 0.3, 40.0), (40, 4, 0.5, 0.3, 60.0),
+                                                       (460, 4, 0.02, 0.25, 20.0), (1000, 4, 0.001, 0.5, 20.0),
+                                                       (70, 2, 1.0, 1.0, 0.0), (2000, 1, 1.0, 1.0, None)])
+def test_sparse_form(nk, nb, density, fill, spread, oracle, built):
+    """k_pairs_sparse_fx: lists shorter than a chunk and long ones, 1 to 8 threads per list, elements of one list 2^-spread
+    apart (a scale per list would lose them), sums that outgrow their exponent (None: 1.9 in every element); against the dense
+    FP64-pipe form per k-point, and what a non-finite coordinate reaches"""
+    from denmat_dynm_development_gb300.dmd import LindbladGPU
+    s = system(oracle, nk, nb, density, 7 * nk + nb)
+    rng = np.random.default_rng(nk)
+    for name in ("P1", "P2"):
+        P = np.array(getattr(s, name))
+        P = np.where(P == 0.0, 1e-30, P) * np.exp2(-(spread or 0.0) * rng.random(P.size))
+        P = np.full(P.size, 1.9 + 0.0j) if spread is None else np.where(rng.random(P.size) < fill, P, 0.0)
+        setattr(s, name, P)
+    kw = dict(nk=s.nk, nb_dm=s.nb_dm, bstart=s.bstart, bend=s.bend, e_dm=s.e_dm, k1st=s.k1st, k2nd=s.k2nd, P1=s.P1, P2=s.P2,
+              prefac_eph=s.prefac_eph, picture=0, expt=1, precision="f64")
+    y = oracle.y_of(s.dm0)
+    t = 13.0 * oracle.fs
+    with LindbladGPU(sparse=True, **kw) as g, LindbladGPU(ee_flag=nb in (2, 4), **kw) as p:
+        for v in (y, y * (1.0 + 1e-2 * rng.standard_normal(y.size))):
+            assert per_k(g.func(t, v), p.func(t, v), nk) < 1e-11
+        np.testing.assert_array_equal(g.func(t, 0.0 * y), p.func(t, 0.0 * y))  # (zeros of either sign)
+        if fill == 1.0:  # (a zero that is not stored takes no NaN)
+            for bad in (np.nan, np.inf):
+                v = y.copy()
+                v[2 * nb * nb * (nk // 2)] = bad
+                np.testing.assert_array_equal(np.isfinite(g.func(t, v)), np.isfinite(p.func(t, v)))
+
+
+def test_sparse_form_with_an_infinite_element(oracle, built):
+    """operators without a fixed-point form stay on the FP64 pipe"""
+    from denmat_dynm_development_gb300.dmd import LindbladGPU
+    s = system(oracle, 20, 4, 1.0, 3)
+    s.P1 = np.array(s.P1)
+    s.P1[5] = np.inf
+    kw = dict(nk=s.nk, nb_dm=s.nb_dm, bstart=s.bstart, bend=s.bend, e_dm=s.e_dm, k1st=s.k1st, k2nd=s.k2nd, P1=s.P1, P2=s.P2,
+              prefac_eph=s.prefac_eph, picture=0, expt=1, precision="f64")
+    y = oracle.y_of(s.dm0)
+    with LindbladGPU(sparse=True, **kw) as g:
+        out = g.func(0.0, y)
+    assert not np.isfinite(out).all() and np.isfinite(out).any()
