@@ -1233,7 +1233,7 @@ int upload_pairs_sparse(dmd_handle* h, const dmd_desc* d) {
     h->sp_fx = 1;
     // threads per list: 8 while they all fit on the chip at once (3 blocks of 256 per SM; 100 k-points, nb = 4: 58 us per
     // RK4 step, 72 with one thread), else as many as leave each 10 products (2000 k-points: 147 products 267 us with
-    // 8 threads, 283 with 4, 340 with 1; 17 products 136, 113, 95; 500 k-points, 42 products 90, 76, 103)
+    // 8 threads, 283 with 4, 340 with 1, before the index words were loaded ahead; 17 products 136, 113, 95; 500 k-points, 42 products 90, 76, 103)
     int nsm = 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
     const long long nthr = (long long)nk * TPR;

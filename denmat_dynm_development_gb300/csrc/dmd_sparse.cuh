@@ -34,7 +34,8 @@
 //   sum       (A0 + A1 2^-32) 2^(emax + T - 1077),  A0 += h rh,  A1 += h rl + l rh, exact in 64 bits for the 8 real
 //             terms of 4 products (A0 2^58 beside the 2^61 at which it is shifted, A1 8 (2^59 + 2^58))
 // It takes 57 us there (43 % of the HBM rate: what bounds it is the latency of index, then coordinate, with 21 warps
-// per SM); an RK4 step of 2000 k-points went from 702 to 267 us, of 100 from 206 to 60.
+// per SM; the next chunk's index words are loaded ahead: 10 us of the step's 267); an RK4 step of 2000 k-points went from
+// 702 to 257 us, of 100 from 206 to 60.
 // The dropped l rl is at most 2^-57 of the largest product, the bits lost to a shift 2^-56 of it, and a sum is rounded
 // to FP64 once.
 #pragma once
@@ -98,6 +99,11 @@ __global__ void __launch_bounds__(256) k_pairs_sparse_fx(int nk, int emax, const
   const unsigned* ip = gidx + (k < nk ? base[k] + l : 0);
   long long x0 = 0, x1 = 0, y0 = 0, y1 = 0;  // A0, A1 of the real and the imaginary part
   int T = kSpT0, top = 0;
+  unsigned un[4];  // the next chunk's index words
+  auto index = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) un[i] = j + i < L ? __ldcs(ip + (size_t)(j + i) * TPR) : 0u;
+  };
   auto chunk = [&](int j, auto tail) {
     int4 v[4];
     unsigned u[4];
@@ -105,11 +111,11 @@ __global__ void __launch_bounds__(256) k_pairs_sparse_fx(int nk, int emax, const
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool ok = !decltype(tail)::value || j + i < L;
+      u[i] = un[i];
+      r[i] = ok ? __ldg(rs + (u[i] >> kSpDBits)) : mk2(0.0, 0.0);
       v[i] = ok ? __ldcs(vp + (size_t)(j + i) * TPR) : make_int4(0, 0, 0, 0);
-      u[i] = ok ? __ldcs(ip + (size_t)(j + i) * TPR) : 0u;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r[i] = !decltype(tail)::value || j + i < L ? __ldg(rs + (u[i] >> kSpDBits)) : mk2(0.0, 0.0);
+    index(j + 4 * S);
     int gx[4], gy[4], gm = T;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -142,6 +148,7 @@ __global__ void __launch_bounds__(256) k_pairs_sparse_fx(int nk, int emax, const
     y1 = fx_fold(y0, y1);
   };
   int j = 4 * s;
+  index(j);
   for (; j + 4 <= L; j += 4 * S) chunk(j, std::false_type());
   if (j < L) chunk(j, std::true_type());
   double2 sum;
