@@ -483,12 +483,13 @@ int launch_finish_prep(dmd_handle* h, const FinishArgs& a, const TimeArg& ta, in
   p.hflag = h->d_hflag + eval;
   p.phase = h->expt;
   p.lin = h->lin;
+  p.same_time = !rkf && a.ta.stage == 1 && ta.stage == 2;  // both at t + h / 2
   p.ta = ta;
   const unsigned g = blocks_for((long long)h->nk * NB * NB, 32);
   auto go = [&](auto arith) {
     typedef decltype(arith) A;
-    if (rkf) k_finish_el<NB, A, true, true><<<g, 32, 0, h->st>>>(a, p, *rkf);
-    else k_finish_el<NB, A, true><<<g, 32, 0, h->st>>>(a, p, RkfStage());
+    if (rkf) k_finish_el<NB, A, true, true><<<g, 64, 0, h->st>>>(a, p, *rkf);
+    else k_finish_el<NB, A, true><<<g, 64, 0, h->st>>>(a, p, RkfStage());
   };
   if (h->fmt == DMD_PREC_F64X) go(ArithDF());
   else if (deviation_form(h->prec)) go(ArithF32());

@@ -23,6 +23,7 @@ struct NextPrep {
   const double* fref;    // deviation and linearized forms
   unsigned int* hflag;   // the next evaluation's flag (FinishArgs::hflag: this one's)
   int phase, lin;
+  int same_time;         // the next time is this evaluation's: its phases stay
   TimeArg ta;
 };
 
@@ -42,16 +43,28 @@ __device__ __forceinline__ double2 group_get(double2 v, int lane) {
 
 // A: coordinate type of the next evaluation (PREP); RKF: stages of the RKF45 step instead of RK4's
 template <int NB, typename A, bool PREP, bool RKF = false>
-__global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p, RkfStage r) {
+__global__ void __launch_bounds__(PREP ? 64 : 32) k_finish_el(FinishArgs a, NextPrep p, RkfStage r) {
   constexpr int NB2 = NB * NB;
-  const int lane = threadIdx.x, e = lane % NB2, i = e / NB, j = e % NB, g0 = lane - e;  // group's first lane
+  __shared__ double2 next_d[PREP ? 32 : 1];
+  const int lane = threadIdx.x & 31, e = lane % NB2, i = e / NB, j = e % NB, g0 = lane - e;  // group's first lane
   const int ji = j * NB + i, tl = g0 + ji;                                             // the transposed element's lane
   const int kl = (blockIdx.x * 32 + lane) / NB2;
   const bool live = kl < a.nk;  // dead groups still take part in the shuffles
   const int k = live ? kl : a.nk - 1;
+  const size_t el = (size_t)k * NB2 + e;
+  const bool new_ph = PREP && p.phase && !p.same_time;
+  if (PREP && threadIdx.x >= 32) {  // second warp: the next phases
+    if (!new_ph) return;
+    double2 dk = mk2(1.0, 0.0);
+    if (i < j) dk = ccis((a.ew[(size_t)k * NB + i] - a.ew[(size_t)k * NB + j]) * eval_time(p.ta));
+    next_d[lane] = dk;
+    __syncthreads();  // (and the first warp has read this evaluation's)
+    if (live && i <= j) p.ph[el] = dk;
+    if (live && i < j) p.ph[(size_t)k * NB2 + ji] = cconj(dk);
+    return;
+  }
   if (a.hflag && blockIdx.x == 0 && lane == 0) *a.hflag = 0u;  // every pair launch of this evaluation has completed
   const double t = eval_time(a.ta);
-  const size_t el = (size_t)k * NB2 + e;
   const double2 y = a.y[el];
   const double2 d = (a.want_eph && a.ph && i != j) ? a.ph[el] : mk2(1.0, 0.0);  // D_k(i, j)
   double2 f = mk2(0.0, 0.0);
@@ -183,6 +196,7 @@ __global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p, RkfS
   }
   if constexpr (PREP) {
     const double2 vo = group_get<NB>(yn, tl);  // the transposed element
+    if (new_ph) __syncthreads();
     if (!live) return;
     typedef typename A::relem V;
     p.acc[ax] = p.acc0 ? p.acc0[ax] : mk2(0.0, 0.0);
@@ -191,7 +205,6 @@ __global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p, RkfS
     V* const ra = rh + (size_t)a.nk * 2 * NB2;
     constexpr bool F64C = std::is_same<V, double>::value;
     if (i == j) {
-      if (p.phase) p.ph[el] = mk2(1.0, 0.0);
       // H_ii = Re rho_ii, A_ii = Im rho_ii; 1 - rho: (1 - Re rho_ii, -Im rho_ii) (set_oneminusdm)
       if (p.fref) {
         const double dv = __dsub_rn(yn.x, p.fref[(size_t)k * NB + i]);
@@ -206,13 +219,7 @@ __global__ void __launch_bounds__(32) k_finish_el(FinishArgs a, NextPrep p, RkfS
       if (yn.y != 0.0) atomicOr(p.hflag, DMD_HFLAG_NONHERM);
       if (F64C && !(isfinite(yn.x) && isfinite(yn.y))) atomicOr(p.hflag, DMD_HFLAG_NONFINITE);
     } else if (i < j) {
-      double2 dn = mk2(1.0, 0.0);
-      if (p.phase) {
-        const double2 dk = ccis((a.ew[(size_t)k * NB + i] - a.ew[(size_t)k * NB + j]) * eval_time(p.ta));
-        p.ph[el] = dk;
-        p.ph[(size_t)k * NB2 + ji] = cconj(dk);
-        dn = cconj(dk);
-      }
+      const double2 dn = new_ph ? cconj(next_d[lane]) : p.phase ? cconj(d) : mk2(1.0, 0.0);
       // H_ij = (rho_ij + conj(rho_ji)) / 2, A_ij = (rho_ij - conj(rho_ji)) / (2i); exact for Hermitian rho
       const double2 hij = mk2(__dmul_rn(__dadd_rn(yn.x, vo.x), 0.5), __dmul_rn(__dsub_rn(yn.y, vo.y), 0.5));
       const double2 dif = mk2(__dsub_rn(yn.x, vo.x), __dadd_rn(yn.y, vo.y));
