@@ -867,6 +867,19 @@ int fx_convert(dmd_handle* h) {
   return DMD_OK;
 }
 
+// Row blocks per work item of the fixed-point contraction (two warps per item, 8 items resident per SM). A row block takes
+// the same time however few pairs it holds, and an item's prologue and flush as long as two or three. So: as
+// few row blocks as make one wave while that is at most 16 (nb = 4, whose row blocks are four times the work: 4), else a third
+// of what one wave takes, within 8 to 16 (2 to 4). us per RK4 step, against items filled by pairs: 2661 row blocks
+// (500 k-points) 83, 122; 12264 175, 234; 18305 225, 311; 33743 392, 399; 87184 880, 929; nb = 4: 2328 157, 221; 7456 437, 528.
+int fx_rows(const dmd::PairLayout& L, int nb, int nsm) {
+  const long long wave = 8LL * nsm, hi = nb == 2 ? 16 : 4;
+  for (int r = 1; r <= hi; ++r)
+    if (dmd::count_items(L, r) <= wave) return r;
+  const long long third = ((long long)L.rb.size() + 3 * wave - 1) / (3 * wave);
+  return (int)std::min(hi, std::max(hi / 2, third));
+}
+
 struct CbDst;
 int fill_pairs_cb(dmd_handle* h, PairSource& src, const std::vector<CbDst>& dst, bool dev);
 
@@ -880,20 +893,13 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   dmd::PairLayout L;
   const int G = h->nb2 / 4, W = 32 / G;  // lanes per pair, columns per column block
   // pairs per work item: 512 (a warp's share on large workloads), fewer when the workload would
-  // not give every SM its 16 resident warps. The fixed-point contraction (two warps per item, whose digits
-  // cost as much as a row block or two) takes items of up to 32 row blocks while they number 2.5 per SM:
-  // 66 against 81 us per launch on 398k pairs (437 and 778 items), 235 against 252 on 2.5M
-  int ppi = 512 / G;
-  {
-    int nsm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
-    const long long want = (long long)nsm * 16;
-    const bool fx = h->fmt == DMD_PREC_F64 && !h->eek;
-    if (fx && h->npair * G * 2 / (32 * 32) > nsm * 5LL) ppi = 32 * 32 / G;
-    else if (h->npair / ppi < want) ppi = (int)std::max<long long>(1, h->npair / want);
-  }
+  // not give every SM its 16 resident warps
+  int ppi = 512 / G, nsm = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
+  if (h->npair / ppi < nsm * 16LL) ppi = (int)std::max<long long>(1, h->npair / (nsm * 16LL));
   if (!dmd::build_pair_layout(h->nk, nb, ew.data(), h->npair, d->k1st, d->k2nd, ppi, W, L))
     return fail(h, DMD_E_ARG, "k-pair index out of range");
+  if (h->fmt == DMD_PREC_F64 && !h->eek) dmd::pack_rows(L, fx_rows(L, nb, nsm));
   h->nitems = (int)L.items.size();
   h->nrb = (long long)L.rb.size();
   if (nb == 2) {

@@ -93,4 +93,29 @@ bool build_pair_layout(int nk, int nb, const double* e_w, long long npair, const
   return true;
 }
 
+// the runs of row blocks of one column block, as f(J, first, end)
+template <typename F>
+static void column_runs(const std::vector<WorkItem>& items, F f) {
+  for (size_t i = 0; i < items.size();) {
+    size_t e = i;
+    while (e < items.size() && items[e].J == items[i].J) ++e;
+    f(items[i].J, items[i].rb0, items[e - 1].rb1);
+    i = e;
+  }
+}
+
+long long count_items(const PairLayout& L, int rows) {
+  long long n = 0;
+  column_runs(L.items, [&](int, int r0, int r1) { n += (r1 - r0 + rows - 1) / rows; });
+  return n;
+}
+
+void pack_rows(PairLayout& L, int rows) {
+  std::vector<WorkItem> items;
+  column_runs(L.items, [&](int J, int r0, int r1) {
+    for (int r = r0; r < r1; r += rows) items.push_back({J, r, std::min(r + rows, r1)});
+  });
+  L.items.swap(items);
+}
+
 }  // namespace dmd

@@ -51,4 +51,9 @@ struct PairLayout {
 bool build_pair_layout(int nk, int nb, const double* e_w, long long npair, const uint64_t* k1, const uint64_t* k2,
                        int pairs_per_item, int width, PairLayout& L);
 
+// Repacks the row blocks into items of `rows` row blocks (<= kMaxRowBlocksPerItem) however few pairs they hold;
+// count_items: how many that makes
+void pack_rows(PairLayout& L, int rows);
+long long count_items(const PairLayout& L, int rows);
+
 }  // namespace dmd
