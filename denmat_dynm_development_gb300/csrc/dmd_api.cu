@@ -867,15 +867,20 @@ int fx_convert(dmd_handle* h) {
   return DMD_OK;
 }
 
-// Row blocks per work item of the fixed-point contraction (two warps per item, 8 items resident per SM). A row block takes
-// the same time however few pairs it holds, and an item's prologue and flush as long as two or three. So: as
-// few row blocks as make one wave while that is at most 16 (nb = 4, whose row blocks are four times the work: 4), else a third
-// of what one wave takes, within 8 to 16 (2 to 4). us per RK4 step, against items filled by pairs: 2661 row blocks
-// (500 k-points) 83, 122; 12264 175, 234; 18305 225, 311; 33743 392, 399; 87184 880, 929; nb = 4: 2328 157, 221; 7456 437, 528.
-int fx_rows(const dmd::PairLayout& L, int nb, int nsm) {
-  const long long wave = 8LL * nsm, hi = nb == 2 ? 16 : 4;
+// Row blocks per work item (0: items filled by pairs). A row block takes the same time however few pairs it holds, and
+// an item's prologue and reverse flush as long as two or three. So: as few row blocks as make one wave while that is at
+// most 16 (nb = 4, whose row blocks are four times the work: 4), else a third of what one wave takes, within 8 to 16 (2
+// to 4). The wave, per SM: 8 items of two warps in fixed point; 16 (nb = 4: 20, all that are resident) of one warp in FP32,
+// where nb = 2 takes one or two row blocks only while the flushes' atomics (512 per item) stay few. us per RK4 step, against
+// items filled by pairs: fixed point, 2661 row blocks (500 k-points) 83, 122; 12264 175, 234; 18305 225, 311; 33743 392, 399;
+// 87184 880, 929; nb = 4: 2328 157, 221; 7456 437, 528. FP32, 2661 row blocks 92, 140; 16378 146, 219; 33771 223, 291;
+// 87184 517, 604; nb = 4: 2328 105, 123; 7456 207, 233. The FP64-pipe forms and the batches keep their items.
+int item_rows(const dmd_handle* h, const dmd::PairLayout& L, int nsm) {
+  const bool fx = h->fmt == DMD_PREC_F64 && !h->eek, f32 = deviation_form(h->prec) && h->nrhs == 1;
+  if (!fx && !f32) return 0;
+  const long long wave = (fx ? 8LL : h->nb == 2 ? 16LL : 20LL) * nsm, hi = h->nb == 2 ? 16 : 4;
   for (int r = 1; r <= hi; ++r)
-    if (dmd::count_items(L, r) <= wave) return r;
+    if (dmd::count_items(L, r) <= (f32 && h->nb == 2 && r < 3 ? wave * 2 / 5 : wave)) return r;
   const long long third = ((long long)L.rb.size() + 3 * wave - 1) / (3 * wave);
   return (int)std::min(hi, std::max(hi / 2, third));
 }
@@ -899,7 +904,7 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   if (h->npair / ppi < nsm * 16LL) ppi = (int)std::max<long long>(1, h->npair / (nsm * 16LL));
   if (!dmd::build_pair_layout(h->nk, nb, ew.data(), h->npair, d->k1st, d->k2nd, ppi, W, L))
     return fail(h, DMD_E_ARG, "k-pair index out of range");
-  if (h->fmt == DMD_PREC_F64 && !h->eek) dmd::pack_rows(L, fx_rows(L, nb, nsm));
+  if (const int rows = item_rows(h, L, nsm)) dmd::pack_rows(L, rows);
   h->nitems = (int)L.items.size();
   h->nrb = (long long)L.rb.size();
   if (nb == 2) {
