@@ -18,11 +18,10 @@ The headline arithmetic is the reference's: plain FP64 (P complex128, FP64 multi
               the RK4 combination in C loops (dmdh_rk4_func) and every RHS call copies y in and
               dydt out (page-locked buffers)
   roofline    k-pair contraction kernel: algorithmic work per launch / its mean event-timed
-              duration, against the ceiling that binds it -- the FP64 multiply-add rate measured in
-              this process for the FP64 form (its work is FP64 multiply-adds; the HBM fraction is
-              reported beside it), the measured HBM copy bandwidth for the other forms
-  forms       the other arithmetics of the same contraction on the same workload (f64x: FP32
-              pairs; f32 and bf16x2: reduced-precision storage with rho as a deviation from f),
+              duration, against the measured HBM copy bandwidth (the FP64 forms multiply in block fixed
+              point on the integer pipes; the FP64 pipe's rate is reported beside it)
+  forms       the other arithmetics of the same contraction on the same workload (f64x: shares the
+              FP64 form's contraction; f32 and bf16x2: reduced-precision storage with rho as a deviation from f),
               each with its steps/s, roofline and RHS error against the oracle's FP64 RHS
   cpu_baseline the oracle port of the reference's RHS on this host (test infrastructure): one RK4
               step of the full workload on one core; its first RHS is also the reference the
@@ -199,7 +198,8 @@ def measured_peak():
 def profile_traffic(precision):
     """DRAM bytes per pair-kernel launch from the committed ncu summary of this arithmetic, as
     (bytes, npair of the captured workload); scaled by the caller to the benchmarked workload."""
-    p = os.path.join(ROOT, "profiles", "pairs_herm_%s_gaas_nk16k.md" % precision)
+    name = "pairs_fx_f64_gaas_nk10k.md" if precision in ("f64", "f64x") else "pairs_herm_%s_gaas_nk16k.md" % precision
+    p = os.path.join(ROOT, "profiles", name)
     try:
         vals = {}
         with open(p) as f:
@@ -411,26 +411,22 @@ def kernel_profile(g, h, steps):
 
 
 def roofline_of(prec, nb, npair, nk, pair_ms, peaks, traffic):
-    """Roofline of the contraction kernel. FP64: bound by the FP64 multiply-add rate measured in
-    this process (its algorithmic flops per launch / the event-timed launch); the HBM fraction of its
-    algorithmic bytes is reported beside it. Other forms: HBM."""
+    """Roofline of the contraction kernel: its algorithmic bytes per event-timed launch against the HBM rate. The FP64
+    forms multiply on the integer pipes (k_pairs_fx); their FP64-equivalent flops are reported beside it with the rate
+    that the FP64 pipe would allow."""
     hbm, hbm_kind = peaks["hbm"]
     bpl = algorithmic_bytes(nb, npair, nk, ELEM_BYTES[prec])
     gbs = bpl / (pair_ms * 1e-3) / 1e9
-    r = {"kernel": "k-pair contraction (k_pairs_herm, %s)" % prec, "avg_launch_ms": pair_ms, "bytes_per_launch": bpl,
-         "traffic": traffic}
-    if prec == "f64":
+    fx = prec in ("f64", "f64x")
+    r = {"kernel": "k-pair contraction (%s, %s)" % ("k_pairs_fx" if fx else "k_pairs_herm", prec), "avg_launch_ms": pair_ms,
+         "bytes_per_launch": bpl, "traffic": traffic, "bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s",
+         "frac": gbs / hbm, "peak_kind": hbm_kind}
+    if fx:
         fl = algorithmic_flops(nb, npair)
-        tf = fl / (pair_ms * 1e-3) / 1e12
-        r.update({"bound": "fp64", "achieved": tf, "peak": peaks["fp64"], "unit": "TFLOP/s",
-                  "frac": tf / peaks["fp64"], "peak_kind": "measured in-process (dmd_peak_fma, FP64 FMA)",
-                  "flops_per_launch": fl, "hbm_achieved_gbs": gbs, "hbm_peak_gbs": hbm, "hbm_frac": gbs / hbm,
-                  "hbm_peak_kind": hbm_kind,
-                  "binding": "FP64 pipe: HBM alone would allow %.3f ms per launch, the measured FP64 rate %.3f ms"
-                             % (bpl / (hbm * 1e9) * 1e3, fl / (peaks["fp64"] * 1e12) * 1e3)})
-    else:
-        r.update({"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
-                  "peak_kind": hbm_kind})
+        r.update({"flops_per_launch": fl, "fp64_equivalent_tflops": fl / (pair_ms * 1e-3) / 1e12,
+                  "fp64_pipe_tflops": peaks["fp64"],
+                  "binding": "HBM: %.3f ms per launch; the FP64 pipe would take %.3f ms (block fixed point on the integer "
+                             "pipes instead)" % (bpl / (hbm * 1e9) * 1e3, fl / (peaks["fp64"] * 1e12) * 1e3)})
     return r
 
 
@@ -540,7 +536,7 @@ def run_gpu(args, w, rank, world, dist):
 
 
 ELEM_BYTES = {"f64": 16, "f64x": 16, "f32": 8, "bf16x2": 8}
-DTYPE = {"f64": "f64", "f64x": "f64 (fp32-pair emulated)", "f32": "f32 (P complex64, rho as deviation from f)",
+DTYPE = {"f64": "f64", "f64x": "f64 (block fixed point, as f64)", "f32": "f32 (P complex64, rho as deviation from f)",
          "bf16x2": "bf16 hi+lo (P 8 B/complex, rho as deviation from f)"}
 
 
@@ -671,7 +667,7 @@ def run_adjoint(args):
     err = np.abs(grad - fd) / np.abs(fd)
     line = {"metric": "adjoint: dS_z(t_f)/d(6 mode scales, n_imp scale), t_f = %g ps" % args.adj_tf_ps,
             "value": adj_s, "unit": "s (forward with checkpoints + backward, 7 gradients)", "n_gpus": 1,
-            "higher_is_better": False, "vs_baseline": None, "dtype": "f64 (fp32-pair emulated forward sums)",
+            "higher_is_better": False, "vs_baseline": None, "dtype": "f64 (block fixed-point forward sums)",
             "data": "synthetic", "forward_s": fwd_s, "adjoint_over_forward": adj_s / fwd_s,
             "rk4_steps": nsteps, "s_z_tf": s_f, "s_z_tf_adjoint_pass": s_a[-1], "grad": grad.tolist(),
             "fd_central_h1e-4": fd.tolist(), "rel_err_vs_fd": err.tolist(), "max_rel_err_vs_fd": float(err.max()),
@@ -727,7 +723,7 @@ def run_adjoint_streamed(args):
     line = {"metric": "adjoint at full size: dS_z(t_f)/d(6 mode scales, n_imp scale), t_f = %g ps" % args.adj_tf_ps,
             "value": adj_s, "unit": "s (forward with checkpoints + backward + per-mode contraction, 7 gradients)",
             "n_gpus": 1, "higher_is_better": False, "vs_baseline": None,
-            "dtype": {"f64": "f64", "f64x": "f64 (fp32-pair emulated forward sums)"}[args.adj_precision] +
+            "dtype": {"f64": "f64", "f64x": "f64 (block fixed-point forward sums, fp32-pair backward)"}[args.adj_precision] +
                      "; backward and dJ/dP in FP64",
             "data": "synthetic", "forward_s": fwd_s, "adjoint_over_forward": adj_s / fwd_s, "rk4_steps": nsteps,
             "setup_s": setup_s, "central_differences_s": fd_s, "gradient_split": getattr(model, "last_timing", None),

@@ -4,8 +4,8 @@
 // Why. This part multiplies FP64 at 1.7 lanes per clock and SM, but adds a 32 x 32 -> 64-bit integer
 // product (mad.wide) at 61 (both measured). The contraction needs 16 nb^4 flops per pair: 2.35 ms on the FP64
 // pipe for 9.7M nb = 2 pairs, 0.75 ms of HBM time. In two-digit fixed point a multiply-add is three
-// mad.wide, a third of the HBM time. Measured, 2.5M nb = 2 pairs (1.27 GB): 235 us per launch, 5.4 TB/s (the FP64
-// pipe: 800 us); 177k nb = 4 pairs (1.45 GB): 320 us, 4.5 TB/s; 70k nb = 2 pairs in L2: 29 us (73). What bounds it
+// mad.wide, a third of the HBM time. Measured per RK4 step, 2.5M nb = 2 pairs (1.27 GB a launch): 878 us (the
+// FP64 pipe: 3.3 ms); 409k nb = 4 pairs (3.35 GB): 2.26 ms, 6.0 TB/s; 70k nb = 2 pairs in L2: 83 us (330). What bounds it
 // is the issue rate (50 %): per row block and matrix 192 mad.wide of some 750 instructions, the rest mainly
 // the cross-lane sums of the forward partials.
 //
