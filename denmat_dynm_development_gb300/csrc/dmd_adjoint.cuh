@@ -341,10 +341,12 @@ __device__ __forceinline__ float4 df_bre(const float4& x) { return make_float4(x
 __device__ __forceinline__ float4 df_bim(const float4& x) { return make_float4(x.y, x.y, x.w, x.w); }
 __device__ __forceinline__ float4 df_bimn(const float4& x) { return make_float4(-x.y, -x.y, -x.w, -x.w); }
 
-// pair operators [pair][P1 | P2][nb^4] (complex128) -> double-float copy, one thread per element
-__global__ void k_p_to_df(size_t n, const double2* __restrict__ P, float4* __restrict__ out) {
+// pair operators (complex128) -> double-floats, one thread per element; out may be P's memory
+__global__ void k_p_to_df(size_t n, const double2* P, float4* out) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) out[i] = dfc_split(P[i].x, P[i].y);
+  if (i >= n) return;
+  const double2 p = P[i];
+  out[i] = dfc_split(p.x, p.y);
 }
 
 // double-float complex (re_h, im_h, re_l, im_l) -> complex128 in place (its conjugate when conj)

@@ -125,7 +125,7 @@ struct dmd_handle {
   double* d_tref = nullptr;    // [t0, h, h/2, h/6]
   long long* d_step = nullptr;
   double* d_red = nullptr;     // reduction partials
-  int* d_flag = nullptr;
+  int* d_flag = nullptr;       // [2]
   double2* d_obs[8] = {nullptr};
   double* d_f[8] = {nullptr};
   double obs_prefac[8] = {0};
@@ -193,6 +193,8 @@ size_t red_elems(const dmd_handle* h) {
 
 // bytes of one stored Q element per arithmetic
 int elem_bytes(int prec) { return (prec == DMD_PREC_F32 || prec == DMD_PREC_BF16X2) ? 8 : 16; }
+// arithmetic of the elements that the fill stores: the f64x form's are the f64 form's (choose_form)
+int stored_format(int prec) { return prec == DMD_PREC_F64X ? DMD_PREC_F64 : prec; }
 // the reduced-precision forms contract rho - diag(f_ref) only
 bool deviation_form(int prec) { return prec == DMD_PREC_F32 || prec == DMD_PREC_BF16X2; }
 
@@ -842,20 +844,21 @@ __global__ void k_cb_fill(long long p0, long long cnt, FillSrc src, double add_s
 // so weakly coupled beside its column block's others that the shared exponents would leave it less than
 // FP64's precision (k_fx_spread). The e-e model rewrites the operators before every evaluation and keeps the
 // FP64-pipe contraction.
-int fx_convert(dmd_handle* h) {
+int fx_convert(dmd_handle* h, int* emax) {
   h->use_fx = 0;
   if (h->fmt != DMD_PREC_F64 || h->eek) return DMD_OK;
   const unsigned g = blocks_for(h->nrb, 4), gk = blocks_for(h->nk, 256);
   double* sc = (double*)h->d_acc;  // scratch: [nk][2], rewritten by every evaluation
-  int bad = 0;
-  CK(cudaMemsetAsync(h->d_flag, 0, sizeof(int), h->st));
+  int seen[2], &bad = seen[0];  // no fixed-point form; exponent of the largest element, plus 1100
+  CK(cudaMemsetAsync(h->d_flag, 0, sizeof(seen), h->st));
   CK(cudaMemsetAsync(sc, 0, (size_t)h->nk * 16, h->st));
   if (h->nb == 2) k_fx_spread<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
   else k_fx_spread<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
   k_fx_spread_check<<<gk, 256, 0, h->st>>>(h->nk, sc, h->d_flag);
   CKL();
-  CK(cudaMemcpyAsync(&bad, h->d_flag, sizeof(bad), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaMemcpyAsync(seen, h->d_flag, sizeof(seen), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
+  *emax = seen[1] - 1100;
   if (bad) return DMD_OK;
   int rc;
   if (!h->d_ex && (rc = dalloc(h, &h->d_ex, (size_t)h->nrb * 4 * h->nb2))) return rc;
@@ -874,15 +877,32 @@ int fx_convert(dmd_handle* h) {
 // where nb = 2 takes one or two row blocks only while the flushes' atomics (512 per item) stay few. us per RK4 step, against
 // items filled by pairs: fixed point, 2661 row blocks (500 k-points) 83, 122; 12264 175, 234; 18305 225, 311; 33743 392, 399;
 // 87184 880, 929; nb = 4: 2328 157, 221; 7456 437, 528. FP32, 2661 row blocks 92, 140; 16378 146, 219; 33771 223, 291;
-// 87184 517, 604; nb = 4: 2328 105, 123; 7456 207, 233. The FP64-pipe forms and the batches keep their items.
+// 87184 517, 604; nb = 4: 2328 105, 123; 7456 207, 233. Operators without a fixed-point form take the same items, us per launch
+// against items filled by pairs: FP64 pipe, 2661 row blocks 43, 76; 16378 147, 272; 87184 701, 800; nb = 4, 7456 328, 325;
+// double-floats 27, 45; 64, 108; 225, 277; 112, 123. The e-e model's handles and the batches keep items filled by pairs.
 int item_rows(const dmd_handle* h, const dmd::PairLayout& L, int nsm) {
-  const bool fx = h->fmt == DMD_PREC_F64 && !h->eek, f32 = deviation_form(h->prec) && h->nrhs == 1;
+  const bool fx = stored_format(h->prec) == DMD_PREC_F64 && !h->eek, f32 = deviation_form(h->prec) && h->nrhs == 1;
   if (!fx && !f32) return 0;
   const long long wave = (fx ? 8LL : h->nb == 2 ? 16LL : 20LL) * nsm, hi = h->nb == 2 ? 16 : 4;
   for (int r = 1; r <= hi; ++r)
     if (dmd::count_items(L, r) <= (f32 && h->nb == 2 && r < 3 ? wave * 2 / 5 : wave)) return r;
   const long long third = ((long long)L.rb.size() + 3 * wave - 1) / (3 * wave);
   return (int)std::min(hi, std::max(hi / 2, third));
+}
+
+// The form of the elements that the fill has stored: fixed point where they have that form; else the f64x form's
+// become double-floats, as far as FP32's exponents go, and the f64 form's stay on the FP64 pipe (us per launch: see
+// item_rows)
+int choose_form(dmd_handle* h) {
+  int emax = 0;
+  const int rc = fx_convert(h, &emax);
+  if (rc || h->use_fx || h->eek || h->prec != DMD_PREC_F64X || emax < -60 || emax > 100) return rc;
+  const size_t n = (size_t)h->npair * 2 * h->nb4;
+  k_p_to_df<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, h->d_P, (float4*)h->d_P);
+  CKL();
+  CK(cudaStreamSynchronize(h->st));
+  h->fmt = DMD_PREC_F64X;
+  return DMD_OK;
 }
 
 struct CbDst;
@@ -980,7 +1000,7 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   ArraySource arrays(d, nb4);
   if (!srcp) srcp = &arrays;
   if ((rc = fill_pairs_cb(h, *srcp, dst, dev))) return rc;
-  return fx_convert(h);
+  return choose_form(h);
 }
 
 // Streams the raw operators through two pinned chunks and the fill kernel: the host reads chunk
@@ -1836,8 +1856,9 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
   h->eek = (d->flags & DMD_FLAG_EE) ? 1 : 0;
   // the f64x form's operators are the f64 form's: the fixed-point contraction is the faster and the more exact
   // one (2.5M nb = 2 pairs 224 against 279 us per launch, 9.9M 730 against 792, 70k 29 against 45; 177k nb = 4
-  // pairs 310 against 351). Double-floats remain where the e-e model rewrites the operators before every evaluation
-  h->fmt = (h->prec == DMD_PREC_F64X && !h->eek) ? DMD_PREC_F64 : h->prec;
+  // pairs 310 against 351). Double-floats remain for operators without that form (choose_form) and where the e-e model
+  // rewrites the operators before every evaluation
+  h->fmt = h->eek ? h->prec : stored_format(h->prec);
   h->use_sp = (d->flags & DMD_FLAG_SPARSE) ? 1 : 0;
   h->nrhs = nrhs;
   h->nstate1 = (size_t)h->nk * h->nbdm * h->nbdm;
@@ -1868,7 +1889,7 @@ static int create_impl(const dmd_desc* d, dmd_handle** out, PairSource* src) {
       (rc = dalloc(h, &h->d_y0, h->nstate)) || (rc = dalloc(h, &h->d_in, h->nstate)) ||
       (rc = dalloc(h, &h->d_in1, h->nstate)) || (rc = dalloc(h, &h->d_out, h->nstate)) ||
       (rc = dalloc(h, &h->d_K, 6 * h->nstate)) || (rc = dalloc(h, &h->d_tref, 4)) ||
-      (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_flag, 1)) || (rc = dalloc(h, &h->d_err, 1)) ||
+      (rc = dalloc(h, &h->d_step, 1)) || (rc = dalloc(h, &h->d_red, red_elems(h))) || (rc = dalloc(h, &h->d_flag, 2)) || (rc = dalloc(h, &h->d_err, 1)) ||
       (rc = dalloc(h, &h->d_hflag, 4)) || (rc = dalloc(h, &h->d_ph, nk * h->nb2)))
     return bail(rc);
   std::vector<double> ew(nk * h->nb);
@@ -3106,6 +3127,7 @@ int dmd_add_operators(dmd_handle* h, const double* P1_add, const double* P2_add,
   // the stored form again from the updated operators (and, in the deviation forms, the constant term)
   const bool dev = deviation_form(h->prec);
   if (dev) CK(cudaMemsetAsync(h->d_acc0, 0, (size_t)h->nk * 2 * h->nb2 * sizeof(double2), h->st));
+  if (!h->eek) h->fmt = stored_format(h->prec);  // chosen anew
   const FillSrc fs = {h->d_Praw, nb4, 2 * nb4, nullptr, 0, 0};
   const unsigned g = blocks_for(h->npair, 128);
   if (h->nb == 2)
@@ -3118,7 +3140,7 @@ int dmd_add_operators(dmd_handle* h, const double* P1_add, const double* P2_add,
   CKL();
   CK(cudaStreamSynchronize(h->st));
   const int fx = h->use_fx;
-  if ((rc = fx_convert(h))) return rc;
+  if ((rc = choose_form(h))) return rc;
   if (h->use_fx != fx) drop_graphs(h);
   return DMD_OK;
 }

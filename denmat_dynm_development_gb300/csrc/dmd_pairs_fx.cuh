@@ -109,7 +109,7 @@ __host__ __device__ constexpr int fx_group(int i) {
 // What the shared exponents cost each k-point, one warp per row block: sc[k][0] adds the largest element of every
 // row block that holds a pair of k, sc[k][1] the largest of that pair itself (k by energy rank). An element is off by
 // at most 2^-62 of its block's largest, FP64 by 2^-53 of itself: with sc[0] <= 2^8 sc[1] the sums of k keep
-// FP64's error. Raises *bad at a non-finite element.
+// FP64's error. Raises *bad at a non-finite element and bad[1] to 1100 + the largest element's exponent.
 template <int NB>
 __global__ void __launch_bounds__(128) k_fx_spread(long long nrb, const RowBlock* __restrict__ rbs, const int* __restrict__ rbJ,
                                                    const double2* __restrict__ P, double* __restrict__ sc,
@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(128) k_fx_spread(long long nrb, const RowBlock
     sum += __shfl_xor_sync(0xffffffffu, sum, o);
   }
   if (lane == 0) {
+    atomicMax(bad + 1, fx_expo(all) + 1100);
     atomicAdd(&sc[2 * (size_t)b.row], all);
     atomicAdd(&sc[2 * (size_t)b.row + 1], sum);
   }
