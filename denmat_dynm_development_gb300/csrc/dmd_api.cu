@@ -53,6 +53,9 @@ struct dmd_handle {
   int use_fx = 0;              // f64 form: operators in block-scaled fixed point (dmd_pairs_fx.cuh)
   int* d_rbJ = nullptr;        // column block of every row block (f64 form)
   int16_t* d_ex = nullptr;     // exponents of the fixed-point operators [row block][line][group]
+  dmd::RowBlock* d_rbz = nullptr;  // d_rb without the reverse terms of zero pairs
+  dmd::FxWeak* d_weak = nullptr;   // sums that the contraction leaves to FP64: room for every one
+  unsigned nweak = 0;
   int* d_pos = nullptr;        // k -> energy rank
   int* d_inv = nullptr;        // energy rank -> k
   dmd::RowBlock* d_rb = nullptr;
@@ -60,7 +63,7 @@ struct dmd_handle {
   int nitems = 0;
   long long nrb = 0;
   unsigned int* d_err = nullptr;  // device error flags (bounded waits)
-  unsigned int* d_hflag = nullptr;  // [4] one per RK4 stage (0 otherwise): set by the prep when a state is not exactly Hermitian
+  unsigned int* d_hflag = nullptr;  // [4] one per RK4 stage (0 otherwise): DMD_HFLAG_* of the evaluation
   double2* d_acc0 = nullptr;   // deviation form: contraction of diag(f_ref), position order [nk][2][nb2]
   double* d_fref = nullptr;    // deviation form: window occupations [nk][nb]
   double2* d_ph = nullptr;     // phases D_k(i, j) of the current evaluation [nk][nb2]
@@ -343,8 +346,9 @@ template <int NB>
 void fx_pair_launches(dmd_handle* h, size_t half) {
   const unsigned g = blocks_for(2LL * h->nitems, 4);
   auto pass = [&](auto k) {
-    k<<<g, 128, FxSmem<NB>::cta_bytes, h->st>>>(h->d_items, h->nitems, h->d_rb, (const int4*)h->d_P, h->d_ex, (const double*)h->d_rs,
-                                                half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval, h->d_err);
+    k<<<g, 128, FxSmem<NB>::cta_bytes, h->st>>>(h->d_items, h->nitems, h->d_rb, h->d_rbz, (const int4*)h->d_P, h->d_ex,
+                                                (const double*)h->d_rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval,
+                                                h->d_weak, h->nweak, h->d_err);
   };
   pass(k_pairs_fx<NB, kFxCtas, false>);
   pass(k_pairs_fx<NB, kFxCtas, true>);
@@ -861,9 +865,14 @@ int fx_convert(dmd_handle* h, int* emax) {
   *emax = seen[1] - 1100;
   if (bad) return DMD_OK;
   int rc;
-  if (!h->d_ex && (rc = dalloc(h, &h->d_ex, (size_t)h->nrb * 4 * h->nb2))) return rc;
-  if (h->nb == 2) k_fx_quantise<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex);
-  else k_fx_quantise<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex);
+  const long long nweak = h->nrb * (h->nb == 2 ? 4 : 6);  // two matrices: flushes of every row block, columns of every item
+  if (nweak >= 1LL << 30) return DMD_OK;  // (the flag counts them in 30 bits)
+  if (!h->d_ex && ((rc = dalloc(h, &h->d_ex, (size_t)h->nrb * 4 * h->nb2)) || (rc = dalloc(h, &h->d_rbz, (size_t)h->nrb)) ||
+                   (rc = dalloc(h, &h->d_weak, (size_t)nweak))))
+    return rc;
+  h->nweak = (unsigned)nweak;
+  if (h->nb == 2) k_fx_quantise<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex, h->d_rbz);
+  else k_fx_quantise<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex, h->d_rbz);
   CKL();
   CK(cudaStreamSynchronize(h->st));
   h->use_fx = 1;
@@ -1502,7 +1511,7 @@ void release(dmd_handle* h) {
                   h->d_y0, h->d_in, h->d_in1, h->d_out, h->d_K, h->d_tref, h->d_step, h->d_red, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
                   h->d_dst, h->d_ee_kvec, h->d_ee_kidx, h->d_ee_kmap, h->d_ee_U, h->d_ee_ewf, h->d_ee_f,
                   h->d_ee_dm, h->d_ee_dm1, h->d_ee_dmf, h->d_ee_dm1f, h->d_ee_scr, h->d_ee_Pee, h->d_ee_vqtab,
-                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ};
+                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ, h->d_rbz, h->d_weak};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->adj_stage) cudaFreeHost(h->adj_stage);
@@ -1783,6 +1792,7 @@ int check_state(dmd_handle* h) {
   CK(cudaStreamSynchronize(h->st));
   if (derr) {
     cudaMemsetAsync(h->d_err, 0, sizeof(derr), h->st);
+    if (!(derr & DMD_DEVERR_TIMEOUT)) return fail(h, DMD_E_CUDA, "the list of weak sums is full");
     return fail(h, DMD_E_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
   }
   const size_t n = 2 * h->nstate;

@@ -40,9 +40,11 @@
 namespace dmd {
 
 // flag raised by the prep kernels: bit 0, some rho_k is not exactly Hermitian; bit 1 (FP64 coordinates
-// only), some coordinate is not finite, which the fixed-point contraction cannot scale (dmd_pairs_fx.cuh)
+// only), some coordinate is not finite, which the fixed-point contraction cannot scale (dmd_pairs_fx.cuh). The bits from 2
+// on count the sums that that contraction has listed for FP64.
 #define DMD_HFLAG_NONHERM 1u
 #define DMD_HFLAG_NONFINITE 2u
+#define DMD_HFLAG_WEAK 4u
 
 // ---------------------------------------------------------------------------------------------
 // double-float helpers (no contraction: every operation is an explicit round-to-nearest op)

@@ -27,6 +27,13 @@
 // block and value (the FP64 kernel issues one per pair and value). Reverse sums keep A1's remainder and are exact
 // to the end of the item.
 //
+// Weak sums. All this is relative to the largest product that an item's exponents allow, which need not be near the ones
+// that a sum has: a cold state's occupations range over tens of bits within 32 columns, and detailed balance pairs the large ones with
+// small elements. So a sum is checked when it is known: a row block's forward sums against the unit of their exponents
+// (error 2^-55 of it, root mean square), a column's reverse sums against theirs (2^-56.5; nb = 4 2^-54.5), over the lines and elements of the
+// matrix. Below 2^-6 (2^-8) of it they are not added but listed, and the gated launch sums them in FP64: what is added is
+// good to some 2^-49 of each k-point's own largest sum, as FP64 sums of a few hundred terms are. At 300 K next to none is listed
+// (96 k-points: less than one per evaluation).
 // A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, the first
 // launch returns and the gated one (which otherwise carries the anti-Hermitian part of a state that is not Hermitian,
 // bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do in FP64. Operators
@@ -45,6 +52,10 @@ constexpr int kFxPBits = 61;         // operator bits
 constexpr int kFxCBits = 59;         // column coordinate bits
 constexpr int kFxBase = 32;          // digit base 2^32
 constexpr int kFxExZero = -20000;    // exponent of a group without a nonzero element
+constexpr int kFxWeakRow = 6, kFxWeakColumn = 8;  // bits below the unit from which on sums are listed
+
+// a listed sum: row block x's lines of flush z, or item x's columns z (bits), of column block y; w: matrix, 2: columns
+typedef int4 FxWeak;
 
 // bits of the row coordinates: a reverse sum's 128 (nb = 2) or 512 (nb = 4) products stay below 2^63
 // in units of 2^32
@@ -54,6 +65,11 @@ __host__ __device__ constexpr int fx_row_bits(int nb) { return nb == 2 ? 59 : 57
 __device__ __forceinline__ int fx_expo(double x) {
   const int f = ((__double2hiint(x) >> 20) & 0x7ff) - 1022;
   return f < -900 ? -900 : f;
+}
+// whether these are zero in every lane
+__device__ __forceinline__ bool fx_all_zero(double a, double b, double c, double d) {
+  const long long u = __double_as_longlong(a) | __double_as_longlong(b) | __double_as_longlong(c) | __double_as_longlong(d);
+  return !__any_sync(0xffffffffu, (u << 1) != 0);
 }
 // x 2^s rounded to an integer (|x 2^s| < 2^62) and split into signed digits: q = h 2^32 + l. Integer
 // arithmetic: the FP64 pipe's conversions and products would cost as much as the item's sums.
@@ -75,7 +91,7 @@ __device__ __forceinline__ double fx_scale(double x, int e) {
   return __hiloint2double(hi ? hi + (int)((unsigned)e << 20) : 0, __double2loint(x));
 }
 __device__ __forceinline__ double fx_decode(int h, int l, int ex) {
-  return scalbn((double)((long long)h * (1LL << kFxBase) + l), ex - kFxPBits);
+  return fx_scale((double)((long long)h * (1LL << kFxBase) + l), ex - kFxPBits);
 }
 __device__ __forceinline__ void fx_mul(long long& a0, long long& a1, int h, int l, int2 r, long long a1_0) {
   asm("mul.wide.s32 %0, %1, %2;" : "=l"(a0) : "r"(h), "r"(r.x));
@@ -156,10 +172,12 @@ __global__ void k_fx_spread_check(int nk, const double* __restrict__ sc, int* __
   if (own > 0.0 && !(all <= 256.0 * own && own > 1e-240)) *bad = 1;  // (fx_expo stops at 2^-900)
 }
 
-// FP64 elements to fixed point in place, one warp per row block; ex: [row block][line][group]
+// FP64 elements to fixed point in place, one warp per row block; ex: [row block][line][group]; rbz: the row blocks without
+// reverse terms of pairs that are zero throughout (their sums are zero, not weak)
 template <int NB>
 __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlock* __restrict__ rbs,
-                                                     unsigned char* __restrict__ P, int16_t* __restrict__ ex) {
+                                                     unsigned char* __restrict__ P, int16_t* __restrict__ ex,
+                                                     RowBlock* __restrict__ rbz) {
   constexpr int NB2 = NB * NB, NL = 2 * NB2;
   const long long r = blockIdx.x * 4LL + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -167,12 +185,14 @@ __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlo
   const RowBlock b = rbs[r];
   const int n = __popc(b.mask), m = NB2 * n;
   double2* p = (double2*)P + (size_t)b.pair0 * 2 * NB2 * NB2;
+  unsigned nonzero = 0;  // by slot
   for (int L = 0; L < NL; ++L, p += m) {
     double mx[2] = {0.0, 0.0};
     for (int t = lane; t < m; t += 32) {
       const int e = t / n;
       const int g = (e / NB == e % NB) ? 0 : 1;
       const double v = fmax(fabs(p[t].x), fabs(p[t].y));
+      if (v > 0.0) nonzero |= 1u << (t - e * n);
       if (g) mx[1] = fmax(mx[1], v);
       else mx[0] = fmax(mx[0], v);
     }
@@ -192,6 +212,10 @@ __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlo
       reinterpret_cast<int4*>(p)[t] = make_int4(x.x, x.y, y.x, y.y);
     }
   }
+  nonzero = __reduce_or_sync(0xffffffffu, nonzero);
+  const int slot = __popc(b.mask & ((1u << lane) - 1u));
+  const unsigned keep = __ballot_sync(0xffffffffu, (b.mask >> lane) & (nonzero >> slot) & 1u);
+  if (lane == 0) rbz[r] = {b.row, b.mask, b.revmask & keep, b.pair0};
 }
 
 // bytes between the (line, re | im) rows of a chunk's forward sums: 32 lanes of 16 bytes and 64 more, so that the
@@ -210,7 +234,9 @@ struct FxSmem {
   static constexpr int dig = 2 * stage_bytes;
   static constexpr int zero = dig + (kItemDigits ? kMaxRowBlocksPerItem : 1) * row_bytes;
   static constexpr int exps = zero + row_bytes;
-  static constexpr int fwd = exps + (kItemDigits ? kMaxRowBlocksPerItem * NB2 * 4 : 0);  // forward sums of a chunk
+  static constexpr int NF = NB == 2 ? 1 : 2;  // flushes of forward sums per row block
+  static constexpr int top = exps + (kItemDigits ? kMaxRowBlocksPerItem * NB2 * 4 : 0);  // their largest units: int per flush
+  static constexpr int fwd = top + kMaxRowBlocksPerItem * NF * 4;                        // forward sums of a chunk
   static constexpr int bars = fwd + 4 * kFxFwdStride;
   static constexpr int warp_bytes = (bars + 16 + 127) / 128 * 128;
   static constexpr size_t cta_bytes = 4 * (size_t)warp_bytes;
@@ -268,6 +294,69 @@ __device__ __noinline__ void fx_item_f64(const WorkItem w, const RowBlock* rbs, 
   }
 }
 
+// The same for listed sums of one part (x i: imag), in pieces that a warp has in flight at once: line L of row block rb, and
+// row block rb's share of the reverse sums of the columns in `cols`
+template <int NB>
+__device__ __noinline__ void fx_row_f64(const int rb, const int J, const int L, const RowBlock* rbs, const int4* P, const int16_t* ex,
+                                        const double* rs, bool imag, double* acc, int nk, int lane) {
+  constexpr int NB2 = NB * NB, NB4 = NB2 * NB2, W = 128 / NB2, NL = 2 * NB2;
+  const int qg = lane / W, sl = lane % W, col = J * W + sl;
+  const RowBlock b = rbs[rb];
+  const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << sl) - 1u));
+  double x = 0.0, y = 0.0;
+  if (((b.mask >> sl) & 1u) && col < nk) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = 4 * qg + i;
+      const int4 v = P[(size_t)b.pair0 * 2 * NB4 + ((size_t)L * NB2 + e) * n + slot];
+      const int xe = ex[((size_t)rb * NL + L) * 2 + ((e / NB == e % NB) ? 0 : 1)];
+      const double c = rs[(size_t)col * 2 * NB2 + (L < NB2 ? 0 : NB2) + e];
+      x = fma(fx_decode(v.x, v.y, xe), c, x);
+      y = fma(fx_decode(v.z, v.w, xe), c, y);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x += __shfl_xor_sync(0xffffffffu, x, o);
+    y += __shfl_xor_sync(0xffffffffu, y, o);
+  }
+  if (lane == 0) {
+    double* d = acc + (size_t)b.row * 4 * NB2 + 2 * L;
+    atomicAdd(d, imag ? -y : x);
+    atomicAdd(d + 1, imag ? x : y);
+  }
+}
+template <int NB>
+__device__ __noinline__ void fx_column_f64(const int rb, const int J, const int m, const unsigned cols, const RowBlock* rbs,
+                                           const int4* P, const int16_t* ex, const double* rs, bool imag, double* acc, int nk,
+                                           int lane) {
+  constexpr int NB2 = NB * NB, NB4 = NB2 * NB2, W = 128 / NB2, NL = 2 * NB2;
+  const int qg = lane / W, sl = lane % W, col = J * W + sl;
+  const RowBlock b = rbs[rb];
+  if (!((cols & b.revmask) >> sl & 1u) || col >= nk) return;
+  const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << sl) - 1u));
+  double x[4] = {0.0, 0.0, 0.0, 0.0}, y[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int a = 0; a < NB2; ++a) {
+    const int L = m * NB2 + a;
+    const double kr = rs[(size_t)b.row * 2 * NB2 + (m ? a : NB2 + a)];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = 4 * qg + i;
+      const int4 v = P[(size_t)b.pair0 * 2 * NB4 + ((size_t)L * NB2 + e) * n + slot];
+      const int xe = ex[((size_t)rb * NL + L) * 2 + ((e / NB == e % NB) ? 0 : 1)];
+      x[i] = fma(fx_decode(v.x, v.y, xe), kr, x[i]);
+      y[i] = fma(-fx_decode(v.z, v.w, xe), kr, y[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    double* d = acc + (size_t)col * 4 * NB2 + (m ? 0 : 2 * NB2) + 2 * (4 * qg + i);
+    atomicAdd(d, imag ? -y[i] : x[i]);
+    atomicAdd(d + 1, imag ? x[i] : y[i]);
+  }
+}
+
 // One warp per work item and matrix (Q1 or Q2): lane (qg, sl) owns column W J + sl and the quarter qg of
 // every line. With both matrices in one warp the reverse sums and the column's digits took 168 registers and
 // left 12 warps per SM, too few to cover the multiply-adds' latency; one matrix fits 5 CTAs. Chunks of
@@ -276,9 +365,10 @@ __device__ __noinline__ void fx_item_f64(const WorkItem w, const RowBlock* rbs, 
 // bits of lanes that remain by exchanges that halve the values, so that lane (group, re | im, line) ends with its
 // total. (Exchanges alone, 8 instructions per value and level, took a sixth of the kernel's instructions.)
 template <int NB, bool IMAG>
-__device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkItem w, const int m, const RowBlock* __restrict__ rbs,
-                                        const int4* __restrict__ P, const int16_t* __restrict__ ex,
+__device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkItem* __restrict__ items, const int item, const WorkItem w, const int m,
+                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P, const int16_t* __restrict__ ex,
                                         const double* __restrict__ rs, double* __restrict__ acc, int nk, int lane,
+                                        unsigned int* __restrict__ flag, FxWeak* __restrict__ weak, unsigned nweak,
                                         unsigned int* __restrict__ errflag) {
   typedef FxSmem<NB> S;
   constexpr int NB2 = S::NB2, NB4 = NB2 * NB2, W = S::W;
@@ -331,17 +421,33 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
   int eS0 = -30000, eS1 = -30000;
   const double* const rr = rs + (size_t)mine.row * 2 * NB2 + ro;
   const short2* const xr = (const short2*)ex + ((size_t)(w.rb0 + (lane < nrb ? lane : 0)) * 2 + m) * NB2;
+  int xm[NF][2];  // the largest exponents of lane r's row block's flushes
+#pragma unroll
+  for (int f = 0; f < NF; ++f) xm[f][0] = xm[f][1] = kFxExZero;
+  int em = -900;
   if (lane < nrb) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
 #pragma unroll 4
-    for (int a = 0; a < NB2; ++a) {
-      const int e = fx_expo(rr[a]);
-      const short2 x = xr[a];
-      eS0 = max(eS0, e + x.x);
-      eS1 = max(eS1, e + x.y);
+      for (int a = f * LF; a < (f + 1) * LF; ++a) {
+        const int e = fx_expo(rr[a]);
+        const short2 x = xr[a];
+        eS0 = max(eS0, e + x.x);
+        eS1 = max(eS1, e + x.y);
+        em = max(em, e);
+        xm[f][0] = max(xm[f][0], x.x);
+        xm[f][1] = max(xm[f][1], x.y);
+      }
     }
   }
   eS0 = __reduce_max_sync(FULL, eS0);
   eS1 = __reduce_max_sync(FULL, eS1);
+  bool row_zero = !__any_sync(FULL, em > -900);  // perhaps: every row coordinate is zero
+  if (row_zero) {
+    long long u = 0;
+    for (int a = 0; a < NB2; ++a) u |= lane < nrb ? __double_as_longlong(rr[a]) << 1 : 0;
+    row_zero = !__any_sync(FULL, u != 0);
+  }
   const int lg = lane & 1, lri = (lane >> 1) & 1, ll = (lane >> 2) % LF;
   int2 cd[4];  // the column's digits
   int eR;      // their exponent, of this lane's group
@@ -354,6 +460,13 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
 #pragma unroll
     for (int i = 0; i < 4; ++i) cd[i] = fx_digits(cv[i], kFxCBits - e[fx_group<NB>(i)]);
     eR = (lg ? e[1] : e[0]) + 2 * kFxBase - kFxPBits - kFxCBits;  // of the forward sums' unit
+    // the exponent field (1022 + e of a double below 2^e) that one of a flush's sums has to exceed
+    const bool zero = max(e[0], e[1]) == -900 && fx_all_zero(cv[0], cv[1], cv[2], cv[3]);  // no sum is weak
+    if (lane < nrb) {
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        ((int*)(wbase + S::top))[lane * NF + f] = zero ? -1 : max(xm[f][0] + e[0], xm[f][1] + e[1]) + 1022 - kFxWeakRow;
+    }
   }
   short exn[NF];   // nb = 4: lane (group, re | im, line of a flush): its lines' exponents and row coordinates,
   double rown[NF]; // one row block ahead
@@ -388,6 +501,7 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
 #pragma unroll
   for (int i = 0; i < 4; ++i) B0[i][0] = B0[i][1] = Br[i][0] = Br[i][1] = 0;
   bool any_rev = false;
+  unsigned weak_rows = 0;  // flushes whose sums are too small for their unit (nb = 4: items hold at most 16 row blocks)
   int cfail = -1;
 #pragma unroll 1
   for (int rbi = 0; rbi < nrb; ++rbi) {
@@ -507,8 +621,11 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
       }
       // the totals of the flush's lines to the row's sums (x i in the anti-Hermitian pass)
       double d = fx_scale((double)v, (NF == 1 || f == 0 ? exv[0] : exv[NF - 1]) + eR);
+      // (no branch here: 2 % on 2.5M pairs)
+      const bool add = __any_sync(FULL, ((__double2hiint(d) >> 20) & 0x7ff) > ((const int*)(wbase + S::top))[rbi * NF + f]);
+      if (!add) weak_rows |= 1u << (rbi * NF + f);
       d += __shfl_xor_sync(FULL, d, 1);
-      if (lg == 0 && lane < 4 * LF) {
+      if (add && lg == 0 && lane < 4 * LF) {
         double* dst = acc + (size_t)brow * 4 * NB2 + 2 * (m * NB2 + f * LF + ll);
         if (IMAG) atomicAdd(dst + (lri ^ 1), lri ? -d : d);
         else atomicAdd(dst + lri, d);
@@ -526,10 +643,27 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
     __syncwarp();
     return;
   }
+  // weak sums are left to the gated launch; in that launch they are summed at once
+  auto list = [&](int x, int z, int kind) {
+    if (lane == 0) {
+      const unsigned i = atomicAdd(flag, DMD_HFLAG_WEAK) / DMD_HFLAG_WEAK;
+      if (i < nweak) weak[i] = make_int4(x, w.J, z, m | kind);
+      else atomicOr(errflag, DMD_DEVERR_LIST);
+    }
+  };
+  for (unsigned u = weak_rows; u; u &= u - 1) {
+    const int q = __ffs(u) - 1, rb = w.rb0 + q / NF, f = q % NF;
+    if (IMAG) {
+      for (int l = 0; l < LF; ++l) fx_row_f64<NB>(rb, w.J, m * NB2 + f * LF + l, rbs, P, ex, rs, true, acc, nk, lane);
+    } else {
+      list(rb, f, 0);
+    }
+  }
   // the column block's sums (Y' from Q1, X' from Q2) through the now free first stage, so that a warp's
   // reductions touch consecutive doubles (one lane per column would touch 32 sectors each)
   if (__any_sync(FULL, any_rev)) {
     double2* const out = (double2*)wbase + (size_t)sl * NB2;
+    int got = 0;  // as for the forward sums, over the column's elements
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int b = NB == 2 ? i : 4 * qg + ((i + qg) & 3);
@@ -542,9 +676,26 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
         const bool low = (unsigned)(h ^ (h >> 31)) < (1u << 14);
         const long long q = low ? (long long)((unsigned long long)B0[i][x] << 16 | Br[i][x] >> 16) : B0[i][x] + (Br[i][x] >> 31);
         v[x] = fx_scale((double)q, low ? e - 16 : e);
+        got = max(got, (__double2hiint(v[x]) >> 20) & 0x7ff);
       }
       // conj(p): the imaginary sum has the opposite sign
       out[b] = IMAG ? mk2(v[1], v[0]) : mk2(v[0], -v[1]);
+    }
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1) got = max(got, __shfl_xor_sync(FULL, got, o));
+    const bool small = any_rev && !row_zero && got <= max(eS0, eS1) + 1022 - kFxWeakColumn;
+    const unsigned cols = __ballot_sync(FULL, small);
+    if (cols) {
+      if (small) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out[4 * qg + i] = mk2(0.0, 0.0);
+      }
+      const int z = (int)(W == 32 ? cols : cols & ((1u << (W & 31)) - 1u));
+      if (IMAG) {
+        for (int rb = w.rb0; rb < w.rb1; ++rb) fx_column_f64<NB>(rb, w.J, m, (unsigned)z, rbs, P, ex, rs, true, acc, nk, lane);
+      } else {
+        list(item, z, 2);
+      }
     }
     __syncwarp();
     constexpr int R = 2 * NB2;  // reals per column: consecutive lanes take consecutive reals of one or more columns
@@ -557,29 +708,47 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
   }
 }
 
-// IMAG: the gated launch behind every evaluation's first one, for the anti-Hermitian part (sums times i) and for
+// IMAG: the gated launch behind every evaluation's first one, for the anti-Hermitian part (sums times i), the listed sums and
 // non-finite states. It costs 2.5 us where there is nothing to do; in the same launch, as a second pass of the warp or
-// as blocks that return at once, it cost the pass that always runs 3 to 50 % from 400k pairs on.
+// as blocks that return at once, it cost the pass that always runs 3 to 50 % from 400k pairs on. rbz: the row blocks without the
+// reverse terms of zero pairs; rbs: with them (a non-finite coordinate times zero is NaN).
 template <int NB, int MINB, bool IMAG>
 __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restrict__ items, int nitems,
-                                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P,
-                                                        const int16_t* __restrict__ ex, const double* __restrict__ rs,
-                                                        size_t half, double* __restrict__ acc, int nk,
-                                                        const unsigned int* __restrict__ flag,
+                                                        const RowBlock* __restrict__ rbs, const RowBlock* __restrict__ rbz,
+                                                        const int4* __restrict__ P, const int16_t* __restrict__ ex,
+                                                        const double* __restrict__ rs, size_t half, double* __restrict__ acc,
+                                                        int nk, unsigned int* flag, FxWeak* weak, unsigned nweak,
                                                         unsigned int* __restrict__ errflag) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const unsigned fl = *flag;
   if (IMAG ? fl == 0u : (fl & DMD_HFLAG_NONFINITE) != 0u) return;
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int task = blockIdx.x * 4 + wib, item = task >> 1, m = task & 1;
+  if (IMAG && !(fl & DMD_HFLAG_NONFINITE)) {
+    const unsigned n = min(fl / DMD_HFLAG_WEAK, nweak);
+    constexpr int NB2 = NB * NB, LF = NB == 2 ? 4 : 8, PARTS = NB == 2 ? 16 : 8;  // a warp per line or row block of a listed sum
+    for (unsigned long long i = task; i < (unsigned long long)n * PARTS; i += gridDim.x * 4) {
+      const FxWeak u = weak[i / PARTS];
+      const int part = (int)(i % PARTS), mu = u.w & 1;
+      if (u.w & 2) {
+        const WorkItem w = items[u.x];
+        for (int rb = w.rb0 + part; rb < w.rb1; rb += PARTS)
+          fx_column_f64<NB>(rb, w.J, mu, (unsigned)u.z, rbs, P, ex, rs, false, acc, nk, lane);
+        __syncwarp();
+      } else if (part < LF) {
+        fx_row_f64<NB>(u.x, u.y, mu * NB2 + u.z * LF + part, rbs, P, ex, rs, false, acc, nk, lane);
+      }
+    }
+    if (!(fl & DMD_HFLAG_NONHERM)) return;
+  }
   if (item >= nitems) return;
   const WorkItem w = items[item];
   if (IMAG && (fl & DMD_HFLAG_NONFINITE)) {
     if (m == 0) fx_item_f64<NB>(w, rbs, P, ex, rs, half, (fl & DMD_HFLAG_NONHERM) != 0u, acc, nk, lane);
     return;
   }
-  fx_item<NB, IMAG>(smem_raw + (size_t)wib * FxSmem<NB>::warp_bytes, w, m, rbs, P, ex, rs + (IMAG ? half : 0), acc, nk, lane,
-                    errflag);
+  fx_item<NB, IMAG>(smem_raw + (size_t)wib * FxSmem<NB>::warp_bytes, items, item, w, m, rbz, P, ex, rs + (IMAG ? half : 0), acc, nk, lane,
+                    flag, weak, nweak, errflag);
 }
 
 }  // namespace dmd

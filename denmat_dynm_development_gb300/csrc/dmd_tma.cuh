@@ -9,6 +9,7 @@ namespace dmd {
 
 // error flag bits written by kernels that wait on mbarriers
 #define DMD_DEVERR_TIMEOUT 1u
+#define DMD_DEVERR_LIST 2u
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
