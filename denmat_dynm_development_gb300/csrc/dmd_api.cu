@@ -51,7 +51,6 @@ struct dmd_handle {
   int use_cb = 0;
   int lin = 0;                 // linearized master equation (DMD_FLAG_LINEAR)
   int use_fx = 0;              // f64 form: operators in block-scaled fixed point (dmd_pairs_fx.cuh)
-  int* d_rbJ = nullptr;        // column block of every row block (f64 form)
   int16_t* d_ex = nullptr;     // exponents of the fixed-point operators [row block][line][group]
   dmd::RowBlock* d_rbz = nullptr;  // d_rb without the reverse terms of zero pairs
   dmd::FxWeak* d_weak = nullptr;   // sums that the contraction leaves to FP64: room for every one
@@ -61,6 +60,7 @@ struct dmd_handle {
   dmd::RowBlock* d_rb = nullptr;
   dmd::WorkItem* d_items = nullptr;
   int nitems = 0;
+  dmd::PairLayout lay;         // row blocks, items and runs as the fill takes them (kept for dmd_add_operators)
   long long nrb = 0;
   unsigned int* d_err = nullptr;  // device error flags (bounded waits)
   unsigned int* d_hflag = nullptr;  // [4] one per RK4 stage (0 otherwise): DMD_HFLAG_* of the evaluation
@@ -357,7 +357,8 @@ void fx_pair_launches(dmd_handle* h, size_t half) {
 template <int NB>
 cudaError_t fx_attrs() {
   const int bytes = (int)FxSmem<NB>::cta_bytes;
-  const cudaError_t e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncSetAttribute(k_fx_split<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFxSplitBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   return e != cudaSuccess ? e
                           : cudaFuncSetAttribute(k_pairs_fx<NB, kFxCtas, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
@@ -844,37 +845,75 @@ __global__ void k_cb_fill(long long p0, long long cnt, FillSrc src, double add_s
   }
 }
 
-// The stored FP64 elements to fixed point (dmd_pairs_fx.cuh) where they have that form: finite, and no k-point
-// so weakly coupled beside its column block's others that the shared exponents would leave it less than
-// FP64's precision (k_fx_spread). The e-e model rewrites the operators before every evaluation and keeps the
-// FP64-pipe contraction.
-int fx_convert(dmd_handle* h, int* emax) {
+// The stored FP64 elements to fixed point (dmd_pairs_fx.cuh), with row blocks split where their pairs' strengths
+// lie too far apart for one exponent. Not where an element is not finite or below 2^-900, where the row blocks multiply so far that
+// the form without them is the faster one (a row block takes the same time however few pairs it holds: 2.6 ns on 2.5M
+// pairs, their FP64-pipe contraction 8.0, in double-floats 2.6 to 3.2), or where there is no memory for the split.
+// The e-e model rewrites the operators before every evaluation and keeps the other forms.
+template <int NB>
+int fx_convert(dmd_handle* h, dmd::PairLayout& L, int* emax) {
   h->use_fx = 0;
   if (h->fmt != DMD_PREC_F64 || h->eek) return DMD_OK;
-  const unsigned g = blocks_for(h->nrb, 4), gk = blocks_for(h->nk, 256);
-  double* sc = (double*)h->d_acc;  // scratch: [nk][2], rewritten by every evaluation
-  int seen[2], &bad = seen[0];  // no fixed-point form; exponent of the largest element, plus 1100
+  struct Tmp {
+    uint8_t* cls = nullptr;
+    int* list = nullptr;
+    dmd::RowBlock* rb = nullptr;
+    ~Tmp() {
+      cudaFree(cls);
+      cudaFree(list);
+      cudaFree(rb);
+    }
+  } tmp;
+  auto room = [&](cudaError_t e) {
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e == cudaSuccess;
+  };
+  const unsigned g = blocks_for(h->nrb, 4);
+  int seen[2];  // no fixed-point form; exponent of the largest element, plus 1100
   CK(cudaMemsetAsync(h->d_flag, 0, sizeof(seen), h->st));
-  CK(cudaMemsetAsync(sc, 0, (size_t)h->nk * 16, h->st));
-  if (h->nb == 2) k_fx_spread<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
-  else k_fx_spread<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, h->d_rbJ, (const double2*)h->d_P, sc, h->d_flag);
-  k_fx_spread_check<<<gk, 256, 0, h->st>>>(h->nk, sc, h->d_flag);
+  if (!room(cudaMalloc((void**)&tmp.cls, (size_t)h->npair))) return DMD_OK;
+  k_fx_class<NB><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (const double2*)h->d_P, tmp.cls, h->d_flag);
   CKL();
+  std::vector<uint8_t> cls((size_t)h->npair);
   CK(cudaMemcpyAsync(seen, h->d_flag, sizeof(seen), cudaMemcpyDeviceToHost, h->st));
+  CK(cudaMemcpyAsync(cls.data(), tmp.cls, cls.size(), cudaMemcpyDeviceToHost, h->st));
   CK(cudaStreamSynchronize(h->st));
   *emax = seen[1] - 1100;
-  if (bad) return DMD_OK;
-  int rc;
-  const long long nweak = h->nrb * (h->nb == 2 ? 4 : 6);  // two matrices: flushes of every row block, columns of every item
-  if (nweak >= 1LL << 30) return DMD_OK;  // (the flag counts them in 30 bits)
-  if (!h->d_ex && ((rc = dalloc(h, &h->d_ex, (size_t)h->nrb * 4 * h->nb2)) || (rc = dalloc(h, &h->d_rbz, (size_t)h->nrb)) ||
-                   (rc = dalloc(h, &h->d_weak, (size_t)nweak))))
-    return rc;
-  h->nweak = (unsigned)nweak;
-  if (h->nb == 2) k_fx_quantise<2><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex, h->d_rbz);
-  else k_fx_quantise<4><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (unsigned char*)h->d_P, h->d_ex, h->d_rbz);
+  const long long nrb = dmd::count_split(L, cls);
+  const long long nweak = nrb * (NB == 2 ? 4 : 6);  // two matrices: flushes of every row block, columns of every item
+  if (seen[0] || 4 * nrb > (h->prec == DMD_PREC_F64X ? 5 : 12) * h->nrb || nweak >= 1LL << 30) return DMD_OK;
+  std::vector<int> list;  // row blocks to split
+  if (nrb > h->nrb) {
+    for (size_t r = 0; r < L.rb.size(); ++r) {
+      bool more = false;
+      for (int i = __builtin_popcount(L.rb[r].mask) - 1; i >= 0; --i) more = more || cls[L.rb[r].pair0 + i];
+      if (more) list.push_back((int)r);
+    }
+    if (!room(cudaMalloc((void**)&tmp.list, list.size() * 4))) return DMD_OK;
+    CK(cudaMemcpy(tmp.list, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
+  }
+  void* old[] = {h->d_ex, h->d_rbz, h->d_weak};
+  for (void* p : old) cudaFree(p);
+  h->d_ex = nullptr;
+  h->d_rbz = nullptr;
+  h->d_weak = nullptr;
+  if (!room(cudaMalloc((void**)&tmp.rb, (size_t)nrb * sizeof(dmd::RowBlock))) ||
+      !room(cudaMalloc((void**)&h->d_ex, (size_t)nrb * 4 * NB * NB * sizeof(int16_t))) ||
+      !room(cudaMalloc((void**)&h->d_rbz, (size_t)nrb * sizeof(dmd::RowBlock))) ||
+      !room(cudaMalloc((void**)&h->d_weak, (size_t)nweak * sizeof(dmd::FxWeak))))
+    return DMD_OK;
+  if (!list.empty()) {
+    k_fx_split<NB><<<(unsigned)list.size(), 256, kFxSplitBytes, h->st>>>(tmp.list, h->d_rb, tmp.cls, h->d_P);
+    CKL();
+    dmd::split_row_blocks(L, cls);
+  }
+  CK(cudaMemcpyAsync(tmp.rb, L.rb.data(), (size_t)nrb * sizeof(dmd::RowBlock), cudaMemcpyHostToDevice, h->st));
+  k_fx_quantise<NB><<<blocks_for(nrb, 4), 128, 0, h->st>>>(nrb, tmp.rb, (unsigned char*)h->d_P, h->d_ex, h->d_rbz);
   CKL();
   CK(cudaStreamSynchronize(h->st));
+  std::swap(h->d_rb, tmp.rb);
+  h->nrb = nrb;
+  h->nweak = (unsigned)nweak;
   h->use_fx = 1;
   return DMD_OK;
 }
@@ -889,9 +928,11 @@ int fx_convert(dmd_handle* h, int* emax) {
 // 87184 517, 604; nb = 4: 2328 105, 123; 7456 207, 233. Operators without a fixed-point form take the same items, us per launch
 // against items filled by pairs: FP64 pipe, 2661 row blocks 43, 76; 16378 147, 272; 87184 701, 800; nb = 4, 7456 328, 325;
 // double-floats 27, 45; 64, 108; 225, 277; 112, 123. The e-e model's handles and the batches keep items filled by pairs.
-int item_rows(const dmd_handle* h, const dmd::PairLayout& L, int nsm) {
+int item_rows(const dmd_handle* h, const dmd::PairLayout& L) {
   const bool fx = stored_format(h->prec) == DMD_PREC_F64 && !h->eek, f32 = deviation_form(h->prec) && h->nrhs == 1;
   if (!fx && !f32) return 0;
+  int nsm = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess || nsm <= 0) nsm = 1;
   const long long wave = (fx ? 8LL : h->nb == 2 ? 16LL : 20LL) * nsm, hi = h->nb == 2 ? 16 : 4;
   for (int r = 1; r <= hi; ++r)
     if (dmd::count_items(L, r) <= (f32 && h->nb == 2 && r < 3 ? wave * 2 / 5 : wave)) return r;
@@ -899,18 +940,26 @@ int item_rows(const dmd_handle* h, const dmd::PairLayout& L, int nsm) {
   return (int)std::min(hi, std::max(hi / 2, third));
 }
 
-// The form of the elements that the fill has stored: fixed point where they have that form; else the f64x form's
-// become double-floats, as far as FP32's exponents go, and the f64 form's stay on the FP64 pipe (us per launch: see
-// item_rows)
-int choose_form(dmd_handle* h) {
+// The form of the elements that the fill has stored, and the items of its contraction: fixed point where they have that
+// form; else the f64x form's become double-floats, as far as FP32's exponents go, and the f64 form's stay on the FP64 pipe
+// (us per launch: see item_rows)
+int choose_form(dmd_handle* h, dmd::PairLayout& L) {
   int emax = 0;
-  const int rc = fx_convert(h, &emax);
-  if (rc || h->use_fx || h->eek || h->prec != DMD_PREC_F64X || emax < -60 || emax > 100) return rc;
-  const size_t n = (size_t)h->npair * 2 * h->nb4;
-  k_p_to_df<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, h->d_P, (float4*)h->d_P);
-  CKL();
-  CK(cudaStreamSynchronize(h->st));
-  h->fmt = DMD_PREC_F64X;
+  int rc = h->nb == 2 ? fx_convert<2>(h, L, &emax) : fx_convert<4>(h, L, &emax);
+  if (rc) return rc;
+  if (!h->use_fx && !h->eek && h->prec == DMD_PREC_F64X && emax >= -60 && emax <= 100) {
+    const size_t n = (size_t)h->npair * 2 * h->nb4;
+    k_p_to_df<<<blocks_for((long long)n, 256), 256, 0, h->st>>>(n, h->d_P, (float4*)h->d_P);
+    CKL();
+    CK(cudaStreamSynchronize(h->st));
+    h->fmt = DMD_PREC_F64X;
+  }
+  if (const int rows = item_rows(h, L)) dmd::pack_rows(L, rows);
+  cudaFree(h->d_items);
+  h->d_items = nullptr;
+  if ((rc = dalloc(h, &h->d_items, L.items.size()))) return rc;
+  CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
+  h->nitems = (int)L.items.size();
   return DMD_OK;
 }
 
@@ -933,8 +982,6 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   if (h->npair / ppi < nsm * 16LL) ppi = (int)std::max<long long>(1, h->npair / (nsm * 16LL));
   if (!dmd::build_pair_layout(h->nk, nb, ew.data(), h->npair, d->k1st, d->k2nd, ppi, W, L))
     return fail(h, DMD_E_ARG, "k-pair index out of range");
-  if (const int rows = item_rows(h, L, nsm)) dmd::pack_rows(L, rows);
-  h->nitems = (int)L.items.size();
   h->nrb = (long long)L.rb.size();
   if (nb == 2) {
     cudaError_t (*const attrs[])() = {
@@ -954,20 +1001,11 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
     CK(fx_attrs<4>());
   }
   int rc;
-  if ((rc = dalloc(h, &h->d_pos, (size_t)h->nk)) || (rc = dalloc(h, &h->d_rb, L.rb.size())) ||
-      (rc = dalloc(h, &h->d_items, L.items.size())))
-    return rc;
+  if ((rc = dalloc(h, &h->d_pos, (size_t)h->nk)) || (rc = dalloc(h, &h->d_rb, L.rb.size()))) return rc;
   CK(cudaMemcpy(h->d_pos, L.pos.data(), L.pos.size() * 4, cudaMemcpyHostToDevice));
   if ((rc = dalloc(h, &h->d_inv, (size_t)h->nk))) return rc;
   CK(cudaMemcpy(h->d_inv, L.inv.data(), L.inv.size() * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_rb, L.rb.data(), L.rb.size() * sizeof(dmd::RowBlock), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
-  if (h->fmt == DMD_PREC_F64 && !h->eek) {
-    std::vector<int> J(L.rb.size());
-    for (const dmd::WorkItem& w : L.items) std::fill(J.begin() + w.rb0, J.begin() + w.rb1, w.J);
-    if ((rc = dalloc(h, &h->d_rbJ, J.size()))) return rc;
-    CK(cudaMemcpy(h->d_rbJ, J.data(), J.size() * 4, cudaMemcpyHostToDevice));
-  }
   const int esz = elem_bytes(h->fmt);
   // deviation form: the constant contraction of diag(f_ref), position order [nk][2][nb2]
   const bool dev = deviation_form(h->prec) && !h->lin;
@@ -1009,7 +1047,12 @@ int upload_pairs_cb(dmd_handle* h, const dmd_desc* d) {
   ArraySource arrays(d, nb4);
   if (!srcp) srcp = &arrays;
   if ((rc = fill_pairs_cb(h, *srcp, dst, dev))) return rc;
-  return choose_form(h);
+  if (h->d_dst && !h->eek) {  // for dmd_add_operators, which fills the row blocks as they are now
+    h->lay.rb = L.rb;
+    h->lay.items = L.items;
+    h->lay.runs = L.runs;
+  }
+  return choose_form(h, L);
 }
 
 // Streams the raw operators through two pinned chunks and the fill kernel: the host reads chunk
@@ -1511,7 +1554,7 @@ void release(dmd_handle* h) {
                   h->d_y0, h->d_in, h->d_in1, h->d_out, h->d_K, h->d_tref, h->d_step, h->d_red, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
                   h->d_dst, h->d_ee_kvec, h->d_ee_kidx, h->d_ee_kmap, h->d_ee_U, h->d_ee_ewf, h->d_ee_f,
                   h->d_ee_dm, h->d_ee_dm1, h->d_ee_dmf, h->d_ee_dm1f, h->d_ee_scr, h->d_ee_Pee, h->d_ee_vqtab,
-                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbJ, h->d_rbz, h->d_weak};
+                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbz, h->d_weak};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->adj_stage) cudaFreeHost(h->adj_stage);
@@ -3149,10 +3192,17 @@ int dmd_add_operators(dmd_handle* h, const double* P1_add, const double* P2_add,
   h->launches += 1 + (h->npair + chunk - 1) / chunk;
   CKL();
   CK(cudaStreamSynchronize(h->st));
-  const int fx = h->use_fx;
-  if ((rc = choose_form(h))) return rc;
-  if (h->use_fx != fx) drop_graphs(h);
-  return DMD_OK;
+  if (h->eek) return DMD_OK;
+  drop_graphs(h);  // the form, the row blocks and the items may be others
+  dmd::PairLayout L = h->lay;
+  if (h->nrb != (long long)L.rb.size()) {
+    cudaFree(h->d_rb);
+    h->d_rb = nullptr;
+    if ((rc = dalloc(h, &h->d_rb, L.rb.size()))) return rc;
+    h->nrb = (long long)L.rb.size();
+  }
+  CK(cudaMemcpy(h->d_rb, L.rb.data(), L.rb.size() * sizeof(dmd::RowBlock), cudaMemcpyHostToDevice));
+  return choose_form(h, L);
 }
 
 int dmd_peak_fma(int device, int fp64, double* tflops) {

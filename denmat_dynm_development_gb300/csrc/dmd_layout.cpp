@@ -43,6 +43,7 @@ bool build_pair_layout(int nk, int nb, const double* e_w, long long npair, const
   L.transposed.resize(npair);
   L.rb.clear();
   L.items.clear();
+  L.runs.clear();
   // row blocks; a repeated (row, column) pair starts a new block so that slots stay unique
   long long q = 0;
   while (q < npair) {
@@ -89,33 +90,70 @@ bool build_pair_layout(int nk, int nb, const double* e_w, long long npair, const
     }
     w.rb1 = (int32_t)i;
     L.items.push_back(w);
+    if (!L.runs.empty() && L.runs.back().J == J) L.runs.back().rb1 = w.rb1;
+    else L.runs.push_back(w);
   }
   return true;
 }
 
-// the runs of row blocks of one column block, as f(J, first, end)
-template <typename F>
-static void column_runs(const std::vector<WorkItem>& items, F f) {
-  for (size_t i = 0; i < items.size();) {
-    size_t e = i;
-    while (e < items.size() && items[e].J == items[i].J) ++e;
-    f(items[i].J, items[i].rb0, items[e - 1].rb1);
-    i = e;
-  }
-}
-
 long long count_items(const PairLayout& L, int rows) {
   long long n = 0;
-  column_runs(L.items, [&](int, int r0, int r1) { n += (r1 - r0 + rows - 1) / rows; });
+  for (const WorkItem& w : L.runs) n += (w.rb1 - w.rb0 + rows - 1) / rows;
   return n;
 }
 
 void pack_rows(PairLayout& L, int rows) {
-  std::vector<WorkItem> items;
-  column_runs(L.items, [&](int J, int r0, int r1) {
-    for (int r = r0; r < r1; r += rows) items.push_back({J, r, std::min(r + rows, r1)});
-  });
-  L.items.swap(items);
+  L.items.clear();
+  for (const WorkItem& w : L.runs)
+    for (int r = w.rb0; r < w.rb1; r += rows) L.items.push_back({w.J, r, std::min(r + rows, w.rb1)});
+}
+
+static int classes(const RowBlock& b, const std::vector<uint8_t>& cls) {
+  int m = 0;
+  for (int i = __builtin_popcount(b.mask) - 1; i >= 0; --i) m = std::max(m, cls[b.pair0 + i] + 1);
+  return m;
+}
+
+long long count_split(const PairLayout& L, const std::vector<uint8_t>& cls) {
+  long long n = 0;
+  for (const RowBlock& b : L.rb) n += classes(b, cls);
+  return n;
+}
+
+void split_row_blocks(PairLayout& L, const std::vector<uint8_t>& cls) {
+  std::vector<std::vector<RowBlock>> rb(1);  // by class
+  std::vector<std::vector<WorkItem>> runs(1);
+  for (const WorkItem& w : L.runs)
+    for (int r = w.rb0; r < w.rb1; ++r) {
+      const RowBlock b = L.rb[r];
+      uint32_t p = b.pair0;
+      for (int c = 0, nc = classes(b, cls); c < nc; ++c) {
+        RowBlock o = {b.row, 0, 0, p};
+        uint32_t q = b.pair0;
+        for (int s = 0; s < 32; ++s) {
+          if (!((b.mask >> s) & 1u)) continue;
+          if (cls[q++] != c) continue;
+          o.mask |= 1u << s;
+          o.revmask |= b.revmask & (1u << s);
+          ++p;
+        }
+        if ((size_t)c == rb.size()) {
+          rb.emplace_back();
+          runs.emplace_back();
+        }
+        const int32_t n = (int32_t)rb[c].size();
+        if (runs[c].empty() || runs[c].back().J != w.J) runs[c].push_back({w.J, n, n});
+        runs[c].back().rb1 = n + 1;
+        rb[c].push_back(o);
+      }
+    }
+  L.rb.clear();
+  L.runs.clear();
+  for (size_t c = 0; c < rb.size(); ++c) {
+    const int32_t r0 = (int32_t)L.rb.size();
+    L.rb.insert(L.rb.end(), rb[c].begin(), rb[c].end());
+    for (const WorkItem& w : runs[c]) L.runs.push_back({w.J, w.rb0 + r0, w.rb1 + r0});
+  }
 }
 
 }  // namespace dmd

@@ -41,6 +41,7 @@ struct PairLayout {
   std::vector<int32_t> inv;       // energy rank -> k
   std::vector<RowBlock> rb;
   std::vector<WorkItem> items;
+  std::vector<WorkItem> runs;     // the row blocks that one item may take in a row: those of a column block
   std::vector<uint32_t> src;      // permuted pair slot -> source pair index
   std::vector<uint8_t> slot_of;   // permuted pair slot -> slot within its row block
   std::vector<uint8_t> transposed;  // permuted pair slot stored as (k2, k1) with (conj P2, conj P1)
@@ -51,9 +52,15 @@ struct PairLayout {
 bool build_pair_layout(int nk, int nb, const double* e_w, long long npair, const uint64_t* k1, const uint64_t* k2,
                        int pairs_per_item, int width, PairLayout& L);
 
-// Repacks the row blocks into items of `rows` row blocks (<= kMaxRowBlocksPerItem) however few pairs they hold;
+// Repacks the runs into items of `rows` row blocks (<= kMaxRowBlocksPerItem) however few pairs they hold;
 // count_items: how many that makes
 void pack_rows(PairLayout& L, int rows);
 long long count_items(const PairLayout& L, int rows);
+
+// Splits every row block by the classes of its pairs (cls: by permuted pair; a block's are 0, 1, ... without gaps), each
+// class taking consecutive pairs of the block in lane order. Blocks of class 0 keep their order; those of the classes above
+// follow in runs of their own, class by class. count_split: how many row blocks that makes.
+void split_row_blocks(PairLayout& L, const std::vector<uint8_t>& cls);
+long long count_split(const PairLayout& L, const std::vector<uint8_t>& cls);
 
 }  // namespace dmd

@@ -122,54 +122,105 @@ __host__ __device__ constexpr int fx_group(int i) {
   return NB == 2 ? ((i == 1 || i == 2) ? 1 : 0) : (i == 0 ? 0 : 1);
 }
 
-// What the shared exponents cost each k-point, one warp per row block: sc[k][0] adds the largest element of every
-// row block that holds a pair of k, sc[k][1] the largest of that pair itself (k by energy rank). An element is off by
-// at most 2^-62 of its block's largest, FP64 by 2^-53 of itself: with sc[0] <= 2^8 sc[1] the sums of k keep
-// FP64's error. Raises *bad at a non-finite element and bad[1] to 1100 + the largest element's exponent.
+// Which pairs of a row block may share its exponents. An element is off by at most 2^-62 of its group's largest in the
+// block, FP64's product with it by 2^-53 of itself: a pair may stay if its own largest element of every group lies within
+// kFxSpread bits of the block's (2^-51 of its own largest, in a sum of FP64's 2^-53 per term). Pairs further below, or in a
+// part of their lines only (spin-flip elements), go to row blocks of their own: class 1, 2, ... by the same rule among those
+// left. 2^8 would split 2 to 10 % of the row blocks of the measured systems, 2^10 0.1 to 1 %.
+// One warp per row block: nb = 2 a lane per pair, nb = 4 four lanes, 8 lines each. Raises *bad at a non-finite element or
+// a group below 2^-900, where fx_expo stops, and bad[1] to 1100 + the largest element's exponent.
+constexpr int kFxSpread = 10;
 template <int NB>
-__global__ void __launch_bounds__(128) k_fx_spread(long long nrb, const RowBlock* __restrict__ rbs, const int* __restrict__ rbJ,
-                                                   const double2* __restrict__ P, double* __restrict__ sc,
-                                                   int* __restrict__ bad) {
-  constexpr int NE = 2 * NB * NB * NB * NB, W = 128 / (NB * NB);
+__global__ void __launch_bounds__(128) k_fx_class(long long nrb, const RowBlock* __restrict__ rbs, const double2* __restrict__ P,
+                                                  uint8_t* __restrict__ cls, int* __restrict__ bad) {
+  constexpr int NB2 = NB * NB, NE = 2 * NB2 * NB2, S = NB == 2 ? 32 : 8, LPL = 8;
+  constexpr unsigned FULL = 0xffffffffu;
   const long long r = blockIdx.x * 4LL + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, slot = lane % S;
   if (r >= nrb) return;
   const RowBlock b = rbs[r];
-  const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << lane) - 1u));
-  const bool on = (b.mask >> lane) & 1u;  // lane: column J W + lane
-  double mx = 0.0;
-  bool fin = true;
-  if (on) {
-    const double2* p = P + (size_t)b.pair0 * NE + slot;
-#pragma unroll 8
-    for (int e = 0; e < NE; ++e) {
-      const double2 v = p[(size_t)e * n];
-      fin = fin && isfinite(v.x) && isfinite(v.y);
-      mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+  const int n = __popc(b.mask);
+  const double2* p = P + (size_t)b.pair0 * NE + (size_t)(lane / S) * LPL * NB2 * n + slot;
+  int ex[LPL][2], top = -1100;
+  bool ok = true;
+#pragma unroll
+  for (int L = 0; L < LPL; ++L) {
+    double mx[2] = {0.0, 0.0};
+    if (slot < n) {
+#pragma unroll
+      for (int e = 0; e < NB2; ++e) {
+        const double2 v = p[(size_t)(L * NB2 + e) * n];
+        ok = ok && isfinite(v.x) && isfinite(v.y);
+        double& m = mx[e / NB == e % NB ? 0 : 1];
+        m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      ex[L][g] = mx[g] > 0.0 ? fx_expo(mx[g]) : kFxExZero;
+      ok = ok && ex[L][g] != -900;
+      top = max(top, ex[L][g]);
     }
   }
-  if (!fin) *bad = 1;
-  double all = mx, sum = mx;
+  if (!ok) *bad = 1;
+  top = __reduce_max_sync(FULL, top);
+  if (lane == 0) atomicMax(bad + 1, top + 1100);
+  bool open = slot < n;
+  for (int c = 0; __any_sync(FULL, open); ++c) {
+    bool in = open;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    all = fmax(all, __shfl_xor_sync(0xffffffffu, all, o));
-    sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  }
-  if (lane == 0) {
-    atomicMax(bad + 1, fx_expo(all) + 1100);
-    atomicAdd(&sc[2 * (size_t)b.row], all);
-    atomicAdd(&sc[2 * (size_t)b.row + 1], sum);
-  }
-  if (on && ((b.revmask >> lane) & 1u)) {
-    const size_t c = (size_t)rbJ[r] * W + lane;
-    atomicAdd(&sc[2 * c], all);
-    atomicAdd(&sc[2 * c + 1], mx);
+    for (int L = 0; L < LPL; ++L)
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        int m = open ? ex[L][g] : kFxExZero;
+#pragma unroll
+        for (int o = 1; o < S; o <<= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
+        in = in && !(ex[L][g] != kFxExZero && m - ex[L][g] > kFxSpread);
+      }
+    unsigned take = __ballot_sync(FULL, in);
+    if (S == 8) take = take & take >> 8 & take >> 16 & take >> 24 & 0xffu;  // all lines of a pair
+    if (take == 0u) {  // every pair left is weak in some line: the first one alone
+      const unsigned left = __ballot_sync(FULL, open);
+      take = left & -left;
+    }
+    if (open && (take >> slot) & 1u) {
+      open = false;
+      if (lane == slot) cls[b.pair0 + slot] = (uint8_t)c;
+    }
   }
 }
-__global__ void k_fx_spread_check(int nk, const double* __restrict__ sc, int* __restrict__ bad) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const double all = k < nk ? sc[2 * (size_t)k] : 0.0, own = k < nk ? sc[2 * (size_t)k + 1] : 0.0;
-  if (own > 0.0 && !(all <= 256.0 * own && own > 1e-240)) *bad = 1;  // (fx_expo stops at 2^-900)
+
+// Row blocks whose pairs have several classes (list: their indices): the elements to the new blocks' order, in place,
+// one block of threads each; shared memory: the row block's elements (nb = 2: 32 pairs of 512 bytes, nb = 4: 8 of 8 KB)
+constexpr int kFxSplitBytes = 64 << 10;
+template <int NB>
+__global__ void __launch_bounds__(256) k_fx_split(const int* __restrict__ list, const RowBlock* __restrict__ rbs,
+                                                  const uint8_t* __restrict__ cls, double2* __restrict__ P) {
+  constexpr int NE = 2 * NB * NB * NB * NB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int off[32], cnt[32];  // of a slot's class: first pair's element in the row block; pairs
+  double2* const buf = (double2*)smem_raw;
+  const RowBlock b = rbs[list[blockIdx.x]];
+  const int n = __popc(b.mask);
+  double2* const p = P + (size_t)b.pair0 * NE;
+  for (int t = threadIdx.x; t < n * NE; t += blockDim.x) buf[t] = p[t];
+  if (threadIdx.x < n) {
+    const int c = cls[b.pair0 + threadIdx.x];
+    int below = 0, same = 0, before = 0;
+    for (int i = 0; i < n; ++i) {
+      const int ci = cls[b.pair0 + i];
+      below += ci < c;
+      same += ci == c;
+      before += ci == c && i < (int)threadIdx.x;
+    }
+    off[threadIdx.x] = below * NE + before;
+    cnt[threadIdx.x] = same;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < n * NE; t += blockDim.x) {
+    const int s = t % n, e = t / n;
+    p[off[s] + e * cnt[s]] = buf[t];
+  }
 }
 
 // FP64 elements to fixed point in place, one warp per row block; ex: [row block][line][group]; rbz: the row blocks without
