@@ -6,6 +6,7 @@
 #include <cstring>
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2361,11 +2362,16 @@ static int rk4_begin(dmd_handle* h) {
   return DMD_OK;
 }
 
-// after the last one: the coordinates prepared for a step that does not follow leave no flag behind
-static int rk4_end(dmd_handle* h) {
-  if (fused_tc(h) || fused_step(h)) CK(cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st));
-  return DMD_OK;
-}
+// Around a run of chained stages: whatever way it ends, the coordinates prepared for a stage that does not follow leave no
+// flag behind (the next evaluation's prep only adds to it)
+struct ChainedStages {
+  dmd_handle* h;
+  explicit ChainedStages(dmd_handle* h_) : h(h_) {}
+  ChainedStages(const ChainedStages&) = delete;
+  ~ChainedStages() {
+    if (fused_tc(h) || fused_step(h)) cudaMemsetAsync(h->d_hflag, 0, 4 * sizeof(unsigned int), h->st);
+  }
+};
 
 int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
   if (!h || nsteps < 0 || !(dt == dt)) return DMD_E_ARG;
@@ -2377,6 +2383,7 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
   CK(cudaMemcpyAsync(h->d_step, &zero, 8, cudaMemcpyHostToDevice, h->st));
   // pageable sources: wait so the host values stay valid
   CK(cudaStreamSynchronize(h->st));
+  const ChainedStages chained(h);
   int rc0;
   if ((rc0 = rk4_begin(h))) return rc0;
   if (h->prof_on) {  // one step at a time, events around every kernel
@@ -2387,7 +2394,6 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
       prof_harvest(h);
     }
     h->t = h->t + (double)nsteps * dt;
-    if ((rc0 = rk4_end(h))) return rc0;
     return check_state(h);
   }
   if (!h->g_rk4) {
@@ -2408,7 +2414,6 @@ int dmd_rk4(dmd_handle* h, double dt, int64_t nsteps) {
     CK(cudaGraphLaunch(h->g_rk4, h->st));
     h->launches += h->step_launches;
   }
-  if ((rc0 = rk4_end(h))) return rc0;
   h->t = h->t + (double)nsteps * dt;  // = t0 + n*h as the stage times see it
   CK(cudaStreamSynchronize(h->st));
   return check_state(h);
@@ -2573,6 +2578,7 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
   if (sign * (t1 - h->t) < 0.0) return fail(h, DMD_E_ODE, "integration limits and step direction disagree");
   int rc;
   const bool fused = fused_step(h);
+  const ChainedStages chained(h);
   bool ready = false;  // fused form: the coordinates at (h->t, y) are there
   while (sign * (t1 - h->t) > 0.0) {
     // gsl_odeiv2_evolve_apply
@@ -2638,7 +2644,6 @@ int dmd_rkf45_apply(dmd_handle* h, double t1, double* hstep, double hmin, double
     }
   }
   if (nfev) *nfev = r.nfev;
-  if ((rc = rk4_end(h))) return rc;  // no flag of the coordinates prepared for a step that does not follow
   return check_state(h);
 }
 
@@ -2791,6 +2796,7 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
       h->step_launches = h->launches - l0;
       h->launches = l0;
     }
+    const ChainedStages chained(h);
     if ((rc = rk4_begin(h))) return rc;
     for (int64_t s = 0; s < nsteps; ++s) {
       CK(cudaGraphLaunch(h->g_rk4_rec, h->st));
@@ -2803,7 +2809,6 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
         if (s_obs) s_obs[j] = v;
       }
     }
-    if ((rc = rk4_end(h))) return rc;
     CK(cudaMemcpyAsync(h->d_y, ysave, n * 16, cudaMemcpyDeviceToDevice, h->st));
     h->t = tsave;
   }
@@ -2989,7 +2994,9 @@ int dmd_group_rk4(dmd_group* g, double dt, int64_t nsteps) {
     cudaGraphExecDestroy(g->exec);
     g->exec = nullptr;
   }
+  std::vector<std::unique_ptr<ChainedStages>> chained;
   for (dmd_handle* hm : g->m) {
+    chained.emplace_back(new ChainedStages(hm));
     const int rc = rk4_begin(hm);
     if (rc) return rc;
     if (cudaStreamSynchronize(hm->st) != cudaSuccess) return fail(hm, DMD_E_CUDA, "group: first stage");
@@ -3034,8 +3041,7 @@ int dmd_group_rk4(dmd_group* g, double dt, int64_t nsteps) {
     dmd_handle* hm = g->m[i];
     hm->launches += g->step_launches[i] * nsteps;
     hm->t = hm->t + (double)nsteps * dt;
-    int r = rk4_end(hm);
-    if (!r) r = check_state(hm);
+    const int r = check_state(hm);
     if (r && !rc) rc = r;
   }
   return rc;
