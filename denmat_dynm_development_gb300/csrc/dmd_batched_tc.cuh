@@ -392,15 +392,16 @@ __global__ void __launch_bounds__(128, kTcStageCtas) k_stage_tc2(FinishArgs a, T
     double2 yn;
     if (a.stage < 3) {
       yn = mk2(fma(hs, widen(f.x), yb.x), fma(hs, widen(f.y), yb.y));
-    } else {  // y + h/6 (k1 + 2 k2 + 2 k3 + k4): the sum as a double-float
+    } else {  // y + h/6 (k1 + 2 k2 + 2 k3 + k4): the sum to 2^-71 of its largest term, as three floats
       const float2 k1 = K[el], k2 = K[n + el], k3 = K[2 * n + el];
       auto sum = [&](float u, float v, float w, float x, double base) {
-        float s, t, r, s2, s3;
+        float s, t, r, q, low, rest;
         two_sum(u, __fadd_rn(v, v), s, t);
-        two_sum(s, __fadd_rn(w, w), s2, r);
-        t = __fadd_rn(t, r);
-        two_sum(s2, x, s3, r);
-        return fma(hs, widen(s3), fma(hs, widen(__fadd_rn(t, r)), base));
+        two_sum(s, __fadd_rn(w, w), s, r);
+        two_sum(s, x, s, q);
+        two_sum(t, r, low, rest);
+        two_sum(low, q, low, t);
+        return fma(hs, widen(s), fma(hs, widen(low), fma(hs, widen(__fadd_rn(rest, t)), base)));
       };
       yn = mk2(sum(k1.x, k2.x, k3.x, f.x, yb.x), sum(k1.y, k2.y, k3.y, f.y, yb.y));
     }
