@@ -2744,8 +2744,16 @@ int dmd_adjoint_rk4(dmd_handle* h, double t0, const double* y0, double dt, int64
   // double-float handles run the backward pair pass in double-float arithmetic (k_adj_contract_df, k_adj_pairs_bulk4)
   const bool dfb = h->prec == DMD_PREC_F64X;
   if (dfb) {
-    w.slots = (int)std::min<int64_t>(kAdjGradStages, 4 * nsteps);
-    if ((rc = w.get(&w.dfv, h->nb == 2 ? (size_t)w.slots * 4 * nk2 : 8 * nk2))) return rc;
+    // nb = 2 keeps the vectors of up to 32 stages for one pass of the gradient; of fewer where the memory does not hold them
+    w.slots = h->nb == 2 ? (int)std::min<int64_t>(kAdjGradStages, 4 * nsteps) : 1;
+    const char* const room = getenv("DMD_ADJ_ROOM");  // tests: bytes that an allocation may take here
+    for (;; w.slots /= 2) {
+      const size_t m = h->nb == 2 ? (size_t)w.slots * 4 * nk2 : 8 * nk2;
+      rc = room && m * sizeof(float4) > (size_t)atoll(room) ? fail(h, DMD_E_NOMEM, "DMD_ADJ_ROOM") : w.get(&w.dfv, m);
+      if (rc != DMD_E_NOMEM || w.slots <= 1) break;
+      cudaGetLastError();
+    }
+    if (rc) return rc;
     if (!h->d_Padf && (rc = dalloc(h, &h->d_Padf, np))) return rc;
     if (!h->padf_ok && np) {
       k_p_to_df<<<blocks_for((long long)np, 256), 256, 0, h->st>>>(np, h->use_cb ? h->d_Praw : h->d_P, h->d_Padf);
