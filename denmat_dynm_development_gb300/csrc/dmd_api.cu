@@ -54,6 +54,7 @@ struct dmd_handle {
   int use_fx = 0;              // f64 form: operators in block-scaled fixed point (dmd_pairs_fx.cuh)
   int16_t* d_ex = nullptr;     // exponents of the fixed-point operators [row block][line][group]
   dmd::RowBlock* d_rbz = nullptr;  // d_rb without the reverse terms of zero pairs
+  int8_t* d_st = nullptr;          // how weak an item's columns are by their elements (k_fx_static)
   dmd::FxWeak* d_weak = nullptr;   // sums that the contraction leaves to FP64: room for every one
   unsigned nweak = 0;
   int* d_pos = nullptr;        // k -> energy rank
@@ -347,7 +348,7 @@ template <int NB>
 void fx_pair_launches(dmd_handle* h, size_t half) {
   const unsigned g = blocks_for(2LL * h->nitems, 4);
   auto pass = [&](auto k) {
-    k<<<g, 128, FxSmem<NB>::cta_bytes, h->st>>>(h->d_items, h->nitems, h->d_rb, h->d_rbz, (const int4*)h->d_P, h->d_ex,
+    k<<<g, 128, FxSmem<NB>::cta_bytes, h->st>>>(h->d_items, h->nitems, h->d_rb, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->d_st,
                                                 (const double*)h->d_rs, half, (double*)h->d_acc, h->nk, h->d_hflag + h->eval,
                                                 h->d_weak, h->nweak, h->d_err);
   };
@@ -857,9 +858,10 @@ int fx_convert(dmd_handle* h, dmd::PairLayout& L, int* emax) {
   if (h->fmt != DMD_PREC_F64 || h->eek) return DMD_OK;
   struct Tmp {
     uint8_t* cls = nullptr;
-    int* list = nullptr;
+    int *list = nullptr, *J = nullptr;
     dmd::RowBlock* rb = nullptr;
     ~Tmp() {
+      cudaFree(J);
       cudaFree(cls);
       cudaFree(list);
       cudaFree(rb);
@@ -871,9 +873,15 @@ int fx_convert(dmd_handle* h, dmd::PairLayout& L, int* emax) {
   };
   const unsigned g = blocks_for(h->nrb, 4);
   int seen[2];  // no fixed-point form; exponent of the largest element, plus 1100
+  std::vector<int> J(L.rb.size());
+  for (const dmd::WorkItem& w : L.runs) std::fill(J.begin() + w.rb0, J.begin() + w.rb1, w.J);
+  if (!room(cudaMalloc((void**)&tmp.cls, (size_t)h->npair)) || !room(cudaMalloc((void**)&tmp.J, J.size() * 4))) return DMD_OK;
+  CK(cudaMemcpy(tmp.J, J.data(), J.size() * 4, cudaMemcpyHostToDevice));
+  int* kmax = (int*)h->d_acc;  // scratch (rewritten by every evaluation): [nk][2 nb^2 lines][2]
+  CK(cudaMemsetAsync(kmax, 0, (size_t)h->nk * 4 * NB * NB * sizeof(int), h->st));
   CK(cudaMemsetAsync(h->d_flag, 0, sizeof(seen), h->st));
-  if (!room(cudaMalloc((void**)&tmp.cls, (size_t)h->npair))) return DMD_OK;
-  k_fx_class<NB><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, (const double2*)h->d_P, tmp.cls, h->d_flag);
+  for (int pass = 0; pass < 2; ++pass)
+    k_fx_class<NB><<<g, 128, 0, h->st>>>(h->nrb, h->d_rb, tmp.J, (const double2*)h->d_P, pass, kmax, tmp.cls, h->d_flag);
   CKL();
   std::vector<uint8_t> cls((size_t)h->npair);
   CK(cudaMemcpyAsync(seen, h->d_flag, sizeof(seen), cudaMemcpyDeviceToHost, h->st));
@@ -893,14 +901,16 @@ int fx_convert(dmd_handle* h, dmd::PairLayout& L, int* emax) {
     if (!room(cudaMalloc((void**)&tmp.list, list.size() * 4))) return DMD_OK;
     CK(cudaMemcpy(tmp.list, list.data(), list.size() * 4, cudaMemcpyHostToDevice));
   }
-  void* old[] = {h->d_ex, h->d_rbz, h->d_weak};
+  void* old[] = {h->d_ex, h->d_rbz, h->d_st, h->d_weak};
   for (void* p : old) cudaFree(p);
   h->d_ex = nullptr;
   h->d_rbz = nullptr;
+  h->d_st = nullptr;
   h->d_weak = nullptr;
   if (!room(cudaMalloc((void**)&tmp.rb, (size_t)nrb * sizeof(dmd::RowBlock))) ||
       !room(cudaMalloc((void**)&h->d_ex, (size_t)nrb * 4 * NB * NB * sizeof(int16_t))) ||
       !room(cudaMalloc((void**)&h->d_rbz, (size_t)nrb * sizeof(dmd::RowBlock))) ||
+      !room(cudaMalloc((void**)&h->d_st, (size_t)nrb * 2 * (128 / (NB * NB)))) ||  // (no more items than row blocks)
       !room(cudaMalloc((void**)&h->d_weak, (size_t)nweak * sizeof(dmd::FxWeak))))
     return DMD_OK;
   if (!list.empty()) {
@@ -961,6 +971,17 @@ int choose_form(dmd_handle* h, dmd::PairLayout& L) {
   if ((rc = dalloc(h, &h->d_items, L.items.size()))) return rc;
   CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
   h->nitems = (int)L.items.size();
+  if (h->use_fx) {
+    unsigned* has = (unsigned*)h->d_acc;  // scratch: rewritten by every evaluation
+    CK(cudaMemsetAsync(has, 0, (size_t)h->nk * 4, h->st));
+    for (int pass = 0; pass < 2; ++pass) {
+      const unsigned g = blocks_for(h->nitems, 4);
+      if (h->nb == 2) k_fx_static<2><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->nk, pass, has, h->d_st);
+      else k_fx_static<4><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->nk, pass, has, h->d_st);
+    }
+    CKL();
+    CK(cudaStreamSynchronize(h->st));
+  }
   return DMD_OK;
 }
 
@@ -1555,7 +1576,7 @@ void release(dmd_handle* h) {
                   h->d_y0, h->d_in, h->d_in1, h->d_out, h->d_K, h->d_tref, h->d_step, h->d_red, h->d_flag, h->d_hflag, h->d_acc0, h->d_fref, h->d_tcB, h->d_tcA, h->d_tiles, h->d_ph, h->d_inv, h->d_x0y0, h->d_v0, h->d_Praw, h->d_kkraw,
                   h->d_dst, h->d_ee_kvec, h->d_ee_kidx, h->d_ee_kmap, h->d_ee_U, h->d_ee_ewf, h->d_ee_f,
                   h->d_ee_dm, h->d_ee_dm1, h->d_ee_dmf, h->d_ee_dm1f, h->d_ee_scr, h->d_ee_Pee, h->d_ee_vqtab,
-                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbz, h->d_weak};
+                  h->d_sp_base, h->d_sp_len, h->d_sp_val, h->d_sp_gidx, h->d_Padf, h->d_ee_Aq, h->d_ee_Eq2, h->d_rec, h->d_ex, h->d_rbz, h->d_st, h->d_weak};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->adj_stage) cudaFreeHost(h->adj_stage);

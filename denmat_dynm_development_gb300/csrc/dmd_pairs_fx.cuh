@@ -52,7 +52,12 @@ constexpr int kFxPBits = 61;         // operator bits
 constexpr int kFxCBits = 59;         // column coordinate bits
 constexpr int kFxBase = 32;          // digit base 2^32
 constexpr int kFxExZero = -20000;    // exponent of a group without a nonzero element
-constexpr int kFxWeakRow = 6, kFxWeakColumn = 8;  // bits below the unit from which on sums are listed
+// Bits below the unit from which on sums are listed. A column that lies that far below by its elements alone (k_fx_static) is weak here
+// and not elsewhere: it is listed where its sum lies kFxWeakMore bits lower still, or fx_weak_most below the unit, and not at
+// all where only off-diagonal coordinates reach it.
+constexpr int kFxWeakRow = 6, kFxWeakMore = 5;
+__host__ __device__ constexpr int fx_weak_column(int nb) { return nb == 2 ? 8 : 6; }  // (the row digits: fx_row_bits)
+__host__ __device__ constexpr int fx_weak_most(int nb) { return fx_weak_column(nb) + 2; }
 
 // a listed sum: row block x's lines of flush z, or item x's columns z (bits), of column block y; w: matrix, 2: columns
 typedef int4 FxWeak;
@@ -91,7 +96,9 @@ __device__ __forceinline__ double fx_scale(double x, int e) {
   return __hiloint2double(hi ? hi + (int)((unsigned)e << 20) : 0, __double2loint(x));
 }
 __device__ __forceinline__ double fx_decode(int h, int l, int ex) {
-  return fx_scale((double)((long long)h * (1LL << kFxBase) + l), ex - kFxPBits);
+  // (a group's exponent is kFxExZero or above -900: the factor is a normal number, and short code matters where this is
+  // called: as scalbn the listed sums' 50 KB of instructions took longer to fetch than to run)
+  return (double)((long long)h * (1LL << kFxBase) + l) * __hiloint2double(ex < -900 ? 0 : (ex - kFxPBits + 1023) << 20, 0);
 }
 __device__ __forceinline__ void fx_mul(long long& a0, long long& a1, int h, int l, int2 r, long long a1_0) {
   asm("mul.wide.s32 %0, %1, %2;" : "=l"(a0) : "r"(h), "r"(r.x));
@@ -123,15 +130,17 @@ __host__ __device__ constexpr int fx_group(int i) {
 }
 
 // Which pairs of a row block may share its exponents. An element is off by at most 2^-62 of its group's largest in the
-// block, FP64's product with it by 2^-53 of itself: a pair may stay if its own largest element of every group lies within
-// kFxSpread bits of the block's (2^-51 of its own largest, in a sum of FP64's 2^-53 per term). Pairs further below, or in a
-// part of their lines only (spin-flip elements), go to row blocks of their own: class 1, 2, ... by the same rule among those
-// left. 2^8 would split 2 to 10 % of the row blocks of the measured systems, 2^10 0.1 to 1 %.
-// One warp per row block: nb = 2 a lane per pair, nb = 4 four lanes, 8 lines each. Raises *bad at a non-finite element or
-// a group below 2^-900, where fx_expo stops, and bad[1] to 1100 + the largest element's exponent.
-constexpr int kFxSpread = 10;
+// block; a group within kFxSpread = 10 bits of it by 2^-51 of its own largest, in a sum of FP64's 2^-53 per term. A pair
+// goes to a row block of its own (class 1, 2, ... by the same rule among those left) where the largest element of a matrix lies
+// further below the block's, or a group that is no weaker than the others of its row's or column's k-point (spin-flip elements; kmax, within
+// kFxSame bits): a single small element beside larger ones of the same sum may lose its low bits. At 300 K that makes 0.1 to 1 % more
+// row blocks (2^8 would make 2 to 10 %; counting every small group 33 % where 82 % of the elements are zero).
+// One warp per row block: nb = 2 a lane per pair, nb = 4 four lanes, 8 lines each. First (pass 0) kmax[k][line][group] and, in
+// `bad`: [0] a non-finite element or a group below 2^-900, where fx_expo stops, [1] 1100 + the largest element's exponent.
+constexpr int kFxSpread = 10, kFxSame = 4, kFxKmax0 = 30000;
 template <int NB>
-__global__ void __launch_bounds__(128) k_fx_class(long long nrb, const RowBlock* __restrict__ rbs, const double2* __restrict__ P,
+__global__ void __launch_bounds__(128) k_fx_class(long long nrb, const RowBlock* __restrict__ rbs, const int* __restrict__ rbJ,
+                                                  const double2* __restrict__ P, int pass, int* __restrict__ kmax,
                                                   uint8_t* __restrict__ cls, int* __restrict__ bad) {
   constexpr int NB2 = NB * NB, NE = 2 * NB2 * NB2, S = NB == 2 ? 32 : 8, LPL = 8;
   constexpr unsigned FULL = 0xffffffffu;
@@ -162,9 +171,42 @@ __global__ void __launch_bounds__(128) k_fx_class(long long nrb, const RowBlock*
       top = max(top, ex[L][g]);
     }
   }
-  if (!ok) *bad = 1;
-  top = __reduce_max_sync(FULL, top);
-  if (lane == 0) atomicMax(bad + 1, top + 1100);
+  int col = 0;  // the slot's column
+  for (int i = 0, q = -1; i < S; ++i)
+    if ((b.mask >> i) & 1u && ++q == slot) col = rbJ[r] * S + i;
+  constexpr int NG = 4 * NB2;  // groups of a pair
+  int* const krow = kmax + (size_t)b.row * NG + (lane / S) * LPL * 2;
+  int* const kcol = kmax + (size_t)col * NG + (lane / S) * LPL * 2;
+  if (!pass) {
+    if (!ok) *bad = 1;
+    top = __reduce_max_sync(FULL, top);
+    if (lane == 0) atomicMax(bad + 1, top + 1100);
+#pragma unroll
+    for (int i = 0; i < 2 * LPL; ++i) {
+      const int e = ex[i / 2][i % 2];
+      int m = slot < n ? e : kFxExZero;
+#pragma unroll
+      for (int o = 1; o < S; o <<= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
+      if (slot == 0 && m != kFxExZero) atomicMax(&krow[i], m + kFxKmax0);
+      if (slot < n && e != kFxExZero && ((b.revmask >> (col % S)) & 1u)) atomicMax(&kcol[i], e + kFxKmax0);
+    }
+    return;
+  }
+  unsigned same = 0;  // groups as strong as the others of a k-point
+  if (slot < n) {
+#pragma unroll
+    for (int i = 0; i < 2 * LPL; ++i) {
+      const int e = ex[i / 2][i % 2] + kFxKmax0 + kFxSame;
+      if (e >= krow[i] || (((b.revmask >> (col % S)) & 1u) && e >= kcol[i])) same |= 1u << i;
+    }
+  }
+  int most[2] = {kFxExZero, kFxExZero};  // the pair's largest of each matrix (nb = 4: of the lane's)
+#pragma unroll
+  for (int i = 0; i < 2 * LPL; ++i) {
+    int& q = most[NB == 2 ? i / (2 * NB2) : 0];
+    q = max(q, ex[i / 2][i % 2]);
+  }
+  if (NB == 4) most[0] = max(most[0], __shfl_xor_sync(FULL, most[0], 8));
   bool open = slot < n;
   for (int c = 0; __any_sync(FULL, open); ++c) {
     bool in = open;
@@ -175,8 +217,15 @@ __global__ void __launch_bounds__(128) k_fx_class(long long nrb, const RowBlock*
         int m = open ? ex[L][g] : kFxExZero;
 #pragma unroll
         for (int o = 1; o < S; o <<= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
-        in = in && !(ex[L][g] != kFxExZero && m - ex[L][g] > kFxSpread);
+        if (ex[L][g] != kFxExZero) in = in && !(m - ex[L][g] > kFxSpread && ((same >> (2 * L + g)) & 1u));
       }
+#pragma unroll
+    for (int q = 0; q < (NB == 2 ? 2 : 1); ++q) {
+      int m = open ? most[q] : kFxExZero;
+#pragma unroll
+      for (int o = 1; o < S; o <<= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
+      in = in && (most[q] == kFxExZero || m - most[q] <= kFxSpread);
+    }
     unsigned take = __ballot_sync(FULL, in);
     if (S == 8) take = take & take >> 8 & take >> 16 & take >> 24 & 0xffu;  // all lines of a pair
     if (take == 0u) {  // every pair left is weak in some line: the first one alone
@@ -267,6 +316,60 @@ __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlo
   const int slot = __popc(b.mask & ((1u << lane) - 1u));
   const unsigned keep = __ballot_sync(0xffffffffu, (b.mask >> lane) & (nonzero >> slot) & 1u);
   if (lane == 0) rbz[r] = {b.row, b.mask, b.revmask & keep, b.pair0};
+}
+
+// How far a column's elements lie below the item's largest where the coordinates are alike: st[item][matrix][column], in bits,
+// from the lines of the diagonal coordinates (the off-diagonal ones are small). kFxNoLine: no element of those lines here, but
+// elsewhere in the k-point's sum (has[k]: bit 0 Y's, bit 1 X's), or none of any line. One warp per item; first (pass 0) has, then st.
+constexpr int kFxNoLine = 127;
+template <int NB>
+__global__ void __launch_bounds__(128) k_fx_static(const WorkItem* __restrict__ items, int nitems, const RowBlock* __restrict__ rbz,
+                                                   const int4* __restrict__ P, const int16_t* __restrict__ ex, int nk, int pass,
+                                                   unsigned* __restrict__ has, int8_t* __restrict__ st) {
+  constexpr int NB2 = NB * NB, NB4 = NB2 * NB2, W = 128 / NB2, NL = 2 * NB2;
+  const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, qg = lane / W, sl = lane % W;
+  if (item >= nitems) return;
+  const WorkItem w = items[item];
+  const int col = w.J * W + sl;
+  for (int m = 0; m < 2; ++m) {
+    int own = kFxExZero, all = kFxExZero, any = kFxExZero;  // the column's and the item's largest; the column's of every line
+    for (int rb = w.rb0; rb < w.rb1; ++rb) {
+      const RowBlock b = rbz[rb];
+      const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << sl) - 1u));
+      const bool rev = (b.revmask >> sl) & 1u;
+      for (int a = 0; a < NB2; ++a) {
+        const bool diag = a / NB == a % NB;
+        const int16_t* x = ex + ((size_t)rb * NL + m * NB2 + a) * 2;
+        if (diag) all = max(all, max((int)x[0], (int)x[1]));
+        if (!((b.mask >> sl) & 1u)) continue;
+        for (int i = 0; i < 4; ++i) {
+          const int e = 4 * qg + i;
+          const int4 v = P[(size_t)b.pair0 * 2 * NB4 + ((size_t)(m * NB2 + a) * NB2 + e) * n + slot];
+          const long long p = (long long)v.x * (1LL << kFxBase) + v.y, q = (long long)v.z * (1LL << kFxBase) + v.w;
+          const unsigned long long u = (unsigned long long)(p ^ (p >> 63)) | (unsigned long long)(q ^ (q >> 63));
+          if (u == 0ull) continue;
+          if (!pass && e / NB == e % NB) atomicOr(&has[b.row], 2u >> m);
+          if (!rev) continue;
+          const int t = 64 - __clzll((long long)u) + x[e / NB == e % NB ? 0 : 1] - kFxPBits;
+          any = max(any, t);
+          if (diag) own = max(own, t);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1) {
+      own = max(own, __shfl_xor_sync(0xffffffffu, own, o));
+      any = max(any, __shfl_xor_sync(0xffffffffu, any, o));
+    }
+    if (qg || col >= nk) continue;
+    if (!pass) {
+      if (own != kFxExZero) atomicOr(&has[col], 1u << m);
+    } else {
+      const bool none = own == kFxExZero;
+      st[((size_t)item * 2 + m) * W + sl] =
+          (int8_t)(none ? (((has[col] >> m) & 1u) || any == kFxExZero ? kFxNoLine : 0) : min(max(all - own, 0), kFxNoLine - 1));
+    }
+  }
 }
 
 // bytes between the (line, re | im) rows of a chunk's forward sums: 32 lanes of 16 bytes and 64 more, so that the
@@ -416,8 +519,8 @@ __device__ __noinline__ void fx_column_f64(const int rb, const int J, const int 
 // bits of lanes that remain by exchanges that halve the values, so that lane (group, re | im, line) ends with its
 // total. (Exchanges alone, 8 instructions per value and level, took a sixth of the kernel's instructions.)
 template <int NB, bool IMAG>
-__device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkItem* __restrict__ items, const int item, const WorkItem w, const int m,
-                                        const RowBlock* __restrict__ rbs, const int4* __restrict__ P, const int16_t* __restrict__ ex,
+__device__ __forceinline__ void fx_item(unsigned char* const wbase, const int item, const WorkItem w, const int m, const RowBlock* __restrict__ rbs,
+                                        const int4* __restrict__ P, const int16_t* __restrict__ ex, const int8_t* __restrict__ st,
                                         const double* __restrict__ rs, double* __restrict__ acc, int nk, int lane,
                                         unsigned int* __restrict__ flag, FxWeak* __restrict__ weak, unsigned nweak,
                                         unsigned int* __restrict__ errflag) {
@@ -734,8 +837,14 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const WorkIt
     }
 #pragma unroll
     for (int o = W; o < 32; o <<= 1) got = max(got, __shfl_xor_sync(FULL, got, o));
-    const bool small = any_rev && !row_zero && got <= max(eS0, eS1) + 1022 - kFxWeakColumn;
-    const unsigned cols = __ballot_sync(FULL, small);
+    const int below = max(eS0, eS1) + 1022 - got;
+    bool small = any_rev && !row_zero && below >= fx_weak_column(NB);
+    unsigned cols = __ballot_sync(FULL, small);
+    if (cols) {
+      const int s = st[((size_t)item * 2 + m) * W + sl];
+      small = small && s != kFxNoLine && below >= min(max(s + kFxWeakMore, fx_weak_column(NB)), fx_weak_most(NB));
+      cols = __ballot_sync(FULL, small);
+    }
     if (cols) {
       if (small) {
 #pragma unroll
@@ -767,7 +876,8 @@ template <int NB, int MINB, bool IMAG>
 __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restrict__ items, int nitems,
                                                         const RowBlock* __restrict__ rbs, const RowBlock* __restrict__ rbz,
                                                         const int4* __restrict__ P, const int16_t* __restrict__ ex,
-                                                        const double* __restrict__ rs, size_t half, double* __restrict__ acc,
+                                                        const int8_t* __restrict__ st, const double* __restrict__ rs, size_t half,
+                                                        double* __restrict__ acc,
                                                         int nk, unsigned int* flag, FxWeak* weak, unsigned nweak,
                                                         unsigned int* __restrict__ errflag) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -798,7 +908,7 @@ __global__ void __launch_bounds__(128, MINB) k_pairs_fx(const WorkItem* __restri
     if (m == 0) fx_item_f64<NB>(w, rbs, P, ex, rs, half, (fl & DMD_HFLAG_NONHERM) != 0u, acc, nk, lane);
     return;
   }
-  fx_item<NB, IMAG>(smem_raw + (size_t)wib * FxSmem<NB>::warp_bytes, items, item, w, m, rbz, P, ex, rs + (IMAG ? half : 0), acc, nk, lane,
+  fx_item<NB, IMAG>(smem_raw + (size_t)wib * FxSmem<NB>::warp_bytes, item, w, m, rbz, P, ex, st, rs + (IMAG ? half : 0), acc, nk, lane,
                     flag, weak, nweak, errflag);
 }
 
