@@ -30,10 +30,11 @@
 // Weak sums. All this is relative to the largest product that an item's exponents allow, which need not be near the ones
 // that a sum has: a cold state's occupations range over tens of bits within 32 columns, and detailed balance pairs the large ones with
 // small elements. So a sum is checked when it is known: a row block's forward sums against the unit of their exponents
-// (error 2^-55 of it, root mean square), a column's reverse sums against theirs (2^-56.5; nb = 4 2^-54.5), over the lines and elements of the
-// matrix. Below 2^-6 (2^-8) of it they are not added but listed, and the gated launch sums them in FP64: what is added is
-// good to some 2^-49 of each k-point's own largest sum, as FP64 sums of a few hundred terms are. At 300 K next to none is listed
-// (96 k-points: less than one per evaluation).
+// (error 2^-55 of it, root mean square), a column's reverse sums against theirs (2^-56.5; nb = 4 2^-54.5), over the lines and
+// elements of the matrix. Below 2^-7 (2^-8; nb = 4 2^-7) of it they are not added but listed, and the gated launch sums them in
+// FP64: each k-point's own largest sum keeps some 2^-48, as FP64 sums of a few hundred terms do. At 300 K next to none is listed. The check
+// takes 1 to 4 % of the main launch (2.5M pairs 205 -> 212 us, 70k 13.4 -> 13.8, 46k nb = 4 pairs 91.9 -> 93.5); an evaluation with
+// some sums listed 2 to 3 us more, one of uniformly random exponents over 60 bits 300 us in place of 218 (the FP64 pipe: 800).
 // A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, the first
 // launch returns and the gated one (which otherwise carries the anti-Hermitian part of a state that is not Hermitian,
 // bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do in FP64. Operators
@@ -55,9 +56,9 @@ constexpr int kFxExZero = -20000;    // exponent of a group without a nonzero el
 // Bits below the unit from which on sums are listed. A column that lies that far below by its elements alone (k_fx_static) is weak here
 // and not elsewhere: it is listed where its sum lies kFxWeakMore bits lower still, or fx_weak_most below the unit, and not at
 // all where only off-diagonal coordinates reach it.
-constexpr int kFxWeakRow = 6, kFxWeakMore = 5;
-__host__ __device__ constexpr int fx_weak_column(int nb) { return nb == 2 ? 8 : 6; }  // (the row digits: fx_row_bits)
-__host__ __device__ constexpr int fx_weak_most(int nb) { return fx_weak_column(nb) + 2; }
+constexpr int kFxWeakRow = 7, kFxWeakMore = 5;
+__host__ __device__ constexpr int fx_weak_column(int nb) { return nb == 2 ? 8 : 7; }  // (the row digits: fx_row_bits)
+__host__ __device__ constexpr int fx_weak_most(int nb) { return fx_weak_column(nb) + 4; }
 
 // a listed sum: row block x's lines of flush z, or item x's columns z (bits), of column block y; w: matrix, 2: columns
 typedef int4 FxWeak;

@@ -5,7 +5,7 @@ Bound. The scattering term is (prefac / 2) (C + C^+), C = (1 - rho) X - Y rho, X
 S the same sums of absolute values, a k-point's term is off by at most prefac nb (|1 - rho| S_X + |rho| S_Y) eps, largest
 elements taken of each. FP64 sums (the oracle's side: a handle with DMD_FLAG_EE, on the FP64 pipe) have eps of some 2^-51 for n of a few
 hundred; fixed-point ones are listed for FP64 from an error of 2^-49 (root mean square) on, four times that for the worst of some
-thousand sums, and as much again for pairs within 2^10 of each other's strength: 2^-46 for both sides together.
+thousand sums, and as much again for elements within 2^10 of their row block's: 2^-46 for both sides together.
 """
 import numpy as np
 import pytest
@@ -195,3 +195,16 @@ def test_zero_pairs_and_strengths_in_every_row_block(oracle, built):
     v[8 * 40] = np.nan
     with handle(s) as g, handle(s, pipe=True) as p:
         np.testing.assert_array_equal(np.isfinite(g.func(0.0, v)), np.isfinite(p.func(0.0, v)))
+
+
+@pytest.mark.parametrize("fill", [0.44, 0.18, 0.05])
+@pytest.mark.parametrize("nk,nb,density", [(40, 2, 1.0), (300, 2, 0.5), (120, 4, 0.3)])
+def test_mostly_zero_operators(nk, nb, density, fill, oracle, built):
+    """operators with most elements zero, in the dense form: columns without an element on the diagonal coordinates' lines, groups of one
+    element. Off-diagonal coordinates 1e-3 of the diagonal ones, and a state that is not Hermitian."""
+    s = system(oracle, nk, nb, density, 5 * nk + nb)
+    rng = np.random.default_rng(2)
+    s.P1, s.P2 = (np.where(rng.random(np.size(P)) < fill, np.asarray(P), 0.0) for P in (s.P1, s.P2))
+    y = oracle.y_of(s.dm0)
+    assert worst(s, y, 5.0 * oracle.fs) < EPS
+    assert worst(s, y * (1.0 + 1e-2 * rng.standard_normal(y.size)), 5.0 * oracle.fs) < EPS
