@@ -21,10 +21,17 @@ FLAG_LINEAR = 1  # DMD_FLAG_LINEAR: P1, P2 are the linear operators Lscij, Lscji
 FLAG_ADJOINT = 2  # DMD_FLAG_ADJOINT: keep the operators in stored order for adjoint_rk4
 FLAG_EE = 4  # DMD_FLAG_EE: keep P_eph (+ P_eimp) in stored order and the column-block map for the e-e model
 FLAG_SPARSE = 8  # DMD_FLAG_SPARSE: contract only the stored elements (alg_sparseP / alg_Pin_is_sparse)
-# sparse="auto" picks the sparse FP64 contraction below this fraction of stored elements: on an nb = 4
-# MoS2-like workload (727k pairs) it ran 4.7x / 2.5x / 1.45x / 1.02x faster than the dense FP64
-# contraction at 9 / 18 / 31 / 44 % stored (bench --sparse)
-SPARSE_AUTO_FILL = 0.4
+# sparse="auto" picks the sparse contraction below this fraction of stored elements: where it is the faster one of the two
+# (us per RK4 step, dense and sparse). nb = 4, 181k pairs: 1224, 1394 at 44 %; 1225, 1046 at 31 %; 697k: 3867, 4771; 3868, 3462;
+# 46k: 433, 434; 435, 342. nb = 2, 71k pairs: 87, 103 at 31 %; 87, 92 at 24 %; 87, 86 at 18 %; 398k: 233, 254; 235, 219; 234, 181.
+# The dense form of the other band counts runs on the FP64 pipe, as all of them did where 44 % was the limit.
+SPARSE_AUTO_FILL = {2: 0.2, 4: 0.35}
+SPARSE_AUTO_FILL_OTHER = 0.4
+
+
+def sparse_pays(nb, fill):
+    """whether the sparse contraction is the faster one for nb bands with this fraction of the elements stored"""
+    return fill < SPARSE_AUTO_FILL.get(nb, SPARSE_AUTO_FILL_OTHER)
 
 
 def stored_fraction(P1, P2, thr=1e-40):
@@ -160,7 +167,7 @@ class LindbladGPU:
         if sparse == "auto":  # the faster form for the operators' fill (dense P given as arrays)
             sparse = (precision in ("f64", 0) and nrhs <= 1 and not (linear or adjoint or ee or ee_flag) and
                       k["P1"] is not None and k["A1"] is None and
-                      stored_fraction(k["P1"], k["P2"]) < SPARSE_AUTO_FILL)
+                      sparse_pays(bend - bstart, stored_fraction(k["P1"], k["P2"])))
         ptr = lambda a: None if a is None else a.ctypes.data  # noqa: E731
         desc = _Desc(nk=nk, nb_dm=nb_dm, bstart=bstart, bend=bend, nkpair=int(k["k1"].size), prefac_eph=prefac_eph,
                      e_dm=ptr(k["e"]), k1st=ptr(k["k1"]), k2nd=ptr(k["k2"]), P1=ptr(k["P1"]), P2=ptr(k["P2"]),
