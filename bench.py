@@ -9,7 +9,8 @@ from the package generator (the reference publishes no dataset for this path).
 One step = one RK4 step = four RHS evaluations, each streaming all of P once (inputs are larger
 than the 129 MB L2, so no flush is needed between steps).
 
-The headline arithmetic is the reference's: plain FP64 (P complex128, FP64 multiply-adds).
+The headline form is the FP64 one (`METRIC` keeps its first name, "plain FP64"): operators in the 8 bytes of a double per real, as
+61-bit integers with shared exponents, exact products and integer sums, FP64 states and updates (`dtype`).
 
   value       RK4 steps/s with the density matrix resident on the GPU (dmd_rk4, CUDA graph); the
               K-step window is timed `--windows` times (CUDA events) and the median is reported,
@@ -536,7 +537,7 @@ def run_gpu(args, w, rank, world, dist):
 
 
 ELEM_BYTES = {"f64": 16, "f64x": 16, "f32": 8, "bf16x2": 8}
-DTYPE = {"f64": "f64", "f64x": "f64 (block fixed point, as f64)", "f32": "f32 (P complex64, rho as deviation from f)",
+DTYPE = {"f64": "f64 (contraction in 61-bit block fixed point)", "f64x": "f64 (block fixed point, as f64)", "f32": "f32 (P complex64, rho as deviation from f)",
          "bf16x2": "bf16 hi+lo (P 8 B/complex, rho as deviation from f)"}
 
 

@@ -339,7 +339,6 @@ __global__ void k_adj_pairs(long long npair, const int2* __restrict__ kk, const 
 // broadcast of the real / imaginary part of a double-float complex (re_h, im_h, re_l, im_l)
 __device__ __forceinline__ float4 df_bre(const float4& x) { return make_float4(x.x, x.x, x.z, x.z); }
 __device__ __forceinline__ float4 df_bim(const float4& x) { return make_float4(x.y, x.y, x.w, x.w); }
-__device__ __forceinline__ float4 df_bimn(const float4& x) { return make_float4(-x.y, -x.y, -x.w, -x.w); }
 
 // pair operators (complex128) -> double-floats, one thread per element; out may be P's memory
 __global__ void k_p_to_df(size_t n, const double2* P, float4* out) {

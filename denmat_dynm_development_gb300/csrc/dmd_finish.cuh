@@ -4,7 +4,7 @@
 // Why. k_finish gives a k-point one thread, whose chain of some 150 to 400 FP64 operations runs at one result per
 // 19 clocks and SM (the FP64 pipe) however few k-points there are: 9 us for 500 k-points, 17 us with a
 // coherent term, 45 us for nb = 4. Here nb^2 lanes share a k-point and exchange operands by shuffles, blocks are one
-// warp so that small systems spread over the SMs, and H(t)'s phases are the prep's. Element by element the
+// warp (with the next stage's phases two) so that small systems spread over the SMs, and H(t)'s phases are the prep's. Element by element the
 // operations and their order are k_finish's. With the next stage's input in registers the same lanes write its
 // coordinates (k_prep_herm's values), reset the sums they have just read and form the phases of the next time,
 // which saves the prep launch of every stage.

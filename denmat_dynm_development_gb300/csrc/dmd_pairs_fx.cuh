@@ -4,7 +4,7 @@
 // Why. This part multiplies FP64 at 1.7 lanes per clock and SM, but adds a 32 x 32 -> 64-bit integer
 // product (mad.wide) at 61 (both measured). The contraction needs 16 nb^4 flops per pair: 2.35 ms on the FP64
 // pipe for 9.7M nb = 2 pairs, 0.75 ms of HBM time. In two-digit fixed point a multiply-add is three
-// mad.wide, a third of the HBM time. Measured per RK4 step, 2.5M nb = 2 pairs (1.27 GB a launch): 878 us (the
+// mad.wide, a third of the HBM time. Measured per RK4 step, 2.5M nb = 2 pairs (1.27 GB a launch): 920 us (the
 // FP64 pipe: 3.3 ms); 409k nb = 4 pairs (3.35 GB): 2.26 ms, 6.0 TB/s; 70k nb = 2 pairs in L2: 83 us (330). What bounds it
 // is the issue rate (50 %): per row block and matrix 192 mad.wide of some 750 instructions, the rest mainly
 // the cross-lane sums of the forward partials.
@@ -38,7 +38,8 @@
 // A state with a non-finite coordinate has no scale: the prep kernel raises bit 1 of the flag, the first
 // launch returns and the gated one (which otherwise carries the anti-Hermitian part of a state that is not Hermitian,
 // bit 0) contracts in FP64 from the decoded elements, so NaN and infinities spread as they do in FP64. Operators
-// with a non-finite element are never converted (dmd_api.cu).
+// with a non-finite element are never converted (dmd_api.cu). Row blocks are split where their pairs are of too uneven strength
+// for one exponent (k_fx_class).
 #pragma once
 #include <type_traits>
 
@@ -514,7 +515,7 @@ __device__ __noinline__ void fx_column_f64(const int rb, const int J, const int 
 
 // One warp per work item and matrix (Q1 or Q2): lane (qg, sl) owns column W J + sl and the quarter qg of
 // every line. With both matrices in one warp the reverse sums and the column's digits took 168 registers and
-// left 12 warps per SM, too few to cover the multiply-adds' latency; one matrix fits 5 CTAs. Chunks of
+// left 12 warps per SM, too few to cover the multiply-adds' latency; one matrix fits 4 CTAs. Chunks of
 // two lines (4 KB) stream through a per-warp ring of two bulk copies. The forward sums (line, re | im,
 // group) of a chunk are added over the warp through shared memory, 8 lanes' entries by each lane, and the two
 // bits of lanes that remain by exchanges that halve the values, so that lane (group, re | im, line) ends with its

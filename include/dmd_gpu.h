@@ -48,13 +48,16 @@ extern "C" {
 
 /* arithmetic of the k-pair contraction */
 #define DMD_PREC_F64 0     /* FP64: P as 61-bit integers with a binary exponent per group of elements (8 bytes per
-                              real, as complex128), exact products and sums in 64-bit integers: errors at or
-                              below those of FP64 multiply-adds. Operators without that form (a non-finite
-                              element, k-points coupled 2^-8 of their neighbours' strength or less) and handles with
-                              DMD_FLAG_EE keep complex128 and FP64 multiply-adds */
-#define DMD_PREC_F64X 1    /* as DMD_PREC_F64 for the contraction (nb = 2, 4); the adjoint's backward pass and, with
-                              DMD_FLAG_EE, the contraction and the e-e rebuild use (hi, lo) FP32 pairs: ~2^-46
-                              products, double-FP32 sums */
+                              real, as complex128), products of 53 bits or more and sums in 64-bit integers. Normwise
+                              the error is below that of FP64 multiply-adds; each k-point's sums are good to some 2^-48
+                              of their own largest (sums that lie far below their exponents are formed in FP64), while
+                              an element of a k-point's sums that is far smaller than the others need not keep FP64's
+                              relative error. Operators without that form (a non-finite element or one below 2^-900,
+                              strengths so uneven that the row blocks would triple) and handles with DMD_FLAG_EE keep
+                              complex128 and FP64 multiply-adds */
+#define DMD_PREC_F64X 1    /* as DMD_PREC_F64 for the contraction (nb = 2, 4); operators without the fixed-point form, the
+                              adjoint's backward pass and, with DMD_FLAG_EE, the contraction and the e-e rebuild use
+                              (hi, lo) FP32 pairs: ~2^-46 products, double-FP32 sums */
 #define DMD_PREC_F32 2     /* P stored complex64, FP32 products; rho enters as its deviation from f_ref */
 #define DMD_PREC_BF16X2 3  /* P stored as bf16 hi + bf16 lo per component (8 bytes per complex), FP32
                               products; rho enters as its deviation from f_ref */
