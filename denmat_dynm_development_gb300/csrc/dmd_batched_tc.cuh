@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(128, 1) k_pairs_tc(const TcTile* __restrict__ 
 // operations per state and k-point.
 // A warp takes one state's elements of a column group's 8 energy ranks, a lane per element (a thread per k-point needs 128
 // registers: 16 warps per SM and 75 us), and walks states with the k-points' constants and phases in registers; its
-// stores are whole 64-byte halves of an operand row. It takes 45 to 55 us there, the FP64 pipe 71 % busy (the update's own
-// multiply-adds and the exact splits); the RK4 step went from 700 to 487 us (1000 k-points, 16 states: 85 us).
+// stores are whole 64-byte halves of an operand row. It takes 43 to 50 us there, the FP64 pipe 64 % busy (the update's own
+// multiply-adds and the exact splits); the RK4 step went from 700 to 484 us (1000 k-points, 16 states: 85 us).
 // Slopes are kept in FP32, which holds them exactly (the finish forms them in FP32; no coherent or drift term here). Conversions and comparisons of doubles run on the FP64 pipe too
 // (with them it was 79 % busy): they are integer operations here, and each real takes one fused multiply-add.
 // ---------------------------------------------------------------------------------------------

@@ -33,7 +33,7 @@
 //   coordinate r = m 2^(f - 1075);  R = (m 2^6) >> (T - (f - d)) = rh 2^32 + rl,  |R| < 2^59
 //   sum       (A0 + A1 2^-32) 2^(emax + T - 1077),  A0 += h rh,  A1 += h rl + l rh, exact in 64 bits for the 8 real
 //             terms of 4 products (A0 2^58 beside the 2^61 at which it is shifted, A1 8 (2^59 + 2^58))
-// It takes 57 us there (43 % of the HBM rate: what bounds it is the latency of index, then coordinate, with 21 warps
+// It takes 51 us there (47 % of the HBM rate: what bounds it is the latency of index, then coordinate, with 21 warps
 // per SM; the next chunk's index words are loaded ahead: 10 us of the step's 267); an RK4 step of 2000 k-points went from
 // 702 to 257 us, of 100 from 206 to 60.
 // The dropped l rl is at most 2^-57 of the largest product, the bits lost to a shift 2^-56 of it, and a sum is rounded
