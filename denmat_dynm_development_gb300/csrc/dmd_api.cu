@@ -972,13 +972,9 @@ int choose_form(dmd_handle* h, dmd::PairLayout& L) {
   CK(cudaMemcpy(h->d_items, L.items.data(), L.items.size() * sizeof(dmd::WorkItem), cudaMemcpyHostToDevice));
   h->nitems = (int)L.items.size();
   if (h->use_fx) {
-    unsigned* has = (unsigned*)h->d_acc;  // scratch: rewritten by every evaluation
-    CK(cudaMemsetAsync(has, 0, (size_t)h->nk * 4, h->st));
-    for (int pass = 0; pass < 2; ++pass) {
-      const unsigned g = blocks_for(h->nitems, 4);
-      if (h->nb == 2) k_fx_static<2><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->nk, pass, has, h->d_st);
-      else k_fx_static<4><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->nk, pass, has, h->d_st);
-    }
+    const unsigned g = blocks_for(h->nitems, 4);
+    if (h->nb == 2) k_fx_static<2><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->d_st);
+    else k_fx_static<4><<<g, 128, 0, h->st>>>(h->d_items, h->nitems, h->d_rbz, (const int4*)h->d_P, h->d_ex, h->d_st);
     CKL();
     CK(cudaStreamSynchronize(h->st));
   }

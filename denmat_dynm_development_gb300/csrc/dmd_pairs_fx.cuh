@@ -55,8 +55,7 @@ constexpr int kFxCBits = 59;         // column coordinate bits
 constexpr int kFxBase = 32;          // digit base 2^32
 constexpr int kFxExZero = -20000;    // exponent of a group without a nonzero element
 // Bits below the unit from which on sums are listed. A column that lies that far below by its elements alone (k_fx_static) is weak here
-// and not elsewhere: it is listed where its sum lies kFxWeakMore bits lower still, or fx_weak_most below the unit, and not at
-// all where only off-diagonal coordinates reach it.
+// and most often not elsewhere: it is listed where its sum lies kFxWeakMore bits lower still, or fx_weak_most below the unit.
 constexpr int kFxWeakRow = 7, kFxWeakMore = 5;
 __host__ __device__ constexpr int fx_weak_column(int nb) { return nb == 2 ? 8 : 7; }  // (the row digits: fx_row_bits)
 __host__ __device__ constexpr int fx_weak_most(int nb) { return fx_weak_column(nb) + 4; }
@@ -321,37 +320,32 @@ __global__ void __launch_bounds__(128) k_fx_quantise(long long nrb, const RowBlo
 }
 
 // How far a column's elements lie below the item's largest where the coordinates are alike: st[item][matrix][column], in bits,
-// from the lines of the diagonal coordinates (the off-diagonal ones are small). kFxNoLine: no element of those lines here, but
-// elsewhere in the k-point's sum (has[k]: bit 0 Y's, bit 1 X's), or none of any line. One warp per item; first (pass 0) has, then st.
-constexpr int kFxNoLine = 127;
+// from the lines of the diagonal coordinates (the off-diagonal ones are mostly small). kFxNone: no element at all. One warp per item.
+constexpr int kFxNone = 127;
 template <int NB>
 __global__ void __launch_bounds__(128) k_fx_static(const WorkItem* __restrict__ items, int nitems, const RowBlock* __restrict__ rbz,
-                                                   const int4* __restrict__ P, const int16_t* __restrict__ ex, int nk, int pass,
-                                                   unsigned* __restrict__ has, int8_t* __restrict__ st) {
+                                                   const int4* __restrict__ P, const int16_t* __restrict__ ex,
+                                                   int8_t* __restrict__ st) {
   constexpr int NB2 = NB * NB, NB4 = NB2 * NB2, W = 128 / NB2, NL = 2 * NB2;
   const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, qg = lane / W, sl = lane % W;
   if (item >= nitems) return;
   const WorkItem w = items[item];
-  const int col = w.J * W + sl;
   for (int m = 0; m < 2; ++m) {
     int own = kFxExZero, all = kFxExZero, any = kFxExZero;  // the column's and the item's largest; the column's of every line
     for (int rb = w.rb0; rb < w.rb1; ++rb) {
       const RowBlock b = rbz[rb];
       const int n = __popc(b.mask), slot = __popc(b.mask & ((1u << sl) - 1u));
-      const bool rev = (b.revmask >> sl) & 1u;
       for (int a = 0; a < NB2; ++a) {
         const bool diag = a / NB == a % NB;
         const int16_t* x = ex + ((size_t)rb * NL + m * NB2 + a) * 2;
         if (diag) all = max(all, max((int)x[0], (int)x[1]));
-        if (!((b.mask >> sl) & 1u)) continue;
+        if (!((b.revmask >> sl) & 1u)) continue;
         for (int i = 0; i < 4; ++i) {
           const int e = 4 * qg + i;
           const int4 v = P[(size_t)b.pair0 * 2 * NB4 + ((size_t)(m * NB2 + a) * NB2 + e) * n + slot];
           const long long p = (long long)v.x * (1LL << kFxBase) + v.y, q = (long long)v.z * (1LL << kFxBase) + v.w;
-          const unsigned long long u = (unsigned long long)(p ^ (p >> 63)) | (unsigned long long)(q ^ (q >> 63));
+          const unsigned long long u = (unsigned long long)(p < 0 ? -p : p) | (unsigned long long)(q < 0 ? -q : q);
           if (u == 0ull) continue;
-          if (!pass && e / NB == e % NB) atomicOr(&has[b.row], 2u >> m);
-          if (!rev) continue;
           const int t = 64 - __clzll((long long)u) + x[e / NB == e % NB ? 0 : 1] - kFxPBits;
           any = max(any, t);
           if (diag) own = max(own, t);
@@ -363,14 +357,9 @@ __global__ void __launch_bounds__(128) k_fx_static(const WorkItem* __restrict__ 
       own = max(own, __shfl_xor_sync(0xffffffffu, own, o));
       any = max(any, __shfl_xor_sync(0xffffffffu, any, o));
     }
-    if (qg || col >= nk) continue;
-    if (!pass) {
-      if (own != kFxExZero) atomicOr(&has[col], 1u << m);
-    } else {
-      const bool none = own == kFxExZero;
-      st[((size_t)item * 2 + m) * W + sl] =
-          (int8_t)(none ? (((has[col] >> m) & 1u) || any == kFxExZero ? kFxNoLine : 0) : min(max(all - own, 0), kFxNoLine - 1));
-    }
+    if (qg) continue;
+    st[((size_t)item * 2 + m) * W + sl] =
+        (int8_t)(any == kFxExZero ? kFxNone : own == kFxExZero ? kFxNone - 1 : min(max(all - own, 0), kFxNone - 1));
   }
 }
 
@@ -844,7 +833,7 @@ __device__ __forceinline__ void fx_item(unsigned char* const wbase, const int it
     unsigned cols = __ballot_sync(FULL, small);
     if (cols) {
       const int s = st[((size_t)item * 2 + m) * W + sl];
-      small = small && s != kFxNoLine && below >= min(max(s + kFxWeakMore, fx_weak_column(NB)), fx_weak_most(NB));
+      small = small && s != kFxNone && below >= min(max(s + kFxWeakMore, fx_weak_column(NB)), fx_weak_most(NB));
       cols = __ballot_sync(FULL, small);
     }
     if (cols) {

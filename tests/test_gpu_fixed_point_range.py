@@ -208,3 +208,7 @@ def test_mostly_zero_operators(nk, nb, density, fill, oracle, built):
     y = oracle.y_of(s.dm0)
     assert worst(s, y, 5.0 * oracle.fs) < EPS
     assert worst(s, y * (1.0 + 1e-2 * rng.standard_normal(y.size)), 5.0 * oracle.fs) < EPS
+    rank = np.argsort(np.argsort(s.e_dm.mean(1)))
+    for kind in ("spot", "tail", "random"):
+        z = np.ascontiguousarray(localised(rng, nk, nb, kind)[rank]).view(np.float64).reshape(-1)
+        assert worst(s, z, 5.0 * oracle.fs) < EPS
