@@ -22,10 +22,11 @@ FLAG_ADJOINT = 2  # DMD_FLAG_ADJOINT: keep the operators in stored order for adj
 FLAG_EE = 4  # DMD_FLAG_EE: keep P_eph (+ P_eimp) in stored order and the column-block map for the e-e model
 FLAG_SPARSE = 8  # DMD_FLAG_SPARSE: contract only the stored elements (alg_sparseP / alg_Pin_is_sparse)
 # sparse="auto" picks the sparse contraction below this fraction of stored elements: where it is the faster one of the two
-# (us per RK4 step, dense and sparse). nb = 4, 181k pairs: 1224, 1394 at 44 %; 1225, 1046 at 31 %; 697k: 3867, 4771; 3868, 3462;
-# 46k: 433, 434; 435, 342. nb = 2, 71k pairs: 87, 103 at 31 %; 87, 92 at 24 %; 87, 86 at 18 %; 398k: 233, 254; 235, 219; 234, 181.
+# (us per RK4 step, dense and sparse). nb = 4, 181k pairs: 1221, 1210 at 37 %; 1221, 1049 at 31 %; 697k: 3867, 4771 at 44 %; 3868,
+# 3462 at 31 %; 46k: 435, 434 at 44 %. nb = 2, 1.6M pairs: 668, 703 at 31 %; 671, 630 at 27 %; 398k: 251, 256; 253, 237; 71k: 109, 113
+# at 37 %; 110, 103 at 31 %.
 # The dense form of the other band counts runs on the FP64 pipe, as all of them did where 44 % was the limit.
-SPARSE_AUTO_FILL = {2: 0.2, 4: 0.35}
+SPARSE_AUTO_FILL = {2: 0.3, 4: 0.35}
 SPARSE_AUTO_FILL_OTHER = 0.4
 
 

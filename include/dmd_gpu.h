@@ -76,7 +76,7 @@ extern "C" {
                                (the reference's default thr_sparseP; explicit zeros of sparse files are
                                dropped as well) and contract those; DMD_PREC_F64, a single state, not
                                with DMD_FLAG_LINEAR, DMD_FLAG_ADJOINT or DMD_FLAG_EE. It pays below
-                               about a third (nb = 4) or a fifth (nb = 2) of the elements stored (bench --sparse) */
+                               about a third of the elements stored (bench --sparse) */
 
 /* pictures (alg.picture) */
 #define DMD_PICTURE_INTERACTION 0
